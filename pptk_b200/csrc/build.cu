@@ -1036,6 +1036,173 @@ __global__ void k_troots(const Rec<T, D>* recs, const int* root_rec, const int64
   root_tnode[c] = nt + c;
 }
 
+// --------------------------------------------------- wide hierarchy ----
+// Type of the traversal data of a tree of point type T (integer trees walk
+// in float).
+template <typename T>
+struct WalkOf {
+  typedef typename std::conditional<std::is_integral<T>::value, float, T>::type type;
+};
+
+// A record that a level of nodes of at most `cap` points divides.
+template <typename T, int D>
+__device__ __forceinline__ bool wide_inner(const Rec<T, D>& r, long long cap) {
+  return r.split_dim >= 0 && r.end - r.begin > cap && r.left >= 0 && r.right >= 0;
+}
+
+// The record that decides record r's range: r itself, or, below a record
+// with one child over the same points, that child (the bound only stops a
+// damaged file's cycle).
+template <typename T, int D>
+__device__ __forceinline__ int wide_resolve(const Rec<T, D>* recs, int r, long long cap) {
+  for (int guard = 0; guard < 4096; guard++) {
+    const Rec<T, D>& x = recs[r];
+    if (x.split_dim < 0 || x.end - x.begin <= cap || (x.left >= 0) == (x.right >= 0)) break;
+    r = x.left >= 0 ? x.left : x.right;
+  }
+  return r;
+}
+
+// Where the nodes of every level begin: at a cloud's first point and at the
+// right child of a record that the level divides.
+template <typename T, int D>
+__global__ void k_wide_mark(const Rec<T, D>* recs, int n_recs, int bucket, int levels, int words,
+                            const int64_t* valid_off, int ncloud, uint32_t* bits, const int* n_dev = nullptr) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < ncloud && valid_off[i + 1] > valid_off[i]) {
+    const int b = (int)valid_off[i];
+    for (int j = 0; j < levels; j++) atomicOr(&bits[j * words + (b >> 5)], 1u << (b & 31));
+  }
+  if (i >= n_recs || (n_dev && i >= *n_dev)) return;
+  const Rec<T, D>& r = recs[i];
+  for (int j = 0; j < levels && wide_inner(r, wide_cap(bucket, j)); j++) {
+    const int b = recs[r.right].begin;
+    atomicOr(&bits[j * words + (b >> 5)], 1u << (b & 31));
+  }
+}
+
+// A word of the node map as its number of nodes, for the scan.
+struct NodeWord {
+  uint32_t bits;
+  __device__ explicit operator int64_t() const { return __popc(bits); }
+};
+
+struct WideMap {
+  const uint32_t* bits;
+  const int* rank;
+  int words, levels, cap;
+  __device__ __forceinline__ int of(int j, int p) const {
+    const int w = j * words + (p >> 5);
+    return rank[w] + __popc(bits[w] & (0xffffffffu >> (31 - (p & 31)))) - 1;
+  }
+  __device__ __forceinline__ bool starts(int j, int p) const { return bits[j * words + (p >> 5)] >> (p & 31) & 1u; }
+};
+
+// Record r as a node of level j.  A record that no node begins at (a damaged
+// file's) is left out; one beyond the capacity (a rebuild that needs more) is
+// reported, and children beyond it are cut off.
+template <typename T, int D>
+__device__ __forceinline__ void wide_write(const Rec<T, D>& r, int j, const WideMap& m,
+                                           WNode<typename WalkOf<T>::type, D>* nodes, int* status) {
+  typedef typename WalkOf<T>::type V;
+  if (r.end <= r.begin || !m.starts(j, r.begin)) return;
+  const int i = m.of(j, r.begin);
+  if (i >= m.cap) {
+    if (status) atomicExch(status, 21);
+    return;
+  }
+  WNode<V, D> w;
+#pragma unroll
+  for (int d = 0; d < D; d++) {
+    w.lo[d] = (V)r.lo[d];
+    w.hi[d] = (V)r.hi[d];
+  }
+  w.begin = r.begin;
+  w.cnt = r.end - r.begin;
+  if (j > 0) {
+    w.begin = m.of(j - 1, r.begin);
+    w.cnt = -max(min(m.of(j - 1, r.end - 1) + 1, i) - w.begin, 0);
+  }
+  nodes[i] = w;
+}
+
+template <typename T, int D>
+__global__ void k_wide_fill(const Rec<T, D>* recs, int n_recs, int bucket, const int* root_rec, int ncloud, WideMap m,
+                            WNode<typename WalkOf<T>::type, D>* nodes, const int* n_dev = nullptr,
+                            int* status = nullptr) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < ncloud && root_rec[i] >= 0)
+    for (int j = m.levels - 1; j >= 0; j--) {
+      const int r = wide_resolve(recs, root_rec[i], wide_cap(bucket, j));
+      if (wide_inner(recs[r], wide_cap(bucket, j))) break;
+      wide_write<T, D>(recs[r], j, m, nodes, status);
+    }
+  if (i >= n_recs || (n_dev && i >= *n_dev)) return;
+  for (int j = 0; j < m.levels && wide_inner(recs[i], wide_cap(bucket, j)); j++)
+    for (int c = 0; c < 2; c++) {
+      const int r = wide_resolve(recs, c ? recs[i].right : recs[i].left, wide_cap(bucket, j));
+      if (!wide_inner(recs[r], wide_cap(bucket, j))) wide_write<T, D>(recs[r], j, m, nodes, status);
+    }
+}
+
+// Marks and ranks the nodes (on a capture-ready forest over the live
+// records, n_dev); wrank's last entry receives their number.
+template <typename T, int D>
+void wide_begin(TreeBase* t, int n_recs, cudaStream_t st, const int* n_dev = nullptr) {
+  int64_t most = 1;  // points of the largest cloud
+  for (int c = 0; c < t->ncloud; c++)
+    most = std::max(most, t->capture ? t->orig_off_h[c + 1] - t->orig_off_h[c] : t->valid_off_h[c + 1] - t->valid_off_h[c]);
+  const int levels = wide_levels(t->bucket, most);
+  const int64_t words = wide_words(t->capture ? t->n : t->nv);
+  if (!t->wbits || t->wlevels != levels || t->wwords != (int)words) {
+    if (t->wbits) dev_free(t->wbits, st);
+    if (t->wrank) dev_free(t->wrank, st);
+    t->wbits = nullptr;
+    t->wrank = nullptr;
+    t->wlevels = levels;
+    t->wwords = (int)words;
+    PPTKG_CUDA(dev_malloc((void**)&t->wbits, sizeof(uint32_t) * levels * words, st));
+    PPTKG_CUDA(dev_malloc((void**)&t->wrank, sizeof(int) * (levels * words + 1), st));
+  }
+  PPTKG_CUDA(cudaMemsetAsync(t->wbits, 0, sizeof(uint32_t) * levels * words, st));
+  k_wide_mark<T, D><<<div_up(std::max(n_recs, t->ncloud), 256), 256, 0, st>>>(
+      (const Rec<T, D>*)t->recs, n_recs, t->bucket, levels, (int)words, t->valid_off, t->ncloud, t->wbits, n_dev);
+  PPTKG_CHECK_LAUNCH();
+  exclusive_scan<NodeWord, int>((const NodeWord*)t->wbits, t->wrank, levels * words, t->wrank + levels * words, st);
+}
+
+template <typename T, int D>
+void wide_alloc(TreeBase* t, int n_wide, cudaStream_t st) {
+  if (t->wide) dev_free(t->wide, st);
+  t->wide = nullptr;
+  t->n_wide = n_wide;
+  PPTKG_CUDA(dev_malloc(&t->wide, (size_t)std::max(n_wide, 1) * sizeof(WNode<typename WalkOf<T>::type, D>), st));
+}
+
+// Fills the nodes; `clear`: entries that no record fills hold nothing.
+template <typename T, int D>
+void wide_fill(TreeBase* t, int n_recs, bool clear, cudaStream_t st, const int* n_dev = nullptr,
+               int* status = nullptr) {
+  typedef WNode<typename WalkOf<T>::type, D> Node;
+  if (t->n_wide <= 0) return;
+  if (clear) PPTKG_CUDA(cudaMemsetAsync(t->wide, 0, sizeof(Node) * (size_t)t->n_wide, st));
+  const WideMap m{t->wbits, t->wrank, t->wwords, t->wlevels, t->n_wide};
+  k_wide_fill<T, D><<<div_up(std::max(n_recs, t->ncloud), 256), 256, 0, st>>>(
+      (const Rec<T, D>*)t->recs, n_recs, t->bucket, t->root_rec, t->ncloud, m, (Node*)t->wide, n_dev, status);
+  PPTKG_CHECK_LAUNCH();
+}
+
+template <typename T, int D>
+void make_wide(TreeBase* t, cudaStream_t st) {
+  int n = 0;
+  wide_begin<T, D>(t, t->n_recs, st);
+  PPTKG_CUDA(cudaMemcpyAsync(&n, t->wrank + (int64_t)t->wlevels * t->wwords, sizeof(int), cudaMemcpyDeviceToHost, st));
+  PPTKG_CUDA(cudaStreamSynchronize(st));
+  wide_alloc<T, D>(t, n, st);
+  wide_fill<T, D>(t, t->n_recs, true, st);
+  PPTKG_CUDA(cudaStreamSynchronize(st));
+}
+
 // ------------------------------------------------------------ host side ----
 // Grid of the grid-stride level kernels: eight 256-thread blocks per SM.
 static int level_grid(int device) {
@@ -1348,14 +1515,20 @@ void make_tnodes(TreeBase* tree, int bucket, cudaStream_t st) {
   const int nr = tree->n_recs;
   const Rec<T, D>* recs = (const Rec<T, D>*)tree->recs;
   BuildBuf<int> flag(nr + 1, st), tid(nr + 1, st);
-  int nt = 0;
+  int nt = 0, n_wide = 0;
+  wide_begin<T, D>(tree, nr, st);
+  PPTKG_CUDA(cudaMemcpyAsync(&n_wide, tree->wrank + (int64_t)tree->wlevels * tree->wwords, sizeof(int),
+                             cudaMemcpyDeviceToHost, st));
   if (nr > 0) {
     k_tflag<T, D><<<div_up(nr, 256), 256, 0, st>>>(recs, nr, bucket, flag.get());
     PPTKG_CHECK_LAUNCH();
     exclusive_scan<int, int>(flag.get(), tid.get(), nr, tid.get() + nr, st);
     PPTKG_CUDA(cudaMemcpyAsync(&nt, tid.get() + nr, sizeof(int), cudaMemcpyDeviceToHost, st));
-    PPTKG_CUDA(cudaStreamSynchronize(st));
   }
+  PPTKG_CUDA(cudaStreamSynchronize(st));
+  // (a capture-ready forest keeps at least the capacity it has)
+  wide_alloc<T, D>(tree, tree->capture ? std::max(n_wide, tree->n_wide) : n_wide, st);
+  wide_fill<T, D>(tree, nr, tree->capture, st);
   TNode<T, D>* nodes = nullptr;
   // a capture-ready forest keeps the capacity that its rebuilds fill
   const int64_t cap = tree->capture ? std::max<int64_t>(tree->cap_tnodes, (int64_t)nt + tree->ncloud)
@@ -1444,8 +1617,13 @@ void forest_capture_ready(TreeBase* t, cudaStream_t st) {
   grow(&t->tnodes, (size_t)t->n_tnodes * sizeof(TNode<T, D>), (size_t)t->cap_tnodes * sizeof(TNode<T, D>));
   t->n_tnodes = (int)t->cap_tnodes;
   t->tdepth += 8;
-  if (!t->dev_meta) PPTKG_CUDA(dev_malloc((void**)&t->dev_meta, 4 * sizeof(int64_t), st));
+  // wide nodes: twice the first build's; the map covers all input rows
   t->capture = true;
+  const int wide_now = t->n_wide;
+  wide_begin<T, D>(t, t->n_recs, st);
+  wide_alloc<T, D>(t, (int)std::min<int64_t>(INT32_MAX / 2, 2 * (int64_t)wide_now + 4096 + t->ncloud * t->wlevels), st);
+  wide_fill<T, D>(t, t->n_recs, true, st);
+  if (!t->dev_meta) PPTKG_CUDA(dev_malloc((void**)&t->dev_meta, 4 * sizeof(int64_t), st));
   PPTKG_CUDA(cudaStreamSynchronize(st));
 }
 
@@ -1557,6 +1735,8 @@ void rebuild_forest(TreeBase* t, const T* d_in, cudaStream_t st, int* status) {
   k_troots<T, D><<<div_up(ncloud, 128), 128, 0, st>>>(recs, t->root_rec, t->valid_off, ncloud, tflag.get(),
                                                       tid.get(), node_lim, nodes, t->root_tnode);
   PPTKG_CHECK_LAUNCH();
+  wide_begin<T, D>(t, rec_cap, st, nrec_dev);
+  wide_fill<T, D>(t, rec_cap, true, st, nrec_dev, status);
 }
 
 template <typename T, int D>
@@ -1603,6 +1783,9 @@ TreeBase::~TreeBase() {
   if (recs) dev_free(recs, stream);
   if (tnodes) dev_free(tnodes, stream);
   if (fwd) dev_free(fwd, stream);
+  if (wide) dev_free(wide, stream);
+  if (wbits) dev_free(wbits, stream);
+  if (wrank) dev_free(wrank, stream);
   if (root_rec) dev_free(root_rec, stream);
   if (root_tnode) dev_free(root_tnode, stream);
   if (valid_off) dev_free(valid_off, stream);
@@ -1617,7 +1800,8 @@ TreeBase::~TreeBase() {
 #define PPTKG_INST_BUILD(T, D)                                                                                  \
   template TreeBase* build_tree<T, D>(const T*, int64_t, int, double, int, cudaStream_t);                      \
   template TreeBase* build_forest<T, D>(const T*, int64_t, const int64_t*, int, int, double, int, cudaStream_t); \
-  template void make_tnodes<T, D>(TreeBase*, int, cudaStream_t);
+  template void make_tnodes<T, D>(TreeBase*, int, cudaStream_t);                                               \
+  template void make_wide<T, D>(TreeBase*, cudaStream_t);
 
 #define PPTKG_INST_CAPTURE(T, D)                                              \
   template void forest_capture_ready<T, D>(TreeBase*, cudaStream_t);          \

@@ -27,9 +27,14 @@ template <typename T, int D>
 TreeBase* build_forest(const T* d_points, int64_t n, const int64_t* orig_off_h, int ncloud, int max_leaf,
                        double empty_split, int bucket, cudaStream_t st);
 
-// (Re)derives the traversal hierarchy for a bucket size.
+// (Re)derives the traversal hierarchies (TNode and WNode) for a bucket size.
 template <typename T, int D>
 void make_tnodes(TreeBase* tree, int bucket, cudaStream_t st);
+
+// (Re)derives the wide hierarchy alone, from the records (a tree read back
+// from a file keeps no copy of it).  Synchronises.
+template <typename T, int D>
+void make_wide(TreeBase* tree, cudaStream_t st);
 
 // Capture mode of a forest built by build_forest (float32 / float64):
 // forest_capture_ready gives its arrays their capacities and fixes the

@@ -190,6 +190,8 @@ TreeBase* load_tree(const char* buf, size_t size, cudaStream_t st) {
   if (h.n < 0 || h.nv < 0 || h.nv > h.n || h.n > (int64_t)INT32_MAX / 2 || h.n_recs < 0 || h.n_tnodes < 0 ||
       h.ncloud < 1 || h.depth < 0 || h.tdepth < 0 || h.bucket < 1 || h.n_tnodes < h.ncloud)
     throw Error(E_INVALID, "stored tree: inconsistent header");
+  // (traversal data is double for float64 points and float for all others)
+  if ((h.dtype == F64) != (h.rec_dtype == F64)) throw Error(E_INVALID, "stored tree: inconsistent header");
   int64_t want[8];
   section_bytes(h.dtype, h.rec_dtype, h.dim, h.n, h.nv, h.n_recs, h.n_tnodes, h.ncloud, want);
   size_t total = sizeof(Header);
@@ -298,6 +300,9 @@ TreeBase* load_tree(const char* buf, size_t size, cudaStream_t st) {
   PPTKG_CUDA(cudaMemcpyAsync(&hb, bad.get(), sizeof(int), cudaMemcpyDeviceToHost, st));
   PPTKG_CUDA(cudaStreamSynchronize(st));
   if (hb) throw Error(E_INVALID, "stored tree: a node, point id or index map entry is out of range");
+  with_types(h.dtype, h.rec_dtype, h.dim, [&](auto, auto tr, auto d) {
+    make_wide<decltype(tr), decltype(d)::value>(t.get(), st);
+  });
   return t.release();
 }
 

@@ -16,6 +16,10 @@ namespace pptkg {
 constexpr int QWARPS = 4;
 constexpr int QTHREADS = QWARPS * 32;
 
+// Stack entries of a walk over a wide hierarchy: the nodes of one step and a
+// mark for the rest of their siblings, for every level above the leaf ranges.
+inline int wide_stack(int levels) { return 34 * (levels > 1 ? levels - 1 : 1); }
+
 template <typename T, int D>
 TreeView<T, D> view_of(const TreeBase* t) {
   TreeView<T, D> v;
@@ -28,6 +32,13 @@ TreeView<T, D> view_of(const TreeBase* t) {
   v.fwd = t->fwd;
   v.n_in = (int)t->n;
   v.pts_cap = (int)(t->capture ? t->n : t->nv);
+  v.wide = (const WNode<T, D>*)t->wide;
+  v.wbits = t->wbits;
+  v.wrank = t->wrank;
+  v.wwords = t->wwords;
+  v.wlevels = t->wlevels;
+  v.n_wide = t->n_wide;
+  v.wstack = wide_stack(t->wlevels);
   v.err = bounds_word(t->device);
   return v;
 }
@@ -42,24 +53,42 @@ __host__ __device__ constexpr size_t stage_bytes() {
   return 32 * (sizeof(PointRec<T, D>) > sizeof(QStage<DistT, D>) ? sizeof(PointRec<T, D>) : sizeof(QStage<DistT, D>));
 }
 
+// r-near walks: a leaf chunk and one stack entry per level.
 template <typename T, int D>
-__host__ __device__ __forceinline__ size_t warp_smem_bytes(int depth, int logcap = 0) {
+__host__ __device__ __forceinline__ size_t rnear_smem_bytes(int depth) {
+  return stage_bytes<T, D>() + (((size_t)depth * sizeof(int) + 15) & ~(size_t)15);
+}
+
+template <typename T, int D>
+__device__ __forceinline__ WarpScratch<T, D> rnear_scratch(int depth) {
+  extern __shared__ __align__(16) unsigned char qsm[];
+  unsigned char* base = qsm + (threadIdx.x >> 5) * rnear_smem_bytes<T, D>(depth);
+  WarpScratch<T, D> ws;
+  ws.buf = (PointRec<T, D>*)base;
+  ws.stack = (int*)(base + stage_bytes<T, D>());
+  return ws;
+}
+
+// kNN walks: the queries, the stack, the distance matrix and candidate ids of
+// a bucket scan, and (normals) `logcap` list slots per lane.
+template <typename T, int D>
+__host__ __device__ __forceinline__ size_t warp_smem_bytes(int stack, int logcap = 0) {
   typedef typename DistOf<T>::type DistT;
-  return stage_bytes<T, D>() + (((size_t)depth * sizeof(StackEnt<T, D>) + 15) & ~(size_t)15) +
+  return stage_bytes<T, D>() + (((size_t)stack * sizeof(int2) + 15) & ~(size_t)15) +
          ((32 * 33 * sizeof(DistT) + 15) & ~(size_t)15) + 32 * 4 + (size_t)logcap * 32 * 4;
 }
 
 template <typename T, int D>
-__device__ __forceinline__ WarpScratch<T, D> warp_scratch(int depth, int logcap = 0) {
+__device__ __forceinline__ WarpScratch<T, D> warp_scratch(int stack, int logcap = 0) {
   typedef typename DistOf<T>::type DistT;
   extern __shared__ __align__(16) unsigned char qsm[];
-  const size_t per = warp_smem_bytes<T, D>(depth, logcap);
+  const size_t per = warp_smem_bytes<T, D>(stack, logcap);
   unsigned char* base = qsm + (threadIdx.x >> 5) * per;
   WarpScratch<T, D> ws;
   ws.buf = (PointRec<T, D>*)base;
   base += stage_bytes<T, D>();
   ws.stack = (int*)base;
-  base += ((size_t)depth * sizeof(StackEnt<T, D>) + 15) & ~(size_t)15;
+  base += ((size_t)stack * sizeof(int2) + 15) & ~(size_t)15;
   ws.dmat = (DistT*)base;
   base += (32 * 33 * sizeof(DistT) + 15) & ~(size_t)15;
   ws.cid = (int*)base;
@@ -159,6 +188,22 @@ __device__ __forceinline__ int forest_query(int slot, const SlotMap& fm, TreeVie
   tv.root = fm.root_tnode[c];
   const int64_t p = fm.valid_off[c] + (slot - fm.slot_off[c]);
   return p < fm.valid_off[c + 1] ? tv.pt(p).id : -1;
+}
+
+// The wide hierarchy's top node of the warp's tree (of its cloud in a
+// forest), or -1.
+template <typename T, int D>
+__device__ __forceinline__ int top_node(int slot, const SlotMap& fm, const TreeView<T, D>& tv) {
+  int p = 0;
+  if (fm.warp_cloud && !fm.views) {
+    const int c = fm.warp_cloud[slot >> 5];
+    p = (int)fm.valid_off[c];
+    if (fm.valid_off[c + 1] <= p) return -1;
+  }
+  if (tv.n_wide <= 0) return -1;
+  // (the capacity binds only after a rebuild that reported it)
+  const int i = tv.wide_of(tv.wlevels - 1, p);
+  return i < tv.n_wide ? i : -1;
 }
 
 // Per-lane stack capacity of the per-lane walk (trees deeper than this use
@@ -491,7 +536,7 @@ __global__ void __launch_bounds__(QTHREADS, knn_min_blocks(KMAX, sizeof(typename
   typedef typename DistOf<T>::type DistT;
   const int slot = blockIdx.x * QTHREADS + threadIdx.x;
   if ((slot & ~31) >= m) return;
-  WarpScratch<T, D> ws = warp_scratch<T, D>(tv.depth);
+  WarpScratch<T, D> ws = warp_scratch<T, D>(tv.wstack);
   int qid = -1, own = -1, anchor = -1;
   DistT q[D];
   bool active = false;
@@ -511,7 +556,7 @@ __global__ void __launch_bounds__(QTHREADS, knn_min_blocks(KMAX, sizeof(typename
   if (active) warm_topk<T, D, DistT>(top, tv, fm, slot, q, anchor, k, own, r2, warm_bound, warm_mult, wlo, wn);
   const bool ok = use_lane_walk<LANE_STACK>(anchor, active, lane_span, tv.depth)
                       ? lane_knn<LANE_STACK, T, D>(tv, q, own, active, r2, top, wlo, wn)
-                      : packet_knn<T, D>(tv, q, own, active, r2, top, ws, wlo, wn);
+                      : wide_knn<T, D>(tv, top_node<T, D>(slot, fm, tv), q, anchor, own, active, r2, top, ws, wlo, wn);
   if (!ok) atomicExch(status, 1);
   if (qid >= 0) {
     int c = 0;
@@ -531,7 +576,7 @@ template <typename T, int D, int KMAX, typename L>
 void launch_knn(const TreeBase* t, L ld, const int* order, int mode, int m, int k, typename DistOf<T>::type r2,
                 int32_t* d_idx, int32_t* d_cnt, int* status, cudaStream_t st, SlotMap fm) {
   if (m <= 0) return;
-  const size_t smem = QWARPS * warp_smem_bytes<T, D>(t->tdepth);
+  const size_t smem = QWARPS * warp_smem_bytes<T, D>(wide_stack(t->wlevels));
   if (smem > 48 * 1024)
     PPTKG_CUDA(cudaFuncSetAttribute(k_knn<T, D, KMAX, L>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   k_knn<T, D, KMAX, L><<<div_up(m, QTHREADS), QTHREADS, smem, st>>>(view_of<T, D>(t), ld, order, mode, m, k, r2,
@@ -696,7 +741,7 @@ __global__ void __launch_bounds__(QTHREADS) k_rnear_count(TreeView<T, D> tv, L l
   typedef typename DistOf<T>::type DistT;
   const int slot = blockIdx.x * QTHREADS + threadIdx.x;
   if ((slot & ~31) >= m) return;
-  WarpScratch<T, D> ws = warp_scratch<T, D>(tv.depth);
+  WarpScratch<T, D> ws = rnear_scratch<T, D>(tv.depth);
   int qid = -1, own = -1;
   DistT q[D];
   bool active = false;
@@ -721,7 +766,7 @@ __global__ void __launch_bounds__(QTHREADS) k_rnear_fill(TreeView<T, D> tv, L ld
   typedef typename DistOf<T>::type DistT;
   const int slot = blockIdx.x * QTHREADS + threadIdx.x;
   if ((slot & ~31) >= m) return;
-  WarpScratch<T, D> ws = warp_scratch<T, D>(tv.depth);
+  WarpScratch<T, D> ws = rnear_scratch<T, D>(tv.depth);
   int qid = -1, own = -1;
   DistT q[D];
   bool active = false;
@@ -951,7 +996,7 @@ int64_t rnear_count(const TreeBase* t, const QuerySpec& qs, double dmax, int64_t
   DevBuf<int> order;
   const int mode = make_order<T, D>(t, qs, order, st);
   const DistT r2 = radius2<DistT>(dmax);
-  const size_t smem = QWARPS * warp_smem_bytes<T, D>(t->tdepth);
+  const size_t smem = QWARPS * rnear_smem_bytes<T, D>(t->tdepth);
   Stage stage("rnear_count", st);
   with_loader<T, D>(t, qs, [&](auto ld) {
     typedef decltype(ld) L;
@@ -984,7 +1029,7 @@ void rnear_fill(const TreeBase* t, const QuerySpec& qs, double dmax, const int64
   DevBuf<int> order;
   const int mode = make_order<T, D>(t, qs, order, st);
   const DistT r2 = radius2<DistT>(dmax);
-  const size_t smem = QWARPS * warp_smem_bytes<T, D>(t->tdepth);
+  const size_t smem = QWARPS * rnear_smem_bytes<T, D>(t->tdepth);
   Stage stage("rnear_fill", st);
   with_loader<T, D>(t, qs, [&](auto ld) {
     typedef decltype(ld) L;
@@ -1107,7 +1152,7 @@ k_normals(TreeView<T, 3> tv, L ld, const int* order, int order_mode, int m,
   constexpr int LOGCAP = normals_logcap(KMAX);
   const int slot = blockIdx.x * QTHREADS + threadIdx.x;
   if ((slot & ~31) >= m) return;
-  WarpScratch<T, 3> ws = warp_scratch<T, 3>(tv.depth, LOGCAP);
+  WarpScratch<T, 3> ws = warp_scratch<T, 3>(tv.wstack, LOGCAP);
   const int lane = threadIdx.x & 31;
   int qid = -1, own = -1, grp = 0, anchor = -1;
   DistT q[3];
@@ -1128,7 +1173,7 @@ k_normals(TreeView<T, 3> tv, L ld, const int* order, int order_mode, int m,
   if (active) warm_topk<T, 3, DistT>(top, tv, fm, slot, q, anchor, k, own, r2, warm_bound, warm_mult, wlo, wn);
   const bool ok = use_lane_walk<LANE_STACK>(anchor, active, lane_span, tv.depth)
                       ? lane_knn<LANE_STACK, T, 3>(tv, q, own, active, r2, top, wlo, wn)
-                      : packet_knn<T, 3>(tv, q, own, active, r2, top, ws, wlo, wn);
+                      : wide_knn<T, 3>(tv, top_node<T, 3>(slot, fm, tv), q, anchor, own, active, r2, top, ws, wlo, wn);
   if (!ok) atomicExch(status, 1);
   if (qid < 0) return;
   if (!active) {
@@ -1198,7 +1243,7 @@ __global__ void __launch_bounds__(QTHREADS) k_normals_rnear(TreeView<T, 3> tv, L
   typedef typename DistOf<T>::type DistT;
   const int slot = blockIdx.x * QTHREADS + threadIdx.x;
   if ((slot & ~31) >= m) return;
-  WarpScratch<T, 3> ws = warp_scratch<T, 3>(tv.depth);
+  WarpScratch<T, 3> ws = rnear_scratch<T, 3>(tv.depth);
   int qid = -1, own = -1;
   DistT q[3];
   bool active = false;
@@ -1374,7 +1419,7 @@ void launch_normals(const TreeBase* t, L ld, const int* order, int mode, int m, 
                     int num_eigen, double gap_thr, T* ev, T* ew, int32_t* sz, int* fix, int* nfix, int* status,
                     cudaStream_t st, SlotMap fm = SlotMap{}, int32_t* kidx = nullptr, int32_t* kcnt = nullptr) {
   if (m <= 0) return;
-  const size_t smem = QWARPS * warp_smem_bytes<T, 3>(t->tdepth, normals_logcap(KMAX));
+  const size_t smem = QWARPS * warp_smem_bytes<T, 3>(wide_stack(t->wlevels), normals_logcap(KMAX));
   if (smem > 48 * 1024)
     PPTKG_CUDA(
         cudaFuncSetAttribute(k_normals<T, KMAX, L, PREC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -1537,7 +1582,7 @@ void normals_query(const TreeBase* t, const QuerySpec& qs_in, int k, float r, in
         view_of<T, 3>(t), ld, order.get(), mode, m, r2, si, num_eigen, d_evecs, d_evals, d_sizes, status.get());
     PPTKG_CHECK_LAUNCH();
   } else if (k == -1) {
-    const size_t smem = QWARPS * warp_smem_bytes<T, 3>(t->tdepth);
+    const size_t smem = QWARPS * rnear_smem_bytes<T, 3>(t->tdepth);
     if (smem > 48 * 1024)
       PPTKG_CUDA(cudaFuncSetAttribute(k_normals_rnear<T, IndexQueries<3, false>>,
                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -1753,7 +1798,7 @@ struct MultiTables {
   DevBuf<int> order, anchor;
   bool ordered = false;
   int64_t n_slots = 0;
-  int depth = 0, n_nodes = 0;
+  int depth = 0, n_nodes = 0, wlevels = 0;
   SlotMap map() const {
     return SlotMap{warp_tree, slot_off, nullptr, nullptr, views, row_off, ordered ? order.get() : nullptr};
   }
@@ -1771,14 +1816,18 @@ void multi_tables(const TreeBase* const* trees, int ntrees, const int64_t* rows,
     v[g] = view_of<T, D>(t);
     mt.depth = std::max(mt.depth, t->tdepth);
     mt.n_nodes = std::max(mt.n_nodes, t->n_tnodes);
+    mt.wlevels = std::max(mt.wlevels, t->wlevels);
     const int64_t m = rows[g + 1] - rows[g];
     if (m < 0) throw Error(E_INVALID, "query offsets must not decrease");
     so[g + 1] = so[g] + (m + 31) / 32 * 32;
   }
   mt.n_slots = so[ntrees];
   if (mt.n_slots > INT32_MAX) throw Error(E_INVALID, "batch too large for one pass");
-  // every view uses the batch-wide stack bound (shared memory is sized once)
-  for (auto& x : v) x.depth = mt.depth;
+  // every view uses the batch-wide stack bounds (shared memory is sized once)
+  for (auto& x : v) {
+    x.depth = mt.depth;
+    x.wstack = wide_stack(mt.wlevels);
+  }
   const size_t nw = (size_t)std::max<int64_t>(mt.n_slots / 32, 1);
   auto up = [](size_t b) { return (b + 255) / 256 * 256; };
   const size_t o_views = 0, o_so = up(sizeof(TreeView<T, D>) * ntrees), o_ro = o_so + up(8 * (ntrees + 1)),
@@ -1802,10 +1851,11 @@ void multi_tables(const TreeBase* const* trees, int ntrees, const int64_t* rows,
 
 // A stand-in tree carrying the batch-wide traversal bounds for the launch
 // helpers (which size shared memory from the tree they are given).
-static TreeBase* bounds_tree(int depth, int n_nodes) {
+static TreeBase* bounds_tree(int depth, int n_nodes, int wlevels) {
   TreeBase* b = new TreeBase();
   b->tdepth = depth;
   b->n_tnodes = n_nodes;
+  b->wlevels = wlevels;
   return b;
 }
 
@@ -1857,7 +1907,7 @@ void multi_knn(const TreeBase* const* trees, int ntrees, const void* d_q, int qd
     qs.m = rows[g + 1] - rows[g];
     return qs;
   }, st, true);
-  std::unique_ptr<TreeBase> bt(bounds_tree(mt.depth, mt.n_nodes));
+  std::unique_ptr<TreeBase> bt(bounds_tree(mt.depth, mt.n_nodes, mt.wlevels));
   DevBuf<int> status(1, st);
   PPTKG_CUDA(cudaMemsetAsync(status.get(), 0, sizeof(int), st));
   const DistT r2 = radius2<DistT>(dmax);
@@ -1890,7 +1940,7 @@ void multi_normals(const TreeBase* const* trees, int ntrees, const int32_t* d_id
     qs.exclude_self = false;
     return qs;
   }, st);
-  std::unique_ptr<TreeBase> bt(bounds_tree(mt.depth, mt.n_nodes));
+  std::unique_ptr<TreeBase> bt(bounds_tree(mt.depth, mt.n_nodes, mt.wlevels));
   DevBuf<int> status(1, st);
   PPTKG_CUDA(cudaMemsetAsync(status.get(), 0, sizeof(int), st));
   const DistT rr = (DistT)(T)r;

@@ -53,10 +53,45 @@ struct alignas(16) TNode {
   int32_t cnt[2];        // points under the child (0: no child)
 };
 
+// One node of the wide hierarchy that the kNN walks use.  Level j cuts the
+// reference tree at nodes of at most wide_cap(bucket, j) points, so its boxes
+// are those of whole nodes, and its nodes lie in tree order; the levels
+// follow one another in one array, the leaf ranges (level 0) first.  The
+// children of a node are the nodes of the level below over the same points:
+// consecutive entries, sixteen or so, which one coalesced load hands to the
+// lanes of a warp, one box test per lane.
+template <typename T, int D>
+struct alignas(16) WNode {
+  T lo[D];
+  int32_t begin;  // level 0: first tree position; above: first child
+  T hi[D];
+  int32_t cnt;  // level 0: points; above: -children
+};
+
+// Points that a node of level j holds at most: half a bucket (one chunk of a
+// warp at the default bucket of 64) times 16^j.
+__host__ __device__ __forceinline__ long long wide_cap(int bucket, int j) {
+  return (long long)(bucket >= 2 ? bucket / 2 : 1) << (4 * j);
+}
+// Levels until one node holds all of n points.
+inline int wide_levels(int bucket, long long n) {
+  int l = 1;
+  while (wide_cap(bucket, l - 1) < n) l++;
+  return l;
+}
+// Words of one level's node map: a bit per tree position.
+inline int64_t wide_words(int64_t n) { return n / 32 + 1; }
+
 template <typename T, int D>
 struct TreeView {
   const PointRec<T, D>* pts;
   const TNode<T, D>* nodes;
+  const WNode<T, D>* wide;
+  const uint32_t* wbits;  // [wlevels][wwords]: bit p % 32 of word p / 32: a node begins at tree position p
+  const int32_t* wrank;   // [wlevels][wwords]: nodes before the word's first (over all levels)
+  int32_t wwords, wlevels;
+  int32_t n_wide;  // nodes of the wide hierarchy (their capacity in a capture-ready forest)
+  int32_t wstack;  // stack entries of a walk, the most of a multi-tree batch
   int32_t nv;
   int32_t depth;    // traversal stack bound (TNode levels)
   int32_t n_nodes;  // TNode count: no traversal visits more nodes than this
@@ -82,6 +117,11 @@ struct TreeView {
   __device__ __forceinline__ const PointRec<T, D>& pt(int i) const { return pts[checked(i, pts_cap, 1)]; }
   __device__ __forceinline__ int pos_of(const int32_t* map, int o) const { return map[checked(o, n_in, 2)]; }
   __device__ __forceinline__ int node_index(int i) const { return checked(i, n_nodes, 3); }
+  // the wide hierarchy's node of level j that holds tree position p
+  __device__ __forceinline__ int wide_of(int j, int p) const {
+    const int c = checked(p, pts_cap, 1), w = j * wwords + (c >> 5);
+    return wrank[w] + __popc(wbits[w] & (0xffffffffu >> (31 - (c & 31)))) - 1;
+  }
 };
 
 // Host-side owner of one device tree, or of a forest of independent trees
@@ -105,6 +145,10 @@ struct TreeBase {
   void* recs = nullptr;     // Rec<T, D>[n_recs]
   void* tnodes = nullptr;   // TNode<T, D>[n_tnodes]
   int32_t* fwd = nullptr;   // original index -> tree position, -1 if dropped
+  void* wide = nullptr;       // WNode<T, D>[n_wide]
+  uint32_t* wbits = nullptr;  // [wlevels * wwords]
+  int32_t* wrank = nullptr;   // [wlevels * wwords + 1], the last: nodes of the last build
+  int n_wide = 0, wlevels = 0, wwords = 0;
   int ncloud = 1;
   int32_t* root_rec = nullptr;    // device [ncloud]: root record per cloud (-1: no valid point)
   int32_t* root_tnode = nullptr;  // device [ncloud]
