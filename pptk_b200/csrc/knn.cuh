@@ -267,8 +267,6 @@ struct WarpScratch {
   int* stack;
   PointRec<T, D>* buf;                   // 32 entries (r-near staging)
   int* log;                              // per-lane neighbour lists, lane-strided; null when unused
-  typename DistOf<T>::type* dmat;        // 32 x 33 distances (kNN bucket scan); null when unused
-  int* cid;                              // 32 candidate ids of the chunk being scanned (kNN)
 };
 
 // A lane's query as the rest of its warp reads it during a bucket scan:
@@ -361,6 +359,12 @@ __device__ __forceinline__ V lanes_max(V v) {
   }
 }
 
+// Lanes with a candidate to insert that make an insertion of the whole warp
+// worth while (wide_knn).  All-point normals / kNN k = 32 of the 20M-point
+// scene: 38.5 / 60.8 ms at 6 lanes, 37.1 / 56.5 at 12, 36.5 / 56.5 at 18,
+// against 40.5 / 68.0 when every chunk's marks are inserted at once.
+constexpr int DRAIN_LANES = 16;
+
 // Exact kNN of the lane's query over the points below node `root` of the
 // wide hierarchy (-1: none), ties in dist2 broken by point id, with the top-k
 // list in the lane's registers.  `own` (tree position or -1) is skipped,
@@ -374,12 +378,6 @@ __device__ __forceinline__ V lanes_max(V v) {
 // boxes of the packet's queries and the packet's largest bound.  Children
 // that pass are put off (inner nodes) or, nearest first, tested by every lane
 // against its own query and scanned if one needs them (leaf ranges).
-//
-// The binary walk that this replaces visited 45 nodes per packet of the
-// 20M-point scene one after the other, each a dependent load and some 400
-// instructions; this one takes 11 steps and 22 leaf tests.  All-point normals
-// (k = 16): 33.0 -> 25.5 ms; kNN of 20M points (k = 32): 75.3 -> 61.5 ms; 1M
-// scattered points: 3.2 -> 2.85 ms.
 //
 // Every leaf range that holds a candidate within a query's final bound is
 // scanned: the packet test bounds every lane's own test from below.  False
@@ -396,60 +394,82 @@ __device__ bool wide_knn(const TreeView<T, D>& tv, int root, const DistT* q, int
   for (int d = 0; d < D; d++) active = active && q[d] == q[d];
   if (root < 0 || !__any_sync(FULL, active)) return true;
   auto need = [&](DistT md) { return active && md < r2 && md <= top.worst(); };
-  // Leaf bucket scan, transposed: lane j holds candidate j of the chunk
-  // (one coalesced 16 B load), and the warp loops only over the lanes whose
-  // query needs this bucket.  For such a query i every lane computes its
-  // candidate's distance to q_i; the row goes to dmat[i][*] and the ballot of
-  // candidates that can enter list i becomes lane i's mark mask.  Each lane
-  // then inserts its marked candidates, reading distances from its row and
-  // the candidates' ids from the chunk's id row.
-  // The queries sit in the warp's staging buffer (unused by kNN walks) so
-  // that lane i's coordinates and bound arrive as one shared broadcast.
+  // Leaf range scan, transposed: lane j holds candidate j of the chunk (one
+  // coalesced load), and the warp loops only over the lanes whose query needs
+  // this range.  For such a query i every lane computes its candidate's
+  // distance to q_i, and the ballot of candidates that can enter list i
+  // becomes lane i's mark mask.  The queries sit in the warp's staging buffer
+  // so that lane i's coordinates and bound arrive as one shared broadcast.
+  //
+  // Marked candidates do not enter the lists at once: a third of the lanes
+  // need a chunk, each has a few marks, and a list insertion costs the warp as
+  // much for one lane as for 32.  A lane keeps the marks of up to two chunks,
+  // and an insertion runs once DRAIN_LANES lanes have one to make (or one
+  // lane's third chunk needs room).  Bounds that lag by a few candidates only
+  // cost some marks that the insertion then rejects.
   QStage<DistT, D>* qst = reinterpret_cast<QStage<DistT, D>*>(ws.buf);
   const DistT r2_below = below(r2);
 #pragma unroll
   for (int d = 0; d < D; d++) qst[lane].q[d] = q[d];
+  unsigned mark0 = 0, mark1 = 0;  // marks held back, and the chunks they belong to
+  int base0 = 0, base1 = 0;
+  // one held-back candidate of every lane that has one enters its list
+  auto take = [&]() {
+    if (mark0) {
+      const int t = __ffs(mark0) - 1;
+      mark0 &= mark0 - 1;
+      const PointRec<T, D> r = tv.pt(base0 + t);
+      top.offer(point_dist2<T, DistT, D>(r.c, q), r.id);
+      if (!mark0) {
+        mark0 = mark1;
+        base0 = base1;
+        mark1 = 0;
+      }
+    }
+  };
   auto scan = [&](int begin, int count, bool mine) {
     const unsigned needm = __ballot_sync(FULL, mine);
     for (int base = begin; base < begin + count; base += 32) {
       const int nb = min(32, begin + count - base);
-      PointRec<T, D> pr;
+      T c[D];
       if (lane < nb) {
-        pr = tv.pt(base + lane);
+        const PointRec<T, D> pr = tv.pt(base + lane);
+#pragma unroll
+        for (int d = 0; d < D; d++) c[d] = pr.c[d];
       } else {
 #pragma unroll
-        for (int d = 0; d < D; d++) pr.c[d] = (T)0;
-        pr.id = -1;
+        for (int d = 0; d < D; d++) c[d] = (T)0;
       }
       // each needing lane publishes its entry bound for this chunk; the
       // loop below reads a query and its bound as one broadcast
       __syncwarp();
       qst[lane].thr = entry_bound(top.worst(), r2_below);
-      ws.cid[lane] = pr.id;
       __syncwarp();
-      const unsigned valid = nb == 32 ? FULL : (1u << nb) - 1u;
       unsigned mark = 0;
       unsigned rem = needm;
       while (rem) {
         const int i = __ffs(rem) - 1;
         rem &= rem - 1;
         const QStage<DistT, D> qi = qst[i];
-        const DistT d2 = point_dist2<T, DistT, D>(pr.c, qi.q);
-        ws.dmat[i * 33 + lane] = d2;
-        const unsigned m = __ballot_sync(FULL, d2 <= qi.thr) & valid;
+        const unsigned m = __ballot_sync(FULL, point_dist2<T, DistT, D>(c, qi.q) <= qi.thr);
         if (lane == i) mark = m;
       }
+      if (nb < 32) mark &= (1u << nb) - 1u;
       // the query's own point never enters its list, and the positions of
       // its warm-start window are in it already
       if (own >= base && own < base + nb) mark &= ~(1u << (own - base));
       mark &= ~window_bits(wlo - base, wn);
-      __syncwarp();
-      while (mark) {
-        const int t = __ffs(mark) - 1;
-        mark &= mark - 1;
-        top.offer(ws.dmat[lane * 33 + t], ws.cid[t]);
+      // (the loop ends: every pass takes a mark of each lane that has one)
+      while (__any_sync(FULL, mark && mark1) || __popc(__ballot_sync(FULL, mark0 != 0)) >= DRAIN_LANES) take();
+      if (mark0) {
+        if (mark) {
+          mark1 = mark;
+          base1 = base;
+        }
+      } else {
+        mark0 = mark;
+        base0 = base;
       }
-      __syncwarp();
     }
   };
   // The packet's queries in two boxes, cut where the distance from one lane's
@@ -583,6 +603,7 @@ __device__ bool wide_knn(const TreeView<T, D>& tv, int root, const DistT* q, int
       cnt = 32;
     }
   }
+  while (__any_sync(FULL, mark0 != 0)) take();
   return true;
 }
 

@@ -69,13 +69,12 @@ __device__ __forceinline__ WarpScratch<T, D> rnear_scratch(int depth) {
   return ws;
 }
 
-// kNN walks: the queries, the stack, the distance matrix and candidate ids of
-// a bucket scan, and (normals) `logcap` list slots per lane.
+// kNN walks: the queries, the stack, and (normals) `logcap` list slots per lane.
 template <typename T, int D>
 __host__ __device__ __forceinline__ size_t warp_smem_bytes(int stack, int logcap = 0) {
   typedef typename DistOf<T>::type DistT;
   return stage_bytes<T, D>() + (((size_t)stack * sizeof(int2) + 15) & ~(size_t)15) +
-         ((32 * 33 * sizeof(DistT) + 15) & ~(size_t)15) + 32 * 4 + (size_t)logcap * 32 * 4;
+         (size_t)logcap * 32 * 4;
 }
 
 template <typename T, int D>
@@ -89,10 +88,6 @@ __device__ __forceinline__ WarpScratch<T, D> warp_scratch(int stack, int logcap 
   base += stage_bytes<T, D>();
   ws.stack = (int*)base;
   base += ((size_t)stack * sizeof(int2) + 15) & ~(size_t)15;
-  ws.dmat = (DistT*)base;
-  base += (32 * 33 * sizeof(DistT) + 15) & ~(size_t)15;
-  ws.cid = (int*)base;
-  base += 32 * 4;
   ws.log = logcap ? (int*)base : nullptr;
   return ws;
 }
