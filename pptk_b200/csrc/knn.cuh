@@ -70,27 +70,27 @@ __device__ __forceinline__ DistT box_max_dist2(const T* lo, const T* hi, const D
 template <int KMAX, typename DistT>
 struct TopK;
 
-// Bitonic sort of N 64-bit keys held in registers (fully unrolled), into
-// descending (desc = true) or ascending order.
-template <int N>
-__device__ __forceinline__ void bitonic_sort(unsigned long long (&a)[N], bool desc) {
+// Sort of N 64-bit keys held in registers (fully unrolled), into descending
+// (desc = true) or ascending order: Batcher's odd-even merge exchange (Knuth,
+// The Art of Computer Programming, vol. 3, algorithm 5.2.2M), 63 exchanges
+// for 16 keys and 191 for 32, against 80 and 240 of a bitonic network (kNN k = 32 of 20M points:
+// 56.5 -> 54.4 ms; k = 16 within the noise).
+template <int N, int P = 1, int K = P>
+__device__ __forceinline__ void network_sort(unsigned long long (&a)[N], bool desc) {
 #pragma unroll
-  for (int size = 2; size <= N; size <<= 1)
-#pragma unroll
-    for (int stride = size / 2; stride > 0; stride >>= 1)
-#pragma unroll
-      for (int i = 0; i < N; i++) {
-        const int j = i ^ stride;
-        if (j > i) {
-          const unsigned long long x = a[i], y = a[j];
-          // blocks alternate direction; the last stage (size == N) has the
-          // requested one
-          const bool up = ((i & size) != 0) == desc;
-          const bool sw = up ? (x > y) : (x < y);
-          a[i] = sw ? y : x;
-          a[j] = sw ? x : y;
-        }
-      }
+  for (int c = 0; c < N - K; c++) {
+    // c = i + j of the algorithm: blocks of K out of every 2K, from K mod P on
+    const int from = K % P;
+    if (c < from || ((c - from) / K) % 2 || c / (2 * P) != (c + K) / (2 * P)) continue;
+    const unsigned long long x = a[c], y = a[c + K];
+    const bool sw = desc ? x < y : y < x;
+    a[c] = sw ? y : x;
+    a[c + K] = sw ? x : y;
+  }
+  if constexpr (K > 1)
+    network_sort<N, P, K / 2>(a, desc);
+  else if constexpr (2 * P < N)
+    network_sort<N, 2 * P, 2 * P>(a, desc);
 }
 
 // float distances: (dist2 bits << 32 | id) packed into one 64-bit key;
@@ -147,7 +147,7 @@ struct TopK<KMAX, float> {
   }
   __device__ __forceinline__ void set_empty(int j) { s[j] = lim; }
   __device__ __forceinline__ void set_dead(int j) { s[j] = 0ull; }
-  __device__ __forceinline__ void sort_desc() { bitonic_sort<KMAX>(s, true); }
+  __device__ __forceinline__ void sort_desc() { network_sort<KMAX>(s, true); }
   // The KMAX smallest of this list (sorted descending) and t (Q <= KMAX
   // keys sorted ascending, read as padded with keys above every list key),
   // sorted descending: the element-wise minimum of the two is a bitonic

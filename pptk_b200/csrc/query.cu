@@ -342,7 +342,7 @@ __device__ __forceinline__ void warm_topk(Top& top, const TreeView<T, D>& tv, co
         unsigned long long t[Q];
 #pragma unroll
         for (int j = 0; j < Q; j++) t[j] = key_at(start + off + j);
-        bitonic_sort<Q>(t, false);
+        network_sort<Q>(t, false);
         top.merge_smallest(t);
       }
       wlo = start;
