@@ -299,11 +299,11 @@ PPTKG_API int64_t pptkg_launch_count(void);
 
 /* Run-time tuning (no reference counterpart; set by the autotuner,
  * pptk_b200/autotune.py).  Settings are process-wide and read at launch.
- *   "lane_span": a kNN / normals warp whose 32 queries span more than this
- *     many tree positions walks the tree per lane rather than as one packet
- *     (-1: always packets).  Default 1024 (with warm-started lists, packets
- *     won down to about one query per ten tree points: 2M random queries on
- *     a 20M-point scene took 6.3 ms as packets, 10.6-12.0 ms with 256).
+ *   "lane_span": kNN and normal batches whose 32-query packets would span
+ *     more than this many tree positions on average (a third of it for
+ *     k > 16) run one warp per query, as do batches of at most 65,536
+ *     queries (-1: packets only, up to k = 64).  Default 1024.  Results do
+ *     not depend on it.
  *   "rnear_warp_queries": pptkg_rnear_count / pptkg_rnear_fill calls, and
  *     normals over r-near neighbourhoods (k = -1), with at most this many
  *     queries give each query a whole warp (the lanes split every bucket)

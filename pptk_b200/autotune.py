@@ -4,9 +4,9 @@ Five settings shape every kNN / normal traversal; none changes a result:
 
 * the leaf bucket size of the traversal hierarchy (``set_bucket`` on a tree
   or forest): larger buckets mean fewer node visits and more candidates;
-* ``lane_span`` (``pptkg_tune_set``): warps whose 32 queries span more tree
-  positions than this walk the tree one query per lane instead of as one
-  32-query packet -- the warps-per-query choice of the kNN walks;
+* ``lane_span`` (``pptkg_tune_set``): batches whose 32-query packets would
+  span more tree positions than this on average run one warp per query
+  instead -- the warps-per-query choice of the kNN walks;
 * ``warm_bound``: whether the warm-started lists also take the seed bound of
   a wider window of tree-order neighbours;
 * ``topk_min``: the k-tiling of the register top-k lists (their compile-time

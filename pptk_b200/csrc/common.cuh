@@ -45,8 +45,9 @@ enum Status {
 extern std::atomic<long long> g_launches;
 
 // Run-time tuning knobs (pptkg_tune_set / pptkg_tune_get), read at launch.
-//  lane_span: a kNN warp whose queries span more than this many tree
-//    positions walks the tree per lane instead of as a packet (-1: never).
+//  lane_span: kNN and normal batches whose 32-query packets would span more
+//    than this many tree positions on average run one warp per query, as do
+//    small batches (-1: never).
 extern std::atomic<int> g_tune_lane_span;
 //  rnear_warp_queries: r-near batches of at most this many queries run one
 //    warp per query instead of 32-query packets (0: never).

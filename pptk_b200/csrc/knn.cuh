@@ -607,14 +607,241 @@ __device__ bool wide_knn(const TreeView<T, D>& tv, int root, const DistT* q, int
   return true;
 }
 
-// Per-lane traversal for warps whose queries lie far apart, where a packet
-// walk would visit the union of 32 unrelated paths one node at a time.  Each
-// lane walks its own near-first depth-first path with a private stack of
-// deferred children (reference, size and box distance, re-tested on pop), so
-// the 32 walks advance side by side and their node loads overlap.  The set of
-// candidates each query accepts is the same as in the packet walk: every
-// point whose distance is within the query's final bound is offered, so the
-// result (the k smallest (dist2, id) pairs) is identical.
+// ------------------------------------------------- one warp per query ----
+// A (distance, point id) pair as one sortable value, ordered like the lists
+// above, and the warp operations on it.
+template <typename DistT>
+struct WarpKey;
+
+template <>
+struct WarpKey<float> {
+  unsigned long long v;  // dist2 bits << 32 | id
+  static __device__ __forceinline__ WarpKey make(float d2, int id) {
+    return {((unsigned long long)__float_as_uint(d2) << 32) | (unsigned)id};
+  }
+  static __device__ __forceinline__ WarpKey none(float r2) { return {(unsigned long long)__float_as_uint(r2) << 32}; }
+  __device__ __forceinline__ bool operator<(const WarpKey& o) const { return v < o.v; }
+  __device__ __forceinline__ float dist() const { return __uint_as_float((unsigned)(v >> 32)); }
+  __device__ __forceinline__ int id() const { return (int)(unsigned)v; }
+  __device__ __forceinline__ WarpKey from(int lane) const { return {__shfl_sync(0xffffffffu, v, lane)}; }
+  __device__ __forceinline__ WarpKey below() const { return {__shfl_up_sync(0xffffffffu, v, 1)}; }
+  __device__ __forceinline__ WarpKey across(int mask) const { return {__shfl_xor_sync(0xffffffffu, v, mask)}; }
+};
+
+template <>
+struct WarpKey<double> {
+  double d;
+  int i;
+  static __device__ __forceinline__ WarpKey make(double d2, int id) { return {d2, id}; }
+  static __device__ __forceinline__ WarpKey none(double r2) { return {r2, -1}; }
+  __device__ __forceinline__ bool operator<(const WarpKey& o) const { return d < o.d || (d == o.d && i < o.i); }
+  __device__ __forceinline__ double dist() const { return d; }
+  __device__ __forceinline__ int id() const { return i; }
+  __device__ __forceinline__ WarpKey from(int lane) const {
+    return {__shfl_sync(0xffffffffu, d, lane), __shfl_sync(0xffffffffu, i, lane)};
+  }
+  __device__ __forceinline__ WarpKey below() const {
+    return {__shfl_up_sync(0xffffffffu, d, 1), __shfl_up_sync(0xffffffffu, i, 1)};
+  }
+  __device__ __forceinline__ WarpKey across(int mask) const {
+    return {__shfl_xor_sync(0xffffffffu, d, mask), __shfl_xor_sync(0xffffffffu, i, mask)};
+  }
+};
+
+// The k <= 32 S smallest keys of one query, spread over the warp: element
+// 32 s + lane, ascending, in the lane's slot s.
+template <int S, typename DistT>
+struct WarpList {
+  typedef WarpKey<DistT> Key;
+  Key a[S];
+  Key limit;  // element k - 1: what a candidate has to beat
+  int k;
+  __device__ __forceinline__ void reset(int k_, DistT r2) {
+    k = k_;
+    limit = Key::none(r2);
+#pragma unroll
+    for (int s = 0; s < S; s++) a[s] = limit;
+  }
+  __device__ __forceinline__ void tighten() {
+#pragma unroll
+    for (int s = 0; s < S; s++)
+      if (s == (k - 1) >> 5) limit = a[s].from((k - 1) & 31);
+  }
+  // c (the same in every lane) takes its place; larger elements move up.
+  __device__ __forceinline__ void insert(Key c) {
+    const int lane = threadIdx.x & 31;
+    int r = 0;
+#pragma unroll
+    for (int s = 0; s < S; s++) r += __popc(__ballot_sync(0xffffffffu, a[s] < c));
+#pragma unroll
+    for (int s = S - 1; s >= 0; s--) {
+      Key up = a[s].below();
+      if (s > 0) {
+        const Key last = a[s > 0 ? s - 1 : 0].from(31);
+        if (lane == 0) up = last;
+      }
+      const int e = 32 * s + lane;
+      if (e == r)
+        a[s] = c;
+      else if (e > r)
+        a[s] = up;
+    }
+    tighten();
+  }
+  static __device__ __forceinline__ void exchange(Key& x, int mask, bool low) {
+    const Key y = x.across(mask);
+    if ((y < x) == low) x = y;
+  }
+  // A key per lane, as many of them as not real: sorted across the warp
+  // (bitonic, 15 exchanges), then merged through the slots.
+  __device__ __forceinline__ void merge(Key c) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int size = 2; size <= 32; size <<= 1)
+#pragma unroll
+      for (int m = size >> 1; m > 0; m >>= 1) exchange(c, m, ((lane & size) == 0 || size == 32) == ((lane & m) == 0));
+#pragma unroll
+    for (int s = 0; s < S; s++) {
+      // a[s] ascending against c descending: the smaller of each pair are the
+      // 32 smallest of both, in a bitonic order that five exchanges sort
+      const Key d = c.across(31);
+      const bool sw = d < a[s];
+      c = sw ? a[s] : d;
+      a[s] = sw ? d : a[s];
+#pragma unroll
+      for (int m = 16; m > 0; m >>= 1) {
+        exchange(a[s], m, (lane & m) == 0);
+        if (s + 1 < S) exchange(c, m, (lane & m) == 0);
+      }
+    }
+    tighten();
+  }
+};
+
+// Exact kNN of one query (q, the same in every lane) by a whole warp, over
+// the points below node `root` of the wide hierarchy: the children of a node
+// are tested one per lane against the query itself, the nearest first, and a
+// leaf range's points one per lane.  `home` (a leaf range, or -1) is scanned
+// first; `own` is skipped.  For batches whose packets would be too few to
+// fill the GPU or whose queries lie too far apart to share a walk.
+template <int S, typename T, int D, typename DistT>
+__device__ __forceinline__ bool warp_knn(const TreeView<T, D>& tv, int root, const DistT* q, int home, int own,
+                                         DistT r2, WarpList<S, DistT>& top, int2* stk) {
+  typedef WarpKey<DistT> Key;
+  const int lane = threadIdx.x & 31;
+  const unsigned FULL = 0xffffffffu;
+  const unsigned lt = (1u << lane) - 1u;
+  auto reach = [&]() { return __float_as_uint(float_above(top.limit.dist())); };
+  unsigned rmax = r2 > (DistT)0 ? reach() : 0u;
+  int sp = 0, steps = 0;
+  bool started = home < 0;
+  int at = started ? root : home, cnt = 1;
+  WNode<T, D> w;
+  if (lane < cnt) w = tv.wide[at + lane];
+  while (true) {
+    if (++steps > tv.n_wide + 1) return false;
+    bool hit = lane < cnt && w.cnt != 0 && !(started && at + lane == home);
+    unsigned md = 0;
+    if (hit) {
+      const DistT b = box_min_dist2<T, DistT, D>(w.lo, w.hi, q);
+      if constexpr (std::is_same<DistT, float>::value)
+        md = __float_as_uint(b);
+      else
+        md = __float_as_uint(__double2float_rd(b));
+      hit = md <= rmax;
+    }
+    unsigned hm = __ballot_sync(FULL, hit);
+    if (hm) {
+      if (__any_sync(FULL, hit && w.cnt > 0)) {
+        do {
+          const unsigned near = __reduce_min_sync(FULL, hit ? md : 0xffffffffu);
+          if (near > rmax) break;
+          const int s = __ffs(__ballot_sync(FULL, hit && md == near)) - 1;
+          if (lane == s) hit = false;
+          hm &= ~(1u << s);
+          const int begin = __shfl_sync(FULL, w.begin, s), end = begin + __shfl_sync(FULL, w.cnt, s);
+          for (int base = begin; base < end; base += 32) {
+            const int p = base + lane;
+            Key c = Key::none(r2);
+            bool in = false;
+            if (p < end) {
+              const PointRec<T, D> pr = tv.pt(p);
+              const DistT d2 = point_dist2<T, DistT, D>(pr.c, q);
+              in = d2 < r2 && p != own;
+              if (in) c = Key::make(d2, pr.id);
+              in = in && c < top.limit;
+            }
+            unsigned mark = __ballot_sync(FULL, in);
+            // a merge costs as much as a dozen insertions
+            if (__popc(mark) > 12) {
+              top.merge(in ? c : Key::none(r2));
+            } else {
+              while (mark) {
+                const Key x = c.from(__ffs(mark) - 1);
+                mark &= mark - 1;
+                if (x < top.limit) top.insert(x);
+              }
+            }
+          }
+          rmax = reach();
+        } while (hm);
+      } else {
+        const int n = __popc(hm);
+        if (sp + n > tv.wstack) return false;
+        const unsigned near = __reduce_min_sync(FULL, hit ? md : 0xffffffffu);
+        const int s = __ffs(__ballot_sync(FULL, hit && md == near)) - 1;
+        const int r = lane == s ? n - 1 : __popc(hm & lt) - (s < lane ? 1 : 0);
+        if (hit) stk[sp + r] = make_int2(at + lane, (int)md);
+        sp += n;
+        __syncwarp();
+      }
+    }
+    if (!started) {
+      started = true;
+      at = root;
+      cnt = 1;
+      if (lane == 0) w = tv.wide[root];
+      continue;
+    }
+    // the topmost entry still within reach (32 are looked at together)
+    int node = -1, from = 0;
+    while (sp > 0) {
+      const int2 e = lane < sp ? stk[sp - 1 - lane] : make_int2(0, -1);
+      const unsigned ok = __ballot_sync(FULL, lane < sp && (e.x < 0 || (unsigned)e.y <= rmax));
+      if (!ok) {
+        sp -= min(sp, 32);
+        continue;
+      }
+      const int s = __ffs(ok) - 1;
+      sp -= s + 1;
+      node = __shfl_sync(FULL, e.x, s);
+      if (node < 0) {
+        node = ~node;
+        from = __shfl_sync(FULL, e.y, s);
+      }
+      break;
+    }
+    __syncwarp();
+    if (node < 0) break;
+    at = tv.wide[node].begin + from;
+    cnt = -tv.wide[node].cnt - from;
+    if (cnt > 32) {
+      if (sp >= tv.wstack) return false;
+      if (lane == 0) stk[sp] = make_int2(~node, from + 32);
+      sp++;
+      __syncwarp();
+      cnt = 32;
+    }
+    if (lane < cnt) w = tv.wide[at + lane];
+  }
+  return true;
+}
+
+// Per-lane traversal for lists in device memory (k > 256).  Each lane walks
+// its own near-first depth-first path of the binary hierarchy with a private
+// stack of deferred children (reference, size and box distance, re-tested on
+// pop), so the 32 walks advance side by side and their node loads overlap.
+// Every point whose distance is within the query's final bound is offered.
 // Requires tv.depth <= LSTACK (the caller checks); false on a corrupt tree.
 template <int LSTACK, typename T, int D, typename DistT, typename Top>
 __device__ bool lane_knn(const TreeView<T, D>& tv, const DistT* q, int own, bool active, DistT r2, Top& top,
@@ -754,18 +981,6 @@ struct HeapTop {
     }
   }
 };
-
-// Warp-uniform choice of the traversal: per-lane walks when the warp's
-// queries span more than `span` tree positions (anchors: tree positions near
-// each query; -1 unknown), packet walks otherwise.
-template <int LSTACK>
-__device__ __forceinline__ bool use_lane_walk(int anchor, bool active, int span, int depth) {
-  const unsigned FULL = 0xffffffffu;
-  const bool known = active && anchor >= 0;
-  const int lo = __reduce_min_sync(FULL, known ? anchor : 0x7fffffff);
-  const int hi = __reduce_max_sync(FULL, known ? anchor : -1);
-  return span >= 0 && depth <= LSTACK && hi > lo && hi - lo > span;
-}
 
 // r-near over the whole tree in ascending tree position (the reference's
 // left-then-right order, kdtree-impl.h:519-558).  In COUNT mode a lane whose

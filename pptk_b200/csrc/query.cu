@@ -201,10 +201,6 @@ __device__ __forceinline__ int top_node(int slot, const SlotMap& fm, const TreeV
   return i < tv.n_wide ? i : -1;
 }
 
-// Per-lane stack capacity of the per-lane walk (trees deeper than this use
-// packet walks only).
-constexpr int LANE_STACK = 64;
-
 // Upper bound on the k-th smallest squared distance from q to the points of
 // the tree positions [lo, hi) other than `own`: for a window of w consecutive
 // positions containing `anchor` (w = k, plus one when `own` is excluded and
@@ -526,8 +522,8 @@ constexpr int knn_min_blocks(int kmax, int dist_bytes) { return (dist_bytes == 4
 template <typename T, int D, int KMAX, typename L>
 __global__ void __launch_bounds__(QTHREADS, knn_min_blocks(KMAX, sizeof(typename DistOf<T>::type))) k_knn(TreeView<T, D> tv, L ld, const int* order, int order_mode, int m,
                                                   int k, typename DistOf<T>::type r2, int32_t* out_idx,
-                                                  int32_t* out_cnt, int* status, SlotMap fm, int lane_span,
-                                                  bool warm_bound, int warm_mult) {
+                                                  int32_t* out_cnt, int* status, SlotMap fm, bool warm_bound,
+                                                  int warm_mult) {
   typedef typename DistOf<T>::type DistT;
   const int slot = blockIdx.x * QTHREADS + threadIdx.x;
   if ((slot & ~31) >= m) return;
@@ -549,10 +545,8 @@ __global__ void __launch_bounds__(QTHREADS, knn_min_blocks(KMAX, sizeof(typename
   top.reset(k, r2);
   int wlo = 0, wn = 0;
   if (active) warm_topk<T, D, DistT>(top, tv, fm, slot, q, anchor, k, own, r2, warm_bound, warm_mult, wlo, wn);
-  const bool ok = use_lane_walk<LANE_STACK>(anchor, active, lane_span, tv.depth)
-                      ? lane_knn<LANE_STACK, T, D>(tv, q, own, active, r2, top, wlo, wn)
-                      : wide_knn<T, D>(tv, top_node<T, D>(slot, fm, tv), q, anchor, own, active, r2, top, ws, wlo, wn);
-  if (!ok) atomicExch(status, 1);
+  if (!wide_knn<T, D>(tv, top_node<T, D>(slot, fm, tv), q, anchor, own, active, r2, top, ws, wlo, wn))
+    atomicExch(status, 1);
   if (qid >= 0) {
     int c = 0;
 #pragma unroll
@@ -576,9 +570,96 @@ void launch_knn(const TreeBase* t, L ld, const int* order, int mode, int m, int 
     PPTKG_CUDA(cudaFuncSetAttribute(k_knn<T, D, KMAX, L>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   k_knn<T, D, KMAX, L><<<div_up(m, QTHREADS), QTHREADS, smem, st>>>(view_of<T, D>(t), ld, order, mode, m, k, r2,
                                                                       d_idx, d_cnt, status, fm,
-                                                                      g_tune_lane_span.load(),
                                                                       g_tune_warm_bound.load() != 0,
                                                                       g_tune_warm_mult.load());
+  PPTKG_CHECK_LAUNCH();
+}
+
+// kNN with one warp per query (warp_knn), k <= 32 S.  Slot i0 + w (of the
+// processing order, or of a multi-tree or forest slot map) is warp w's.
+// POS: tree positions to row w, for the normal pass, instead of original
+// indices to the query's row.
+template <typename T, int D, int S, typename L, bool POS>
+__global__ void __launch_bounds__(QTHREADS) k_knn_warp(TreeView<T, D> tv, L ld, const int* order, int order_mode,
+                                                       int i0, int m, int k, typename DistOf<T>::type r2,
+                                                       int32_t* out_idx, int32_t* out_cnt, int* status, SlotMap fm) {
+  typedef typename DistOf<T>::type DistT;
+  extern __shared__ __align__(16) int2 kw_stack[];
+  const int w = blockIdx.x * QWARPS + (threadIdx.x >> 5);
+  if (w >= m) return;
+  const int lane = threadIdx.x & 31;
+  int own = -1, anchor = -1;
+  DistT q[D];
+  const int qid = fm.warp_cloud ? forest_query(i0 + w, fm, tv) : query_of(i0 + w, order, order_mode, tv);
+  if (qid < 0) return;
+  bool active = ld.load(qid, tv, q, own, &anchor);
+#pragma unroll
+  for (int d = 0; d < D; d++) active = active && q[d] == q[d];  // (no neighbours of a NaN)
+  WarpList<S, DistT> top;
+  top.reset(k, r2);
+  const int root = active ? top_node<T, D>(i0 + w, fm, tv) : -1;
+  if (root >= 0) {
+    const int home = anchor >= 0 ? min(tv.wide_of(0, min(anchor, tv.pts_cap - 1)), tv.n_wide - 1) : -1;
+    if (!warp_knn<S, T, D, DistT>(tv, root, q, home, own, r2, top, kw_stack + (threadIdx.x >> 5) * tv.wstack) &&
+        lane == 0)
+      atomicExch(status, 1);
+  }
+  const WarpKey<DistT> none = WarpKey<DistT>::none(r2);
+  const int64_t row = POS ? w : qid;
+  int n = 0;
+#pragma unroll
+  for (int s = 0; s < S; s++) {
+    const int e = 32 * s + lane;
+    const bool v = e < k && top.a[s] < none;
+    n += __popc(__ballot_sync(0xffffffffu, v));
+    if (e < k) out_idx[row * k + e] = v ? (POS ? tv.pos_of(tv.fwd, top.a[s].id()) : top.a[s].id()) : -1;
+  }
+  if (out_cnt && lane == 0) out_cnt[row] = n;
+}
+
+// Largest k of the warp lists.
+constexpr int WARP_MAX_K = 256;
+// Warp-per-query batches above this size are sorted by tree position first.
+constexpr int WARP_UNSORTED = 65536;
+
+// Whether a batch of m queries on trees of nv points runs one warp per query
+// in place of 32-query packets: beyond the packets' lists (k > 64) always;
+// otherwise a batch too small to fill the GPU with packets, or whose packets
+// would span more than lane_span tree positions on average (a third of it
+// for lists of more than 16, whose insertions packets pay for more dearly).
+// us, packets / warps, points of a scene in no order:
+//   k = 16, 2M points:  30k 375 / 166, 60k 376 / 269, 100k 418 / 375, 200k 543 / 636
+//   k = 16, 20M points: 60k 860 / 305, 200k 1075 / 750, 400k 1483 / 1365, 700k 2040 / 2249
+//   k = 32, 2M points:  60k 629 / 327, 200k 969 / 836, 400k 1526 / 1550
+//   k = 32, 20M points: 200k 1864 / 974, 1M 4703 / 4157, 2M 7743 / 8065
+//   normals, k = 16, 2M points: 10k 432 / 117, 60k 368 / 276, 100k 438 / 510
+inline bool by_warp(int64_t nv, int64_t m, int k) {
+  if (k > WARP_MAX_K) return false;
+  if (k > KNN_MAX_K) return true;
+  const int span = g_tune_lane_span.load();
+  if (span < 0) return false;
+  const int f = k > 16 ? 3 : 1;
+  return m <= 65536 || 32 * f * nv > m * span;
+}
+
+template <typename T, int D, typename L, bool POS>
+void launch_knn_warp(const TreeBase* t, L ld, const int* order, int mode, int i0, int m, int k,
+                     typename DistOf<T>::type r2, int32_t* d_idx, int32_t* d_cnt, int* status, cudaStream_t st,
+                     SlotMap fm = SlotMap{}) {
+  if (m <= 0) return;
+  const size_t smem = (size_t)QWARPS * wide_stack(t->wlevels) * sizeof(int2);
+  auto go = [&](auto kern) {
+    kern<<<div_up(m, QWARPS), QTHREADS, smem, st>>>(view_of<T, D>(t), ld, order, mode, i0, m, k, r2, d_idx, d_cnt,
+                                                    status, fm);
+  };
+  if (k <= 32)
+    go(k_knn_warp<T, D, 1, L, POS>);
+  else if (k <= 64)
+    go(k_knn_warp<T, D, 2, L, POS>);
+  else if (k <= 128)
+    go(k_knn_warp<T, D, 4, L, POS>);
+  else
+    go(k_knn_warp<T, D, 8, L, POS>);
   PPTKG_CHECK_LAUNCH();
 }
 
@@ -667,7 +748,7 @@ template <typename T, int D, typename L>
 void launch_knn_big(const TreeBase* t, L ld, const int* order, int mode, int m, int k, typename DistOf<T>::type r2,
                     int32_t* d_idx, int32_t* d_cnt, int* status, cudaStream_t st) {
   typedef typename DistOf<T>::type DistT;
-  if (t->tdepth > BIG_STACK) throw Error(E_UNSUPPORTED, "k > 64 on a tree deeper than 128 levels");
+  if (t->tdepth > BIG_STACK) throw Error(E_UNSUPPORTED, "k > 256 on a tree deeper than 128 levels");
   const size_t per_query = (size_t)k * (sizeof(DistT) + sizeof(int));
   const int chunk = (int)std::max<size_t>(1, std::min<size_t>((size_t)m, ((size_t)2 << 30) / per_query));
   DevBuf<DistT> hd((size_t)chunk * k, st);
@@ -689,41 +770,34 @@ void knn_query(const TreeBase* t, const QuerySpec& qs, int k, double dmax, int32
   if (m <= 0) return;
   DevBuf<int> status(1, st);
   PPTKG_CUDA(cudaMemsetAsync(status.get(), 0, sizeof(int), st));
-  DevBuf<int> order, anchors(qs.pts ? m : 0, st);
-  const int mode = make_order<T, D>(t, qs, order, st, false, anchors.get());
+  const bool warps = by_warp(t->nv, m, k);
+  const bool sorted = !warps || m > WARP_UNSORTED;
+  DevBuf<int> order, anchors(qs.pts && sorted ? m : 0, st);
+  int mode = 0;
+  if (sorted)
+    mode = make_order<T, D>(t, qs, order, st, false, anchors.get());
+  else
+    check_indices(t, qs, st);
   const DistT r2 = radius2<DistT>(dmax);
   Stage stage("knn", st);
-  if (k > KNN_MAX_K) {
-    if (qs.pts) {
-      if (qs.qdtype == F64)
-        launch_knn_big<T, D>(t, PointQueries<double, D>{(const double*)qs.pts}, order.get(), mode, m, k, r2, d_idx,
-                             d_cnt, status.get(), st);
-      else
-        launch_knn_big<T, D>(t, PointQueries<float, D>{(const float*)qs.pts}, order.get(), mode, m, k, r2, d_idx,
-                             d_cnt, status.get(), st);
-    } else if (qs.exclude_self) {
-      launch_knn_big<T, D>(t, IndexQueries<D, true>{qs.idx, t->fwd}, order.get(), mode, m, k, r2, d_idx, d_cnt,
-                           status.get(), st);
-    } else {
-      launch_knn_big<T, D>(t, IndexQueries<D, false>{qs.idx, t->fwd}, order.get(), mode, m, k, r2, d_idx, d_cnt,
-                           status.get(), st);
-    }
-    check_status(status.get(), st, "knn");
-    return;
-  }
+  auto run = [&](auto ld) {
+    typedef decltype(ld) L;
+    if (warps)
+      launch_knn_warp<T, D, L, false>(t, ld, order.get(), mode, 0, m, k, r2, d_idx, d_cnt, status.get(), st);
+    else if (k > KNN_MAX_K)
+      launch_knn_big<T, D>(t, ld, order.get(), mode, m, k, r2, d_idx, d_cnt, status.get(), st);
+    else
+      dispatch_knn<T, D>(t, ld, order.get(), mode, m, k, r2, d_idx, d_cnt, status.get(), st);
+  };
   if (qs.pts) {
     if (qs.qdtype == F64)
-      dispatch_knn<T, D>(t, PointQueries<double, D>{(const double*)qs.pts, anchors.get()}, order.get(), mode, m, k,
-                         r2, d_idx, d_cnt, status.get(), st);
+      run(PointQueries<double, D>{(const double*)qs.pts, anchors.get()});
     else
-      dispatch_knn<T, D>(t, PointQueries<float, D>{(const float*)qs.pts, anchors.get()}, order.get(), mode, m, k, r2,
-                         d_idx, d_cnt, status.get(), st);
+      run(PointQueries<float, D>{(const float*)qs.pts, anchors.get()});
   } else if (qs.exclude_self) {
-    dispatch_knn<T, D>(t, IndexQueries<D, true>{qs.idx, t->fwd}, order.get(), mode, m, k, r2, d_idx, d_cnt,
-                       status.get(), st);
+    run(IndexQueries<D, true>{qs.idx, t->fwd});
   } else {
-    dispatch_knn<T, D>(t, IndexQueries<D, false>{qs.idx, t->fwd}, order.get(), mode, m, k, r2, d_idx, d_cnt,
-                       status.get(), st);
+    run(IndexQueries<D, false>{qs.idx, t->fwd});
   }
   check_status(status.get(), st, "knn");
 }
@@ -1123,6 +1197,32 @@ constexpr int normals_min_blocks(int kmax, int dist_bytes, int prec) {
   return b < 1 ? 1 : (b > 8 ? 8 : b);
 }
 
+// Covariance, eigensolve and output of one query's neighbourhood (tree
+// positions lane_log[32 j], j < n).
+template <typename T, int KMAX, int PREC, typename DistT>
+__device__ __forceinline__ void normals_tail(const TreeView<T, 3>& tv, const int* lane_log, int n, const DistT* q,
+                                             int qid, int grp, int num_eigen, double gap_thr, T* evecs, T* evals,
+                                             int32_t* sizes, int* fix, int* nfix) {
+  if (PREC == PREC_FP64) {
+    Sym3<double> C = log_covariance<T, double, DistT>(tv, lane_log, n, q);
+    double w[3], V[9];
+    eigh3<double>(C, w, V);
+    write_pca<T, double>(qid, n, w, V, num_eigen, evecs, evals, sizes);
+  } else {
+    Sym3<float> C = log_covariance<T, float, DistT>(tv, lane_log, n, q);
+    float w[3], V[9];
+    eigh3<float>(C, w, V);
+    write_pca<T, float>(qid, n, w, V, num_eigen, evecs, evals, sizes);
+    if (fix && n > 0 && !(rel_gap<float>(w) >= (float)gap_thr)) {
+      // queue [query, count, neighbour positions] for the FP64 re-solve
+      int* e = fix + (int64_t)atomicAdd(nfix, 1) * (KMAX + 2);
+      e[0] = qid;
+      e[1] = n | (grp << 8);
+      for (int j = 0; j < n; j++) e[2 + j] = lane_log[j * 32];
+    }
+  }
+}
+
 // Fused kNN + PCA.  In the FP32 precision mode a neighbourhood whose two
 // smallest eigenvalues nearly coincide (relative gap < gap_thr) is queued in
 // `fix` for an FP64 re-solve by a second launch of this kernel in FP64 mode.
@@ -1140,9 +1240,8 @@ __global__ void __launch_bounds__(QTHREADS, normals_min_blocks(KMAX, sizeof(type
 k_normals(TreeView<T, 3> tv, L ld, const int* order, int order_mode, int m,
                                                       int k, typename DistOf<T>::type r2, int num_eigen,
                                                       double gap_thr, T* evecs, T* evals, int32_t* sizes,
-                                                      int* fix, int* nfix, int* status, SlotMap fm, int lane_span,
-                                                      bool warm_bound, int warm_mult, int32_t* knn_idx,
-                                                      int32_t* knn_cnt) {
+                                                      int* fix, int* nfix, int* status, SlotMap fm, bool warm_bound,
+                                                      int warm_mult, int32_t* knn_idx, int32_t* knn_cnt) {
   typedef typename DistOf<T>::type DistT;
   constexpr int LOGCAP = normals_logcap(KMAX);
   const int slot = blockIdx.x * QTHREADS + threadIdx.x;
@@ -1166,10 +1265,8 @@ k_normals(TreeView<T, 3> tv, L ld, const int* order, int order_mode, int m,
   top.reset(k, r2);
   int wlo = 0, wn = 0;
   if (active) warm_topk<T, 3, DistT>(top, tv, fm, slot, q, anchor, k, own, r2, warm_bound, warm_mult, wlo, wn);
-  const bool ok = use_lane_walk<LANE_STACK>(anchor, active, lane_span, tv.depth)
-                      ? lane_knn<LANE_STACK, T, 3>(tv, q, own, active, r2, top, wlo, wn)
-                      : wide_knn<T, 3>(tv, top_node<T, 3>(slot, fm, tv), q, anchor, own, active, r2, top, ws, wlo, wn);
-  if (!ok) atomicExch(status, 1);
+  if (!wide_knn<T, 3>(tv, top_node<T, 3>(slot, fm, tv), q, anchor, own, active, r2, top, ws, wlo, wn))
+    atomicExch(status, 1);
   if (qid < 0) return;
   if (!active) {
     write_invalid<T>(qid, num_eigen, evecs, evals, sizes);
@@ -1209,24 +1306,98 @@ k_normals(TreeView<T, 3> tv, L ld, const int* order, int order_mode, int m,
     for (int j = KMAX - 1; j >= 0; j--)
       if (j < k && top.valid(j)) lane_log[(n++) * 32] = tv.pos_of(tv.fwd, top.id(j));
   }
-  if (PREC == PREC_FP64) {
-    Sym3<double> C = log_covariance<T, double, DistT>(tv, lane_log, n, q);
-    double w[3], V[9];
-    eigh3<double>(C, w, V);
-    write_pca<T, double>(qid, n, w, V, num_eigen, evecs, evals, sizes);
-  } else {
-    Sym3<float> C = log_covariance<T, float, DistT>(tv, lane_log, n, q);
-    float w[3], V[9];
-    eigh3<float>(C, w, V);
-    write_pca<T, float>(qid, n, w, V, num_eigen, evecs, evals, sizes);
-    if (fix && n > 0 && !(rel_gap<float>(w) >= (float)gap_thr)) {
-      // queue [query, count, neighbour positions] for the FP64 re-solve
-      int* e = fix + (int64_t)atomicAdd(nfix, 1) * (KMAX + 2);
-      e[0] = qid;
-      e[1] = n | (grp << 8);
-      for (int j = 0; j < n; j++) e[2 + j] = lane_log[j * 32];
-    }
+  normals_tail<T, KMAX, PREC>(tv, lane_log, n, q, qid, grp, num_eigen, gap_thr, evecs, evals, sizes, fix, nfix);
+}
+
+// The normals of k_normals for batches too small, or queries too far apart,
+// for packets: a warp answers `per` queries (1 .. 32, a power of two) one
+// after the other (warp_knn), lane g keeping the g-th neighbourhood, and then
+// solves them side by side.
+template <typename T, int KMAX, typename L, int PREC>
+__global__ void __launch_bounds__(QTHREADS) k_normals_warp(TreeView<T, 3> tv, L ld, const int* order, int order_mode,
+                                                           int m, int per, int k, typename DistOf<T>::type r2,
+                                                           int num_eigen, double gap_thr, T* evecs, T* evals,
+                                                           int32_t* sizes, int* fix, int* nfix, int* status,
+                                                           SlotMap fm, int32_t* knn_idx, int32_t* knn_cnt) {
+  typedef typename DistOf<T>::type DistT;
+  typedef WarpKey<DistT> Key;
+  constexpr int S = KMAX > 32 ? 2 : 1;
+  const int lane = threadIdx.x & 31;
+  const unsigned FULL = 0xffffffffu;
+  const int first = (blockIdx.x * QWARPS + (threadIdx.x >> 5)) * per;
+  if (first >= m) return;
+  int qid = -1, own = -1, grp = 0, anchor = -1;
+  DistT q[3] = {(DistT)0, (DistT)0, (DistT)0};
+  bool active = false;
+  const int slot = first + lane;
+  if (fm.warp_cloud) {
+    grp = fm.views ? fm.warp_cloud[first >> 5] : 0;
+    const int row = forest_query(lane < per ? slot : first, fm, tv);  // (one tree for the warp)
+    if (lane < per) qid = row;
+  } else if (lane < per && slot < m) {
+    qid = query_of(slot, order, order_mode, tv);
   }
+  if (qid >= 0) active = ld.load(qid, tv, q, own, &anchor);
+  const bool number = q[0] == q[0] && q[1] == q[1] && q[2] == q[2];
+  // per warp: the stack, then the neighbour positions, strided by lane
+  extern __shared__ __align__(16) int2 kw_stack[];
+  const size_t each = tv.wstack + (size_t)KMAX * 16;
+  int2* stk = kw_stack + (threadIdx.x >> 5) * each;
+  int* log = reinterpret_cast<int*>(stk + tv.wstack);
+  const int root = top_node<T, 3>(first, fm, tv);
+  int n = 0;
+  for (unsigned rest = __ballot_sync(FULL, active); rest; rest &= rest - 1) {
+    const int g = __ffs(rest) - 1;
+    DistT qg[3];
+#pragma unroll
+    for (int d = 0; d < 3; d++) qg[d] = __shfl_sync(FULL, q[d], g);
+    const int id = __shfl_sync(FULL, qid, g), mine = __shfl_sync(FULL, own, g), anc = __shfl_sync(FULL, anchor, g);
+    WarpList<S, DistT> top;
+    top.reset(k, r2);
+    if (root >= 0 && __shfl_sync(FULL, (int)number, g)) {
+      const int home = anc >= 0 ? min(tv.wide_of(0, min(anc, tv.pts_cap - 1)), tv.n_wide - 1) : -1;
+      if (!warp_knn<S, T, 3, DistT>(tv, root, qg, home, mine, r2, top, stk) && lane == 0) atomicExch(status, 1);
+    }
+    const Key none = Key::none(r2);
+    int found = 0, before = 0;
+#pragma unroll
+    for (int s = 0; s < S; s++) {
+      const bool v = 32 * s + lane < k && top.a[s] < none;
+      found += __popc(__ballot_sync(FULL, v));
+      if constexpr (ExcludesSelf<L>::value)
+        before += __popc(__ballot_sync(FULL, v && top.a[s] < Key::make((DistT)0, id)));
+    }
+#pragma unroll
+    for (int s = 0; s < S; s++) {
+      const int e = 32 * s + lane;
+      const bool v = e < found;
+      if constexpr (ExcludesSelf<L>::value) {
+        // the query point goes in at its place, the list is cut to k
+        if (e < k) knn_idx[(int64_t)id * k + e] = v ? top.a[s].id() : -1;
+        const int at = e + (e >= before ? 1 : 0);
+        if (v && at < k) log[at * 32 + g] = tv.pos_of(tv.fwd, top.a[s].id());
+      } else if (v) {
+        log[e * 32 + g] = tv.pos_of(tv.fwd, top.a[s].id());
+      }
+    }
+    if constexpr (ExcludesSelf<L>::value) {
+      if (before < k && lane == 0) log[before * 32 + g] = mine;
+      if (knn_cnt && lane == 0) knn_cnt[id] = found;
+      found = min(found + 1, k);
+    }
+    if (lane == g) n = found;
+    __syncwarp();
+  }
+  if (qid < 0) return;
+  if (!active) {
+    write_invalid<T>(qid, num_eigen, evecs, evals, sizes);
+    if constexpr (ExcludesSelf<L>::value) {
+      for (int j = 0; j < k; j++) knn_idx[(int64_t)qid * k + j] = -1;
+      if (knn_cnt) knn_cnt[qid] = 0;
+    }
+    return;
+  }
+  normals_tail<T, KMAX, PREC>(tv, log + lane, n, q, qid, grp, num_eigen, gap_thr, evecs, evals, sizes, fix, nfix);
 }
 
 // r-near neighbourhoods (k == -1): moments accumulated during the traversal
@@ -1412,32 +1583,45 @@ __global__ void k_refine64(const PointRec<T, 3>* pts, const int* fix, const int*
 template <typename T, int KMAX, typename L, int PREC>
 void launch_normals(const TreeBase* t, L ld, const int* order, int mode, int m, int k, typename DistOf<T>::type r2,
                     int num_eigen, double gap_thr, T* ev, T* ew, int32_t* sz, int* fix, int* nfix, int* status,
-                    cudaStream_t st, SlotMap fm = SlotMap{}, int32_t* kidx = nullptr, int32_t* kcnt = nullptr) {
+                    cudaStream_t st, bool warps, SlotMap fm = SlotMap{}, int32_t* kidx = nullptr,
+                    int32_t* kcnt = nullptr) {
   if (m <= 0) return;
+  if (warps) {
+    // at least 32 warps per SM, then more queries per warp (they share the
+    // cost of its solves)
+    int per = 1;
+    while (per < 32 && m / (2 * per) >= 4736) per *= 2;
+    const size_t smem = QWARPS * (wide_stack(t->wlevels) + (size_t)KMAX * 16) * sizeof(int2);
+    k_normals_warp<T, KMAX, L, PREC><<<div_up(m, QWARPS * per), QTHREADS, smem, st>>>(
+        view_of<T, 3>(t), ld, order, mode, m, per, k, r2, num_eigen, gap_thr, ev, ew, sz, fix, nfix, status, fm, kidx,
+        kcnt);
+    PPTKG_CHECK_LAUNCH();
+    return;
+  }
   const size_t smem = QWARPS * warp_smem_bytes<T, 3>(wide_stack(t->wlevels), normals_logcap(KMAX));
   if (smem > 48 * 1024)
     PPTKG_CUDA(
         cudaFuncSetAttribute(k_normals<T, KMAX, L, PREC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   k_normals<T, KMAX, L, PREC><<<div_up(m, QTHREADS), QTHREADS, smem, st>>>(
       view_of<T, 3>(t), ld, order, mode, m, k, r2, num_eigen, gap_thr, ev, ew, sz, fix, nfix, status, fm,
-      g_tune_lane_span.load(), g_tune_warm_bound.load() != 0, g_tune_warm_mult.load(), kidx, kcnt);
+      g_tune_warm_bound.load() != 0, g_tune_warm_mult.load(), kidx, kcnt);
   PPTKG_CHECK_LAUNCH();
 }
 
 template <typename T, int KMAX, typename L>
 void normals_pass(const TreeBase* t, L ld, const int* order, int mode, int m, int k, typename DistOf<T>::type r2,
                   int num_eigen, int prec, double gap_thr, T* ev, T* ew, int32_t* sz, int* status, cudaStream_t st,
-                  SlotMap fm = SlotMap{}, int32_t* kidx = nullptr, int32_t* kcnt = nullptr) {
+                  bool warps, SlotMap fm, int32_t* kidx, int32_t* kcnt) {
   if (prec == PREC_FP64) {
     launch_normals<T, KMAX, L, PREC_FP64>(t, ld, order, mode, m, k, r2, num_eigen, gap_thr, ev, ew, sz, nullptr,
-                                          nullptr, status, st, fm, kidx, kcnt);
+                                          nullptr, status, st, warps, fm, kidx, kcnt);
     return;
   }
   // FP32 pass, then an FP64 re-solve of the queued small-gap neighbourhoods
   DevBuf<int> fix((size_t)std::max(m, 1) * (KMAX + 2), st), nfix(1, st);
   PPTKG_CUDA(cudaMemsetAsync(nfix.get(), 0, sizeof(int), st));
   launch_normals<T, KMAX, L, PREC_FP32>(t, ld, order, mode, m, k, r2, num_eigen, gap_thr, ev, ew, sz, fix.get(),
-                                        nfix.get(), status, st, fm, kidx, kcnt);
+                                        nfix.get(), status, st, warps, fm, kidx, kcnt);
   {
     Stage s("normals.refine64", st);
     k_refine64<T, KMAX><<<div_up(m, 256), 256, 0, st>>>((const PointRec<T, 3>*)t->pts, fix.get(), nfix.get(),
@@ -1450,23 +1634,23 @@ void normals_pass(const TreeBase* t, L ld, const int* order, int mode, int m, in
 template <typename T, typename L>
 void dispatch_normals(const TreeBase* t, L ld, const int* order, int mode, int m, int k,
                       typename DistOf<T>::type r2, int num_eigen, int prec, double gap_thr, T* ev, T* ew,
-                      int32_t* sz, int* status, cudaStream_t st, SlotMap fm = SlotMap{}, int32_t* kidx = nullptr,
-                      int32_t* kcnt = nullptr) {
+                      int32_t* sz, int* status, cudaStream_t st, bool warps, SlotMap fm = SlotMap{},
+                      int32_t* kidx = nullptr, int32_t* kcnt = nullptr) {
   const int kc = std::max(k, g_tune_topk_min.load());
   if (kc <= 4)
-    normals_pass<T, 4, L>(t, ld, order, mode, m, k, r2, num_eigen, prec, gap_thr, ev, ew, sz, status, st, fm, kidx,
+    normals_pass<T, 4, L>(t, ld, order, mode, m, k, r2, num_eigen, prec, gap_thr, ev, ew, sz, status, st, warps, fm, kidx,
                           kcnt);
   else if (kc <= 8)
-    normals_pass<T, 8, L>(t, ld, order, mode, m, k, r2, num_eigen, prec, gap_thr, ev, ew, sz, status, st, fm, kidx,
+    normals_pass<T, 8, L>(t, ld, order, mode, m, k, r2, num_eigen, prec, gap_thr, ev, ew, sz, status, st, warps, fm, kidx,
                           kcnt);
   else if (kc <= 16)
-    normals_pass<T, 16, L>(t, ld, order, mode, m, k, r2, num_eigen, prec, gap_thr, ev, ew, sz, status, st, fm, kidx,
+    normals_pass<T, 16, L>(t, ld, order, mode, m, k, r2, num_eigen, prec, gap_thr, ev, ew, sz, status, st, warps, fm, kidx,
                            kcnt);
   else if (kc <= 32)
-    normals_pass<T, 32, L>(t, ld, order, mode, m, k, r2, num_eigen, prec, gap_thr, ev, ew, sz, status, st, fm, kidx,
+    normals_pass<T, 32, L>(t, ld, order, mode, m, k, r2, num_eigen, prec, gap_thr, ev, ew, sz, status, st, warps, fm, kidx,
                            kcnt);
   else
-    normals_pass<T, 64, L>(t, ld, order, mode, m, k, r2, num_eigen, prec, gap_thr, ev, ew, sz, status, st, fm, kidx,
+    normals_pass<T, 64, L>(t, ld, order, mode, m, k, r2, num_eigen, prec, gap_thr, ev, ew, sz, status, st, warps, fm, kidx,
                            kcnt);
 }
 
@@ -1527,16 +1711,21 @@ template <typename T, typename L>
 void normals_big(const TreeBase* t, L ld, const int* order, int mode, int m, int k, typename DistOf<T>::type r2,
                  int num_eigen, T* ev, T* ew, int32_t* sz, int* status, cudaStream_t st) {
   typedef typename DistOf<T>::type DistT;
-  if (t->tdepth > BIG_STACK) throw Error(E_UNSUPPORTED, "k > 64 on a tree deeper than 128 levels");
+  const bool heaps = k > WARP_MAX_K;
+  if (heaps && t->tdepth > BIG_STACK) throw Error(E_UNSUPPORTED, "k > 256 on a tree deeper than 128 levels");
   const size_t per_query = (size_t)k * (sizeof(DistT) + 2 * sizeof(int)) + sizeof(int);
   const int chunk = (int)std::max<size_t>(1, std::min<size_t>((size_t)m, ((size_t)2 << 30) / per_query));
-  DevBuf<DistT> hd((size_t)chunk * k, st);
-  DevBuf<int> hp((size_t)chunk * k, st), pos((size_t)chunk * k, st), cnt(chunk, st);
+  DevBuf<DistT> hd(heaps ? (size_t)chunk * k : 0, st);
+  DevBuf<int> hp(heaps ? (size_t)chunk * k : 0, st), pos((size_t)chunk * k, st), cnt(chunk, st);
   for (int m0 = 0; m0 < m; m0 += chunk) {
     const int mc = std::min(chunk, m - m0);
-    k_knn_big<T, 3, L, true><<<div_up(mc, 128), 128, 0, st>>>(view_of<T, 3>(t), ld, order, mode, m0, mc, k, r2,
-                                                                hd.get(), hp.get(), pos.get(), cnt.get(), status);
-    PPTKG_CHECK_LAUNCH();
+    if (k <= WARP_MAX_K) {
+      launch_knn_warp<T, 3, L, true>(t, ld, order, mode, m0, mc, k, r2, pos.get(), cnt.get(), status, st);
+    } else {
+      k_knn_big<T, 3, L, true><<<div_up(mc, 128), 128, 0, st>>>(view_of<T, 3>(t), ld, order, mode, m0, mc, k, r2,
+                                                                  hd.get(), hp.get(), pos.get(), cnt.get(), status);
+      PPTKG_CHECK_LAUNCH();
+    }
     k_normals_pos<T, L><<<div_up(mc, 128), 128, 0, st>>>(view_of<T, 3>(t), ld, order, mode, m0, mc, k, pos.get(),
                                                           cnt.get(), num_eigen, ev, ew, sz);
     PPTKG_CHECK_LAUNCH();
@@ -1556,11 +1745,14 @@ void normals_query(const TreeBase* t, const QuerySpec& qs_in, int k, float r, in
   DevBuf<int> status(1, st);
   PPTKG_CUDA(cudaMemsetAsync(status.get(), 0, sizeof(int), st));
   DevBuf<int> order;
-  int mode = make_order<T, 3>(t, qs, order, st);
-  if (mode == 2) {
-    // tree order covers valid points only: rows of dropped points (none when
-    // n == nv) need no separate pass
-  }
+  // (tree order covers valid points only: rows of dropped points, none when
+  // n == nv, need no separate pass)
+  const bool warps = k > 0 && by_warp(t->nv, m, k);
+  int mode = 0;
+  if (warps && m <= WARP_UNSORTED)
+    check_indices(t, qs, st);
+  else
+    mode = make_order<T, 3>(t, qs, order, st);
   // the radius travels as a C float (estimate_normals.cpp:264) and is cast to
   // the input type (:17-22) before being squared in the distance type
   const DistT rr = (DistT)(T)r;
@@ -1591,7 +1783,7 @@ void normals_query(const TreeBase* t, const QuerySpec& qs_in, int k, float r, in
     int prec = precision;
     if (prec == PREC_AUTO) prec = sizeof(T) == 4 ? PREC_FP32 : PREC_FP64;
     dispatch_normals<T, IndexQueries<3, false>>(t, ld, order.get(), mode, m, k, r2, num_eigen, prec, gap_thr, d_evecs,
-                                                d_evals, d_sizes, status.get(), st);
+                                                d_evals, d_sizes, status.get(), st, warps);
   }
   check_status(status.get(), st, "normals");
 }
@@ -1715,12 +1907,17 @@ void forest_knn(const TreeBase* t, int k, double dmax, bool exclude_self, int32_
   StatusWord status(st);
   const DistT r2 = radius2<DistT>(dmax);
   Stage stage("forest.knn", st);
+  auto run = [&](auto ld) {
+    if (by_warp(n_slots, n_slots, k))
+      launch_knn_warp<T, D, decltype(ld), false>(t, ld, nullptr, 0, 0, (int)n_slots, k, r2, d_idx, d_cnt,
+                                                 status.get(), st, fm);
+    else
+      dispatch_knn<T, D>(t, ld, nullptr, 0, (int)n_slots, k, r2, d_idx, d_cnt, status.get(), st, fm);
+  };
   if (exclude_self)
-    dispatch_knn<T, D>(t, IndexQueries<D, true>{nullptr, t->fwd}, nullptr, 0, (int)n_slots, k, r2, d_idx, d_cnt,
-                       status.get(), st, fm);
+    run(IndexQueries<D, true>{nullptr, t->fwd});
   else
-    dispatch_knn<T, D>(t, IndexQueries<D, false>{nullptr, t->fwd}, nullptr, 0, (int)n_slots, k, r2, d_idx, d_cnt,
-                       status.get(), st, fm);
+    run(IndexQueries<D, false>{nullptr, t->fwd});
   status.check(st, "forest knn");
 }
 
@@ -1759,14 +1956,14 @@ void forest_normals(const TreeBase* t, int k, float r, int num_eigen, int precis
     Stage stage("forest.knn_normals", st);
     dispatch_normals<T, IndexQueries<3, true>>(t, IndexQueries<3, true>{nullptr, t->fwd}, nullptr, 0, (int)n_slots,
                                                k, r2, num_eigen, prec, gap_thr, d_evecs, d_evals, d_sizes,
-                                               status.get(), st, fm, d_idx, d_cnt);
+                                               status.get(), st, by_warp(n_slots, n_slots, k), fm, d_idx, d_cnt);
     status.check(st, "forest kNN + normals");
     return;
   }
   Stage stage("forest.normals", st);
   dispatch_normals<T, IndexQueries<3, false>>(t, IndexQueries<3, false>{nullptr, t->fwd}, nullptr, 0, (int)n_slots,
                                               k, r2, num_eigen, prec, gap_thr, d_evecs, d_evals, d_sizes, status.get(),
-                                              st, fm);
+                                              st, by_warp(n_slots, n_slots, k), fm);
   status.check(st, "forest normals");
 }
 
@@ -1794,6 +1991,7 @@ struct MultiTables {
   bool ordered = false;
   int64_t n_slots = 0;
   int depth = 0, n_nodes = 0, wlevels = 0;
+  int64_t nv = 0;  // points of the trees asked
   SlotMap map() const {
     return SlotMap{warp_tree, slot_off, nullptr, nullptr, views, row_off, ordered ? order.get() : nullptr};
   }
@@ -1814,6 +2012,7 @@ void multi_tables(const TreeBase* const* trees, int ntrees, const int64_t* rows,
     mt.wlevels = std::max(mt.wlevels, t->wlevels);
     const int64_t m = rows[g + 1] - rows[g];
     if (m < 0) throw Error(E_INVALID, "query offsets must not decrease");
+    if (m > 0) mt.nv += t->nv;
     so[g + 1] = so[g] + (m + 31) / 32 * 32;
   }
   mt.n_slots = so[ntrees];
@@ -1895,24 +2094,31 @@ void multi_knn(const TreeBase* const* trees, int ntrees, const void* d_q, int qd
   multi_tables<T, D>(trees, ntrees, rows, mt, st);
   if (mt.n_slots == 0) return;
   const size_t qbytes = (qdtype == F64 ? sizeof(double) : sizeof(float)) * D;
-  multi_order<T, D>(trees, ntrees, rows, mt, [&](int g) {
-    QuerySpec qs;
-    qs.pts = (const char*)d_q + rows[g] * qbytes;
-    qs.qdtype = qdtype;
-    qs.m = rows[g + 1] - rows[g];
-    return qs;
-  }, st, true);
+  const bool warps = by_warp(mt.nv, rows[ntrees], k);
+  if (!warps || rows[ntrees] > WARP_UNSORTED)
+    multi_order<T, D>(trees, ntrees, rows, mt, [&](int g) {
+      QuerySpec qs;
+      qs.pts = (const char*)d_q + rows[g] * qbytes;
+      qs.qdtype = qdtype;
+      qs.m = rows[g + 1] - rows[g];
+      return qs;
+    }, st, true);
   std::unique_ptr<TreeBase> bt(bounds_tree(mt.depth, mt.n_nodes, mt.wlevels));
   DevBuf<int> status(1, st);
   PPTKG_CUDA(cudaMemsetAsync(status.get(), 0, sizeof(int), st));
   const DistT r2 = radius2<DistT>(dmax);
   Stage stage("multi.knn", st);
+  auto run = [&](auto ld) {
+    if (warps)
+      launch_knn_warp<T, D, decltype(ld), false>(bt.get(), ld, nullptr, 0, 0, (int)mt.n_slots, k, r2, d_idx, d_cnt,
+                                                 status.get(), st, mt.map());
+    else
+      dispatch_knn<T, D>(bt.get(), ld, nullptr, 0, (int)mt.n_slots, k, r2, d_idx, d_cnt, status.get(), st, mt.map());
+  };
   if (qdtype == F64)
-    dispatch_knn<T, D>(bt.get(), PointQueries<double, D>{(const double*)d_q, mt.anchor.get()}, nullptr, 0,
-                       (int)mt.n_slots, k, r2, d_idx, d_cnt, status.get(), st, mt.map());
+    run(PointQueries<double, D>{(const double*)d_q, mt.anchor.get()});
   else
-    dispatch_knn<T, D>(bt.get(), PointQueries<float, D>{(const float*)d_q, mt.anchor.get()}, nullptr, 0,
-                       (int)mt.n_slots, k, r2, d_idx, d_cnt, status.get(), st, mt.map());
+    run(PointQueries<float, D>{(const float*)d_q, mt.anchor.get()});
   check_status(status.get(), st, "multi-tree knn");
 }
 
@@ -1928,13 +2134,15 @@ void multi_normals(const TreeBase* const* trees, int ntrees, const int32_t* d_id
   if (mt.n_slots == 0) return;
   // query indices are checked against their own tree's rows by the kernels
   // (status 4); the ordering pass maps bad ones to the end of the order
-  multi_order<T, 3>(trees, ntrees, rows, mt, [&](int g) {
-    QuerySpec qs;
-    qs.idx = d_idx + rows[g];
-    qs.m = rows[g + 1] - rows[g];
-    qs.exclude_self = false;
-    return qs;
-  }, st);
+  const bool warps = by_warp(mt.nv, rows[ntrees], k);
+  if (!warps || rows[ntrees] > WARP_UNSORTED)
+    multi_order<T, 3>(trees, ntrees, rows, mt, [&](int g) {
+      QuerySpec qs;
+      qs.idx = d_idx + rows[g];
+      qs.m = rows[g + 1] - rows[g];
+      qs.exclude_self = false;
+      return qs;
+    }, st);
   std::unique_ptr<TreeBase> bt(bounds_tree(mt.depth, mt.n_nodes, mt.wlevels));
   DevBuf<int> status(1, st);
   PPTKG_CUDA(cudaMemsetAsync(status.get(), 0, sizeof(int), st));
@@ -1945,7 +2153,7 @@ void multi_normals(const TreeBase* const* trees, int ntrees, const int32_t* d_id
   // fwd comes from each warp's TreeView (null here)
   dispatch_normals<T, IndexQueries<3, false>>(bt.get(), IndexQueries<3, false>{d_idx, nullptr, status.get()}, nullptr,
                                               0, (int)mt.n_slots, k, r2, num_eigen, prec, gap_thr, d_evecs, d_evals,
-                                              d_sizes, status.get(), st, mt.map());
+                                              d_sizes, status.get(), st, warps, mt.map());
   check_status(status.get(), st, "multi-tree normals");
 }
 
@@ -1999,16 +2207,17 @@ static void normals_noalloc_k(const TreeBase* t, const int32_t* idx, int m, int 
   typedef IndexQueries<3, false> L;
   L ld{idx, t->fwd};
   const int mode = (!idx && m == t->nv && t->n == t->nv) ? 2 : 0;
+  const bool warps = by_warp(t->nv, m, k);
   int* status = scratch;
   int* nfix = scratch + 1;
   int* fix = scratch + NOALLOC_QUEUE_OFFSET;
   if (prec == PREC_FP64) {
     launch_normals<T, KMAX, L, PREC_FP64>(t, ld, nullptr, mode, m, k, r2, num_eigen, 0.0, ev, ew, sz, nullptr,
-                                          nullptr, status, st);
+                                          nullptr, status, st, warps);
     return;
   }
   launch_normals<T, KMAX, L, PREC_FP32>(t, ld, nullptr, mode, m, k, r2, num_eigen, 1e-3, ev, ew, sz, fix, nfix,
-                                        status, st);
+                                        status, st, warps);
   k_refine64<T, KMAX><<<div_up(m, 256), 256, 0, st>>>((const PointRec<T, 3>*)t->pts, fix, nfix, num_eigen, ev, ew,
                                                       sz, nullptr);
   PPTKG_CHECK_LAUNCH();
