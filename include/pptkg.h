@@ -306,11 +306,12 @@ PPTKG_API int64_t pptkg_launch_count(void);
  *     not depend on it.
  *   "rnear_warp_queries": pptkg_rnear_count / pptkg_rnear_fill calls, and
  *     normals over r-near neighbourhoods (k = -1), with at most this many
- *     queries give each query a whole warp (the lanes split every bucket)
- *     instead of packing 32 queries into a warp (0: never).
- *     Default 262144 (below it, 32-query packets leave B200's 148 SMs short
- *     of warps).  Hit lists and neighbourhood sizes do not depend on it;
- *     normals agree to FP64 rounding (their sums add in another order).
+ *     queries, or whose packets would span more than 512 tree positions,
+ *     give each query a whole warp (the lanes split every bucket) instead of
+ *     packing 32 queries into a warp (0: never).  Default 262144 (below it,
+ *     32-query packets leave B200's 148 SMs short of warps).  Hit lists and
+ *     neighbourhood sizes do not depend on it; normals agree to FP64
+ *     rounding (their sums add in another order).
  *   "warm_bound": kNN / normals lists start from the k tree positions
  *     around each query's anchor; with 1 their bound is also lowered to the
  *     k-th distance over a wider window of tree-order neighbours (fewer

@@ -948,7 +948,8 @@ __global__ void __launch_bounds__(SUB_THREADS) k_subtree(const Seg<T, D>* small,
 
 // ------------------------------------------------------- finishing ----
 template <typename T, int D>
-__global__ void k_finish(SoA<T, D> soa, int nv, PointRec<T, D>* pts, int* fwd, const int64_t* nv_dev = nullptr) {
+__global__ void k_finish(SoA<T, D> soa, int nv, PointRec<T, D>* pts, int* fwd, int* ids,
+                         const int64_t* nv_dev = nullptr) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (nv_dev) nv = (int)*nv_dev;  // capture mode: the valid count is on the device
   if (i >= nv) return;
@@ -957,6 +958,7 @@ __global__ void k_finish(SoA<T, D> soa, int nv, PointRec<T, D>* pts, int* fwd, c
   for (int d = 0; d < D; d++) r.c[d] = soa.x[d][i];
   r.id = soa.id[i];
   pts[i] = r;
+  ids[i] = r.id;
   fwd[r.id] = i;
 }
 
@@ -1103,7 +1105,7 @@ struct WideMap {
 // reported, and children beyond it are cut off.
 template <typename T, int D>
 __device__ __forceinline__ void wide_write(const Rec<T, D>& r, int j, const WideMap& m,
-                                           WNode<typename WalkOf<T>::type, D>* nodes, int* status) {
+                                           WNode<typename WalkOf<T>::type, D>* nodes, int2* span, int* status) {
   typedef typename WalkOf<T>::type V;
   if (r.end <= r.begin || !m.starts(j, r.begin)) return;
   const int i = m.of(j, r.begin);
@@ -1124,24 +1126,25 @@ __device__ __forceinline__ void wide_write(const Rec<T, D>& r, int j, const Wide
     w.cnt = -max(min(m.of(j - 1, r.end - 1) + 1, i) - w.begin, 0);
   }
   nodes[i] = w;
+  span[i] = make_int2(r.begin, r.end - r.begin);
 }
 
 template <typename T, int D>
 __global__ void k_wide_fill(const Rec<T, D>* recs, int n_recs, int bucket, const int* root_rec, int ncloud, WideMap m,
-                            WNode<typename WalkOf<T>::type, D>* nodes, const int* n_dev = nullptr,
+                            WNode<typename WalkOf<T>::type, D>* nodes, int2* span, const int* n_dev = nullptr,
                             int* status = nullptr) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < ncloud && root_rec[i] >= 0)
     for (int j = m.levels - 1; j >= 0; j--) {
       const int r = wide_resolve(recs, root_rec[i], wide_cap(bucket, j));
       if (wide_inner(recs[r], wide_cap(bucket, j))) break;
-      wide_write<T, D>(recs[r], j, m, nodes, status);
+      wide_write<T, D>(recs[r], j, m, nodes, span, status);
     }
   if (i >= n_recs || (n_dev && i >= *n_dev)) return;
   for (int j = 0; j < m.levels && wide_inner(recs[i], wide_cap(bucket, j)); j++)
     for (int c = 0; c < 2; c++) {
       const int r = wide_resolve(recs, c ? recs[i].right : recs[i].left, wide_cap(bucket, j));
-      if (!wide_inner(recs[r], wide_cap(bucket, j))) wide_write<T, D>(recs[r], j, m, nodes, status);
+      if (!wide_inner(recs[r], wide_cap(bucket, j))) wide_write<T, D>(recs[r], j, m, nodes, span, status);
     }
 }
 
@@ -1174,9 +1177,12 @@ void wide_begin(TreeBase* t, int n_recs, cudaStream_t st, const int* n_dev = nul
 template <typename T, int D>
 void wide_alloc(TreeBase* t, int n_wide, cudaStream_t st) {
   if (t->wide) dev_free(t->wide, st);
+  if (t->wspan) dev_free(t->wspan, st);
   t->wide = nullptr;
+  t->wspan = nullptr;
   t->n_wide = n_wide;
   PPTKG_CUDA(dev_malloc(&t->wide, (size_t)std::max(n_wide, 1) * sizeof(WNode<typename WalkOf<T>::type, D>), st));
+  PPTKG_CUDA(dev_malloc((void**)&t->wspan, (size_t)std::max(n_wide, 1) * sizeof(int2), st));
 }
 
 // Fills the nodes; `clear`: entries that no record fills hold nothing.
@@ -1185,16 +1191,34 @@ void wide_fill(TreeBase* t, int n_recs, bool clear, cudaStream_t st, const int* 
                int* status = nullptr) {
   typedef WNode<typename WalkOf<T>::type, D> Node;
   if (t->n_wide <= 0) return;
-  if (clear) PPTKG_CUDA(cudaMemsetAsync(t->wide, 0, sizeof(Node) * (size_t)t->n_wide, st));
+  if (clear) {
+    PPTKG_CUDA(cudaMemsetAsync(t->wide, 0, sizeof(Node) * (size_t)t->n_wide, st));
+    PPTKG_CUDA(cudaMemsetAsync(t->wspan, 0, sizeof(int2) * (size_t)t->n_wide, st));
+  }
   const WideMap m{t->wbits, t->wrank, t->wwords, t->wlevels, t->n_wide};
   k_wide_fill<T, D><<<div_up(std::max(n_recs, t->ncloud), 256), 256, 0, st>>>(
-      (const Rec<T, D>*)t->recs, n_recs, t->bucket, t->root_rec, t->ncloud, m, (Node*)t->wide, n_dev, status);
+      (const Rec<T, D>*)t->recs, n_recs, t->bucket, t->root_rec, t->ncloud, m, (Node*)t->wide, t->wspan,
+      n_dev, status);
   PPTKG_CHECK_LAUNCH();
+}
+
+template <typename V, int D>
+__global__ void k_ids(const PointRec<V, D>* pts, int64_t nv, int* ids) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < nv) ids[i] = pts[i].id;
 }
 
 template <typename T, int D>
 void make_wide(TreeBase* t, cudaStream_t st) {
   int n = 0;
+  if (!t->ids) {
+    typedef typename WalkOf<T>::type V;
+    PPTKG_CUDA(dev_malloc((void**)&t->ids, std::max<int64_t>(t->nv, 1) * sizeof(int), st));
+    if (t->nv > 0) {
+      k_ids<V, D><<<div_up(t->nv, 256), 256, 0, st>>>((const PointRec<V, D>*)t->pts, t->nv, t->ids);
+      PPTKG_CHECK_LAUNCH();
+    }
+  }
   wide_begin<T, D>(t, t->n_recs, st);
   PPTKG_CUDA(cudaMemcpyAsync(&n, t->wrank + (int64_t)t->wlevels * t->wwords, sizeof(int), cudaMemcpyDeviceToHost, st));
   PPTKG_CUDA(cudaStreamSynchronize(st));
@@ -1468,9 +1492,10 @@ TreeBase* build_forest(const T* d_in, int64_t n, const int64_t* orig_off_h, int 
   PPTKG_CUDA(dev_malloc((void**)&pts, std::max<int64_t>(nv, 1) * sizeof(PointRec<T, D>), st));
   tree->pts = pts;
   PPTKG_CUDA(dev_malloc((void**)&tree->fwd, std::max<int64_t>(n, 1) * sizeof(int), st));
+  PPTKG_CUDA(dev_malloc((void**)&tree->ids, std::max<int64_t>(nv, 1) * sizeof(int), st));
   if (n > 0) PPTKG_CUDA(cudaMemsetAsync(tree->fwd, 0xff, n * sizeof(int), st));
   if (nv > 0) {
-    k_finish<T, D><<<div_up(nv, 256), 256, 0, st>>>(soa, nv, pts, tree->fwd);
+    k_finish<T, D><<<div_up(nv, 256), 256, 0, st>>>(soa, nv, pts, tree->fwd, tree->ids);
     PPTKG_CHECK_LAUNCH();
   }
 
@@ -1613,6 +1638,7 @@ void forest_capture_ready(TreeBase* t, cudaStream_t st) {
     *p = q;
   };
   grow(&t->pts, (size_t)t->nv * sizeof(PointRec<T, D>), (size_t)n * sizeof(PointRec<T, D>));
+  grow((void**)&t->ids, (size_t)t->nv * sizeof(int), (size_t)n * sizeof(int));
   grow(&t->recs, (size_t)t->n_recs * sizeof(Rec<T, D>), (size_t)t->cap_recs * sizeof(Rec<T, D>));
   grow(&t->tnodes, (size_t)t->n_tnodes * sizeof(TNode<T, D>), (size_t)t->cap_tnodes * sizeof(TNode<T, D>));
   t->n_tnodes = (int)t->cap_tnodes;
@@ -1716,7 +1742,7 @@ void rebuild_forest(TreeBase* t, const T* d_in, cudaStream_t st, int* status) {
   if (n > 0) {
     PPTKG_CUDA(cudaMemsetAsync(t->fwd, 0xff, n * sizeof(int), st));
     k_finish<T, D><<<div_up(n, 256), 256, 0, st>>>(soa, (int)n, (PointRec<T, D>*)t->pts, t->fwd,
-                                                   t->valid_off + ncloud);
+                                                   t->ids, t->valid_off + ncloud);
     PPTKG_CHECK_LAUNCH();
   }
   // traversal hierarchy over the live records
@@ -1784,6 +1810,8 @@ TreeBase::~TreeBase() {
   if (tnodes) dev_free(tnodes, stream);
   if (fwd) dev_free(fwd, stream);
   if (wide) dev_free(wide, stream);
+  if (wspan) dev_free(wspan, stream);
+  if (ids) dev_free(ids, stream);
   if (wbits) dev_free(wbits, stream);
   if (wrank) dev_free(wrank, stream);
   if (root_rec) dev_free(root_rec, stream);

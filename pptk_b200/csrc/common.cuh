@@ -49,8 +49,8 @@ extern std::atomic<long long> g_launches;
 //    than this many tree positions on average run one warp per query, as do
 //    small batches (-1: never).
 extern std::atomic<int> g_tune_lane_span;
-//  rnear_warp_queries: r-near batches of at most this many queries run one
-//    warp per query instead of 32-query packets (0: never).
+//  rnear_warp_queries: r-near batches of at most this many queries, or too
+//    scattered for packets, run one warp per query (0: never).
 extern std::atomic<int> g_tune_rnear_warp_queries;
 //  warm_bound: after the warm start of a kNN list, also lower its bound to
 //    the k-th distance of the 32 (k <= 16) or 3 x k tree-order neighbours

@@ -33,6 +33,8 @@ TreeView<T, D> view_of(const TreeBase* t) {
   v.n_in = (int)t->n;
   v.pts_cap = (int)(t->capture ? t->n : t->nv);
   v.wide = (const WNode<T, D>*)t->wide;
+  v.wspan = t->wspan;
+  v.ids = t->ids;
   v.wbits = t->wbits;
   v.wrank = t->wrank;
   v.wwords = t->wwords;
@@ -861,109 +863,119 @@ __global__ void __launch_bounds__(QTHREADS) k_rnear_fill(TreeView<T, D> tv, L ld
   if (overflow || w != wend) atomicExch(status, 2);
 }
 
-// r-near walk with one warp per query, for batches too small to fill the
-// GPU as 32-query packets (a packet lane walks its own hits one by one, so a
-// few thousand queries with 1e4-1e5 hits each leave most of the GPU idle).
-// The warp walks its query's path once, with all lanes in step, and calls
-// visit(begin, n, whole) warp-uniformly for every leaf bucket the ball
-// touches and every child box inside the ball (whole = true: all of its
-// positions are hits), positions [begin, begin + n).  Children are visited
-// left before right, so the ranges come in ascending tree position, the
-// order of the reference's left-then-right walk (kdtree-impl.h:519-558).
-// Subtree start positions are carried down the walk (a left child starts
-// where its parent does, a right child cnt[0] later) and checked against
-// every leaf reached.  visit returns false to stop the walk; the result is
-// false then, or on a corrupt tree or a full stack.
+// r-near walk with one warp per query, over the wide hierarchy.  A step tests
+// a node's children, one per lane: outside the ball, inside it (every point
+// is a hit, see box_max_dist2) or cut by it.  visit(begin, n, whole) is then
+// called warp-uniformly for tree positions [begin, begin + n) that are all
+// hits (whole) or have to be tested, in ascending position, the order of the
+// reference's left-then-right walk (kdtree-impl.h:519-558): inner nodes that
+// the ball cuts are entered before their later siblings.  Neighbouring
+// children of one kind make one call, so the short leaf ranges along the
+// ball's surface fill the lanes of a chunk.  visit returns false to stop; the
+// result is false then, or on a full stack or a corrupt hierarchy.
+//
+// 20,000 queries of 45k hits each on the 20M-point scene (r = 0.5 m), count
+// and fill: 7.9 ms with a walk of the binary hierarchy and ids read from the
+// point records, 3.3 ms so (3.6 GB of hits; 1.1 TB/s).
 template <typename T, int D, typename DistT, typename Visit>
-__device__ __forceinline__ bool warp_rnear_walk(const TreeView<T, D>& tv, const DistT* q, DistT r2, int* stk,
-                                                int stack_ints, Visit visit) {
+__device__ __forceinline__ bool warp_rnear_walk(const TreeView<T, D>& tv, int root, const DistT* q, DistT r2,
+                                                int4* stk, Visit visit) {
   const int lane = threadIdx.x & 31;
-  bool bad = false;
-  // child c of nd, whose positions start at cb: visits it, or returns the
-  // inner node to descend into (-1: nothing to descend into)
-  auto take = [&](const TNode<T, D>& nd, int c, int cb) -> int {
-    const int n = nd.cnt[c];
-    if (n == 0 || !(box_min_dist2<T, DistT, D>(nd.lo[c], nd.hi[c], q) < r2)) return -1;
-    if (box_max_dist2<T, DistT, D>(nd.lo[c], nd.hi[c], q) < r2) {
-      if (!visit(cb, n, true)) bad = true;
-      return -1;
+  const unsigned FULL = 0xffffffffu;
+  if (root < 0) return true;
+  int sp = 0, steps = 0;
+  int at = root, cnt = 1;  // siblings of this step
+  unsigned todo = 0, inside = 0;
+  bool fresh = true;
+  while (true) {
+    if (++steps > 2 * tv.n_wide + 2) return false;
+    if (fresh && cnt > 32) {
+      // the rest of the siblings comes after these
+      if (sp >= tv.wstack) return false;
+      __syncwarp();
+      if (lane == 0) stk[sp] = make_int4(at + 32, cnt - 32, 0, 1);
+      sp++;
+      cnt = 32;
     }
-    if (nd.ref[c] < 0) {
-      if (-nd.ref[c] - 1 != cb || !visit(cb, n, false)) bad = true;
-      return -1;
-    }
-    return nd.ref[c];
-  };
-  int sp = 0, cur = tv.root, b = 0, visits = 0;
-  while (!bad) {
-    if (++visits > tv.n_nodes) {  // a tree is acyclic: more visits mean a corrupt node array
-      bad = true;
-      break;
-    }
-    const TNode<T, D> nd = load_node(tv.nodes, tv.node_index(cur));
-    const int b1 = b + nd.cnt[0];
-    int next = take(nd, 0, b);
-    if (next >= 0) {
-      // into the left subtree; the right child waits if the ball reaches it
-      if (nd.cnt[1] > 0 && box_min_dist2<T, DistT, D>(nd.lo[1], nd.hi[1], q) < r2) {
-        if (2 * sp + 2 > stack_ints) {
-          bad = true;
-          break;
-        }
-        __syncwarp();
-        if (lane == 0) {
-          stk[2 * sp] = cur * 2 + 1;
-          stk[2 * sp + 1] = b1;
-        }
-        __syncwarp();
-        sp++;
+    int2 span = make_int2(0, 0);
+    int first = 0, kids = 0;
+    bool hit = false, whole = false;
+    if (fresh ? lane < cnt : (todo >> lane & 1u)) {
+      const WNode<T, D> w = tv.wide[at + lane];
+      span = tv.wspan[at + lane];
+      first = w.begin;
+      kids = w.cnt > 0 ? 0 : -w.cnt;
+      if (fresh) {
+        hit = w.cnt != 0 && box_min_dist2<T, DistT, D>(w.lo, w.hi, q) < r2;
+        whole = hit && box_max_dist2<T, DistT, D>(w.lo, w.hi, q) < r2;
       }
-      cur = next;
-      continue;
     }
-    next = take(nd, 1, b1);
-    if (next >= 0) {
-      cur = next;
-      b = b1;
-      continue;
+    if (fresh) {
+      todo = __ballot_sync(FULL, hit);
+      inside = __ballot_sync(FULL, whole);
     }
-    bool found = false;
-    while (sp > 0 && !bad) {
-      --sp;
-      const int e = stk[2 * sp], eb = stk[2 * sp + 1];
-      const int r = take(load_node(tv.nodes, tv.node_index(e >> 1)), e & 1, eb);
-      if (r >= 0) {
-        cur = r;
-        b = eb;
-        found = true;
+    // ranges: whole nodes, and leaf ranges that the ball cuts
+    const unsigned leaf = __ballot_sync(FULL, kids == 0);
+    int next = -1;
+    while (todo) {
+      const int s = __ffs(todo) - 1;
+      const bool in = inside >> s & 1u;
+      if (!in && !(leaf >> s & 1u)) {
+        next = s;
         break;
       }
+      // the siblings from s on of the same kind
+      const unsigned kind = in ? inside : todo & ~inside & leaf;
+      const unsigned stop = ~kind & (0xffffffffu << s);
+      const int e = stop ? __ffs(stop) - 2 : 31;
+      todo &= e == 31 ? 0u : 0xffffffffu << (e + 1);
+      const int b = __shfl_sync(FULL, span.x, s), last = __shfl_sync(FULL, span.x + span.y, e);
+      if (!visit(b, last - b, in)) return false;
     }
-    if (!found) break;
+    if (next >= 0) {
+      todo &= todo - 1;
+      if (todo) {
+        if (sp >= tv.wstack) return false;
+        __syncwarp();
+        if (lane == 0) stk[sp] = make_int4(at, (int)todo, (int)inside, 0);
+        sp++;
+      }
+      const int a = __shfl_sync(FULL, first, next);
+      cnt = __shfl_sync(FULL, kids, next);
+      at = a;
+      fresh = true;
+      continue;
+    }
+    if (sp == 0) return true;
+    __syncwarp();
+    const int4 e = stk[--sp];
+    at = e.x;
+    fresh = e.w == 1;
+    cnt = fresh ? e.y : 32;
+    todo = fresh ? 0u : (unsigned)e.y;
+    inside = (unsigned)e.z;
   }
-  return !bad;
 }
 
 // r-near counts or hit lists with one warp per query (warp_rnear_walk):
-// lane j tests position base + j of each chunk of a leaf bucket, a box
-// inside the ball is taken whole (the fill reads only its ids, the count adds
-// its size), and hits are written at their ballot rank, so they come out in
-// ascending tree position: the same set and order as the packet walk.
+// positions that are hits as a whole are counted, or their ids copied, without
+// a test; of the others lane j tests position base + j of each chunk and hits
+// are written at their ballot rank, so they come out in ascending tree
+// position: the same set and order as the packet walk.
 // COUNT: counts[qid] = hits, the query's own point excluded as in
 // k_rnear_count; otherwise out[off[qid] ...] = original indices of the hits.
 template <typename T, int D, typename L, bool COUNT>
 __global__ void __launch_bounds__(QTHREADS) k_rnear_warp(TreeView<T, D> tv, L ld, const int* order, int order_mode,
-                                                         int m, typename DistOf<T>::type r2, int stack_ints,
-                                                         int64_t* counts, const int64_t* off, int32_t* out,
-                                                         int* status) {
+                                                         int m, typename DistOf<T>::type r2, int64_t* counts,
+                                                         const int64_t* off, int32_t* out, int* status) {
   typedef typename DistOf<T>::type DistT;
-  extern __shared__ __align__(16) int rw_stack[];
+  extern __shared__ __align__(16) int4 rw_stack[];
   const int w = blockIdx.x * QWARPS + (threadIdx.x >> 5);
   if (w >= m) return;
   const int lane = threadIdx.x & 31;
   const unsigned FULL = 0xffffffffu;
   const unsigned lt = (1u << lane) - 1u;
-  int* stk = rw_stack + (threadIdx.x >> 5) * stack_ints;
+  int4* stk = rw_stack + (threadIdx.x >> 5) * tv.wstack;
   const int qid = query_of(w, order, order_mode, tv);
   DistT q[D];
   int own = -1;
@@ -975,8 +987,29 @@ __global__ void __launch_bounds__(QTHREADS) k_rnear_warp(TreeView<T, D> tv, L ld
     wend = off[qid + 1];
   }
   auto visit = [&](int begin, int n, bool whole) -> bool {
-    if (COUNT && whole) {
-      cnt += n;
+    if (whole) {
+      if (COUNT) {
+        cnt += n;
+        return true;
+      }
+      // two runs of ids, before and after the query's own point
+      const int end = begin + n;
+      const bool has = own >= begin && own < end;
+      if (wp + n - (has ? 1 : 0) > wend) return false;
+      for (int part = 0; part < 2; part++) {
+        const int b = part ? (has ? own + 1 : end) : begin, e = part ? end : (has ? own : end);
+        int32_t* o = out + wp - b;
+        int p = b + lane;
+        for (; p + 96 < e; p += 128) {
+          const int i0 = tv.id_at(p), i1 = tv.id_at(p + 32), i2 = tv.id_at(p + 64), i3 = tv.id_at(p + 96);
+          o[p] = i0;
+          o[p + 32] = i1;
+          o[p + 64] = i2;
+          o[p + 96] = i3;
+        }
+        for (; p < e; p += 32) o[p] = tv.id_at(p);
+        wp += e - b;
+      }
       return true;
     }
     bool bad = false;
@@ -985,14 +1018,9 @@ __global__ void __launch_bounds__(QTHREADS) k_rnear_warp(TreeView<T, D> tv, L ld
       bool hit = false;
       int32_t id = 0;
       if (p < begin + n) {
-        if (whole) {
-          hit = p != own;
-          if (hit) id = tv.pt(p).id;
-        } else {
-          const PointRec<T, D> pr = tv.pt(p);
-          hit = point_dist2<T, DistT, D>(pr.c, q) < r2 && (COUNT || p != own);
-          id = pr.id;
-        }
+        const PointRec<T, D> pr = tv.pt(p);
+        hit = point_dist2<T, DistT, D>(pr.c, q) < r2 && (COUNT || p != own);
+        id = pr.id;
       }
       const unsigned hm = __ballot_sync(FULL, hit);
       if (COUNT) {
@@ -1010,7 +1038,11 @@ __global__ void __launch_bounds__(QTHREADS) k_rnear_warp(TreeView<T, D> tv, L ld
     }
     return !__any_sync(FULL, bad);  // warp-uniform
   };
-  const bool ok = !active || warp_rnear_walk<T, D, DistT>(tv, q, r2, stk, stack_ints, visit);
+  bool number = active;  // (no hits of a NaN)
+#pragma unroll
+  for (int d = 0; d < D; d++) number = number && q[d] == q[d];
+  const int root = number && tv.n_wide > 0 ? tv.wide_of(tv.wlevels - 1, 0) : -1;
+  const bool ok = warp_rnear_walk<T, D, DistT>(tv, root, q, r2, stk, visit);
   if (lane != 0) return;
   if (COUNT) {
     if (own >= 0 && cnt > 0) cnt -= 1;  // the point itself is always a hit when r2 > 0
@@ -1021,21 +1053,25 @@ __global__ void __launch_bounds__(QTHREADS) k_rnear_warp(TreeView<T, D> tv, L ld
   }
 }
 
-// Per-warp stack of k_rnear_warp: (child ref, start position) pairs, one per
-// level at most.
-inline int rnear_warp_stack_ints(int depth) { return (2 * (depth + 1) + 3) & ~3; }
-
 template <typename T, int D, typename L, bool COUNT>
 void launch_rnear_warp(const TreeBase* t, L ld, const int* order, int mode, int m, typename DistOf<T>::type r2,
                        int64_t* counts, const int64_t* off, int32_t* out, int* status, cudaStream_t st) {
-  const int si = rnear_warp_stack_ints(t->tdepth);
-  const size_t smem = (size_t)QWARPS * si * sizeof(int);
-  if (smem > 48 * 1024)
-    PPTKG_CUDA(cudaFuncSetAttribute(k_rnear_warp<T, D, L, COUNT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)smem));
+  const size_t smem = (size_t)QWARPS * wide_stack(t->wlevels) * sizeof(int4);
   k_rnear_warp<T, D, L, COUNT><<<div_up(m, QWARPS), QTHREADS, smem, st>>>(view_of<T, D>(t), ld, order, mode, m, r2,
-                                                                            si, counts, off, out, status);
+                                                                            counts, off, out, status);
   PPTKG_CHECK_LAUNCH();
+}
+
+// Whether an r-near batch of m queries on nv points runs one warp per query:
+// batches of at most rnear_warp_queries, and larger ones whose packets would
+// span more than 512 tree positions on average.  us, packets / warps, count
+// and fill: 300k uniform points, 300k queries of 30 hits 1362 / 1404, of 254
+// hits 2197 / 2856; 20M-point scene, 20k of 47k hits 163170 / 3302, 500k of
+// 1.8k hits 29944 / 6463, 1M of 432 hits 16005 / 7118, 2M (a span of 320) of
+// 49 hits 6519 / 7760.
+inline bool rnear_by_warp(int64_t nv, int64_t m) {
+  const int most = g_tune_rnear_warp_queries.load();
+  return m <= most || (most > 0 && 32 * nv > 512 * m);
 }
 
 template <typename T, int D, typename F>
@@ -1052,6 +1088,15 @@ void with_loader(const TreeBase* t, const QuerySpec& qs, F&& f) {
   }
 }
 
+// make_order, or (small warp-per-query batches) the queries as they come,
+// their indices checked all the same.
+template <typename T, int D>
+int ordered_unless(bool as_is, const TreeBase* t, const QuerySpec& qs, DevBuf<int>& order, cudaStream_t st) {
+  if (!as_is) return make_order<T, D>(t, qs, order, st);
+  check_indices(t, qs, st);
+  return 0;
+}
+
 template <typename T, int D>
 int64_t rnear_count(const TreeBase* t, const QuerySpec& qs, double dmax, int64_t* d_off, cudaStream_t st) {
   typedef typename DistOf<T>::type DistT;
@@ -1063,13 +1108,14 @@ int64_t rnear_count(const TreeBase* t, const QuerySpec& qs, double dmax, int64_t
   DevBuf<int> status(1, st);
   PPTKG_CUDA(cudaMemsetAsync(status.get(), 0, sizeof(int), st));
   DevBuf<int> order;
-  const int mode = make_order<T, D>(t, qs, order, st);
+  const bool warps = rnear_by_warp(t->nv, m);
+  const int mode = ordered_unless<T, D>(warps && m <= WARP_UNSORTED, t, qs, order, st);
   const DistT r2 = radius2<DistT>(dmax);
   const size_t smem = QWARPS * rnear_smem_bytes<T, D>(t->tdepth);
   Stage stage("rnear_count", st);
   with_loader<T, D>(t, qs, [&](auto ld) {
     typedef decltype(ld) L;
-    if (m <= g_tune_rnear_warp_queries.load()) {
+    if (warps) {
       launch_rnear_warp<T, D, L, true>(t, ld, order.get(), mode, m, r2, d_off, nullptr, nullptr, status.get(), st);
       return;
     }
@@ -1096,13 +1142,14 @@ void rnear_fill(const TreeBase* t, const QuerySpec& qs, double dmax, const int64
   DevBuf<int> status(1, st);
   PPTKG_CUDA(cudaMemsetAsync(status.get(), 0, sizeof(int), st));
   DevBuf<int> order;
-  const int mode = make_order<T, D>(t, qs, order, st);
+  const bool warps = rnear_by_warp(t->nv, m);
+  const int mode = ordered_unless<T, D>(warps && m <= WARP_UNSORTED, t, qs, order, st);
   const DistT r2 = radius2<DistT>(dmax);
   const size_t smem = QWARPS * rnear_smem_bytes<T, D>(t->tdepth);
   Stage stage("rnear_fill", st);
   with_loader<T, D>(t, qs, [&](auto ld) {
     typedef decltype(ld) L;
-    if (m <= g_tune_rnear_warp_queries.load()) {
+    if (warps) {
       launch_rnear_warp<T, D, L, false>(t, ld, order.get(), mode, m, r2, nullptr, d_off, d_out, status.get(), st);
       return;
     }
@@ -1465,15 +1512,15 @@ __global__ void __launch_bounds__(QTHREADS) k_normals_rnear(TreeView<T, 3> tv, L
 template <typename T, typename L>
 __global__ void __launch_bounds__(QTHREADS) k_normals_rnear_warp(TreeView<T, 3> tv, L ld, const int* order,
                                                                  int order_mode, int m, typename DistOf<T>::type r2,
-                                                                 int stack_ints, int num_eigen, T* evecs, T* evals,
-                                                                 int32_t* sizes, int* status) {
+                                                                 int num_eigen, T* evecs, T* evals, int32_t* sizes,
+                                                                 int* status) {
   typedef typename DistOf<T>::type DistT;
-  extern __shared__ __align__(16) int rw_stack[];
+  extern __shared__ __align__(16) int4 rw_stack[];
   const int w = blockIdx.x * QWARPS + (threadIdx.x >> 5);
   if (w >= m) return;
   const int lane = threadIdx.x & 31;
   const unsigned FULL = 0xffffffffu;
-  int* stk = rw_stack + (threadIdx.x >> 5) * stack_ints;
+  int4* stk = rw_stack + (threadIdx.x >> 5) * tv.wstack;
   const int qid = query_of(w, order, order_mode, tv);
   DistT q[3];
   int own = -1;
@@ -1502,7 +1549,9 @@ __global__ void __launch_bounds__(QTHREADS) k_normals_rnear_warp(TreeView<T, 3> 
     __syncwarp();
     return true;
   };
-  const bool ok = !active || warp_rnear_walk<T, 3, DistT>(tv, q, r2, stk, stack_ints, visit);
+  const bool number = active && q[0] == q[0] && q[1] == q[1] && q[2] == q[2];  // (no hits of a NaN)
+  const int root = number && tv.n_wide > 0 ? tv.wide_of(tv.wlevels - 1, 0) : -1;
+  const bool ok = warp_rnear_walk<T, 3, DistT>(tv, root, q, r2, stk, visit);
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
 #pragma unroll
@@ -1747,26 +1796,18 @@ void normals_query(const TreeBase* t, const QuerySpec& qs_in, int k, float r, in
   DevBuf<int> order;
   // (tree order covers valid points only: rows of dropped points, none when
   // n == nv, need no separate pass)
-  const bool warps = k > 0 && by_warp(t->nv, m, k);
-  int mode = 0;
-  if (warps && m <= WARP_UNSORTED)
-    check_indices(t, qs, st);
-  else
-    mode = make_order<T, 3>(t, qs, order, st);
+  const bool warps = k == -1 ? rnear_by_warp(t->nv, m) : by_warp(t->nv, m, k);
+  const int mode = ordered_unless<T, 3>(warps && m <= WARP_UNSORTED, t, qs, order, st);
   // the radius travels as a C float (estimate_normals.cpp:264) and is cast to
   // the input type (:17-22) before being squared in the distance type
   const DistT rr = (DistT)(T)r;
   const DistT r2 = rr * rr;
   IndexQueries<3, false> ld{qs.idx, t->fwd};
   Stage stage("normals", st);
-  if (k == -1 && m <= g_tune_rnear_warp_queries.load()) {
-    const int si = rnear_warp_stack_ints(t->tdepth);
-    const size_t smem = (size_t)QWARPS * si * sizeof(int);
-    if (smem > 48 * 1024)
-      PPTKG_CUDA(cudaFuncSetAttribute(k_normals_rnear_warp<T, IndexQueries<3, false>>,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  if (k == -1 && warps) {
+    const size_t smem = (size_t)QWARPS * wide_stack(t->wlevels) * sizeof(int4);
     k_normals_rnear_warp<T, IndexQueries<3, false>><<<div_up(m, QWARPS), QTHREADS, smem, st>>>(
-        view_of<T, 3>(t), ld, order.get(), mode, m, r2, si, num_eigen, d_evecs, d_evals, d_sizes, status.get());
+        view_of<T, 3>(t), ld, order.get(), mode, m, r2, num_eigen, d_evecs, d_evals, d_sizes, status.get());
     PPTKG_CHECK_LAUNCH();
   } else if (k == -1) {
     const size_t smem = QWARPS * rnear_smem_bytes<T, 3>(t->tdepth);

@@ -87,6 +87,8 @@ struct TreeView {
   const PointRec<T, D>* pts;
   const TNode<T, D>* nodes;
   const WNode<T, D>* wide;
+  const int2* wspan;      // per wide node: first tree position, points
+  const int32_t* ids;     // original index by tree position
   const uint32_t* wbits;  // [wlevels][wwords]: bit p % 32 of word p / 32: a node begins at tree position p
   const int32_t* wrank;   // [wlevels][wwords]: nodes before the word's first (over all levels)
   int32_t wwords, wlevels;
@@ -115,6 +117,7 @@ struct TreeView {
     return i;
   }
   __device__ __forceinline__ const PointRec<T, D>& pt(int i) const { return pts[checked(i, pts_cap, 1)]; }
+  __device__ __forceinline__ int id_at(int i) const { return ids[checked(i, pts_cap, 1)]; }
   __device__ __forceinline__ int pos_of(const int32_t* map, int o) const { return map[checked(o, n_in, 2)]; }
   __device__ __forceinline__ int node_index(int i) const { return checked(i, n_nodes, 3); }
   // the wide hierarchy's node of level j that holds tree position p
@@ -146,6 +149,8 @@ struct TreeBase {
   void* tnodes = nullptr;   // TNode<T, D>[n_tnodes]
   int32_t* fwd = nullptr;   // original index -> tree position, -1 if dropped
   void* wide = nullptr;       // WNode<T, D>[n_wide]
+  int2* wspan = nullptr;      // [n_wide]
+  int32_t* ids = nullptr;     // [nv]: tree position -> original index
   uint32_t* wbits = nullptr;  // [wlevels * wwords]
   int32_t* wrank = nullptr;   // [wlevels * wwords + 1], the last: nodes of the last build
   int n_wide = 0, wlevels = 0, wwords = 0;

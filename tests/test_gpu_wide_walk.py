@@ -80,6 +80,28 @@ def test_walk_in_a_forest_and_a_loaded_tree(gpu, port, span, tmp_path):
             assert np.array_equal(cnt[rows], oc) and np.array_equal(idx[rows], np.where(oi < 0, -1, oi + off[c])), c
 
 
+@pytest.mark.parametrize("n", [1, 33, 513, 8193, 40_000])
+@pytest.mark.parametrize("kind", ["uniform", "skewed", "chain", "copies"])
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+def test_rnear_walk_equals_the_oracle(gpu, port, dtype, kind, n):
+    # hits in ascending tree position: nodes inside the ball as runs of ids
+    # (around the query's own point), runs of cut leaf ranges, more siblings
+    # than lanes; from no hit to every point
+    P = _cloud(kind, n, dtype)
+    rng = np.random.default_rng(6)
+    t, o = gpu.kdtree._build(P), port.PortTree(P)
+    rows = rng.integers(0, n, min(n, 120)).astype(np.int32)
+    Q = np.concatenate([P[rows], rng.random((30, 3)).astype(dtype)])
+    for r in (0.0, 1e-6, 0.02, 0.3, 1.1, 5.0):
+        r = float(np.float32(r))
+        for got, want in ((gpu.kdtree.rnear(t, Q, r), o.rnear(Q, r)),
+                          (gpu.kdtree.rnear(t, rows, r), o.rnear_self(rows, r))):
+            assert np.array_equal(got[0], want[0]) and np.array_equal(got[1], want[1]), r
+    Q[::5, 2] = np.nan
+    off, _ = gpu.kdtree.rnear(t, Q, 0.3)
+    assert (np.diff(off)[::5] == 0).all()
+
+
 @pytest.mark.parametrize("dtype", [np.float32, np.float64])
 @pytest.mark.parametrize("k", [3, 16, 40, 100])
 def test_normals_by_warp_equal_those_of_packets(gpu, dtype, k):
