@@ -6,7 +6,7 @@
 // its own range, so building all nodes of a level at once gives the same
 // permutation.  Nodes with more than `small_cap` points are processed by
 // grid-wide kernels over 4096-point tiles; smaller subtrees are finished by
-// one CTA each, entirely in shared memory.
+// one warp each, entirely in shared memory.
 //
 // The reference partition (PartitionIndices, kdtree-impl.h:192-246) is two
 // Hoare passes with converging cursors.  Each pass pairs the j-th misplaced
@@ -14,6 +14,7 @@
 // right zone (descending), so it is reproduced by ranking the two kinds of
 // misplaced elements with scans and swapping rank-matched pairs.
 #include <algorithm>
+#include <cstddef>
 #include <vector>
 
 #include "build.cuh"
@@ -24,6 +25,7 @@ namespace pptkg {
 
 constexpr int BT = 256;     // threads per tile block
 constexpr int SWAP_U = 4;   // pairs a k_swap thread has in flight
+constexpr int SPLIT_U = 8;  // points a k_split thread has in flight
 constexpr int TILE = 4096;  // points per tile
 constexpr int TITEMS = TILE / BT;
 
@@ -36,25 +38,45 @@ struct Seg {
   long long n_orig;  // input rows of the segment's cloud (the reference's num_points)
   T lo[D], hi[D];  // loose extent (the reference's node_box), trimmed in place
   typename OrdOf<T>::type tlo[D], thi[D];
+  // tight boxes of the points below the split value and of the others,
+  // which are the children's unless ties moved the split
+  typename OrdOf<T>::type clo[2][D], chi[2][D];
   int act;
   int sd;
   T sv;
   int L1, L2;
   int G;
   int tile0, ntiles;
+  int boxed;  // tlo / thi are known (from the parent)
 };
+
+// A segment for k_subtree.
+template <typename T, int D>
+struct Small {
+  int b, e;
+  int up;  // 2 * parent record + side, or -1 - cloud
+  int lvl;
+  long long n_orig;
+  T lo[D], hi[D];
+};
+
+// Ties of segments of at most this many points are moved by one block.
+constexpr int TIE_BLOCK = 8192;
 
 constexpr int MAX_LEVELS = 4096;  // grid-wide levels (segments above small_cap points)
 
 struct BuildCtl {
   int status;
-  int n_tiles;
   int nsmall;
   int small_next;
   int rec_count;
   int depth;
-  int level_cnt[MAX_LEVELS + 1];  // large segments per level
-  int rec_base[MAX_LEVELS + 1];
+  int ties;     // 1 + the last level with points at a split value
+  int big;      // 1 + the last level with such points in a segment too large for one block
+  int stalled;  // 1 + the level that waits for a tie pass that the host has not launched
+  int unboxed;  // 1 + the last level with segments whose box is not known
+  int level_cnt[MAX_LEVELS + 1];    // large segments per level
+  int level_tiles[MAX_LEVELS + 1];  // their tiles
 };
 
 // ----------------------------------------------------------------- helpers
@@ -168,6 +190,45 @@ __device__ __forceinline__ int num_left_rule(int lim1, int lim2, int count) {
   return nl;
 }
 
+template <typename T, int D>
+__device__ __forceinline__ Small<T, D> small_of(const Seg<T, D>& g) {
+  Small<T, D> s;
+  s.b = g.b;
+  s.e = g.e;
+  s.up = g.parent < 0 ? g.parent : 2 * g.parent + g.side;
+  s.lvl = g.lvl;
+  s.n_orig = g.n_orig;
+  for (int d = 0; d < D; d++) {
+    s.lo[d] = g.lo[d];
+    s.hi[d] = g.hi[d];
+  }
+  return s;
+}
+
+template <typename T, int D>
+__device__ __forceinline__ void seg_clear(Seg<T, D>& g) {
+  for (int d = 0; d < D; d++) {
+    g.tlo[d] = ord_t<T>(Limits<T>::max());
+    g.thi[d] = ord_t<T>(Limits<T>::lowest());
+    for (int c = 0; c < 2; c++) {
+      g.clo[c][d] = ord_t<T>(Limits<T>::max());
+      g.chi[c][d] = ord_t<T>(Limits<T>::lowest());
+    }
+  }
+  g.L1 = g.L2 = 0;
+  g.act = 0;
+  g.G = 0;
+  g.boxed = 0;
+}
+
+// A large segment takes its tiles and its record.
+template <typename T, int D>
+__device__ __forceinline__ void take_place(Seg<T, D>& g, int lvl, BuildCtl* ctl) {
+  g.ntiles = div_up_dev(g.e - g.b, TILE);
+  g.tile0 = atomicAdd(&ctl->level_tiles[lvl], g.ntiles);
+  g.rec = atomicAdd(&ctl->rec_count, 1);
+}
+
 // ------------------------------------------------------- input staging ----
 template <typename T, int D>
 __global__ void k_valid(const T* __restrict__ in, int64_t n, int* __restrict__ flag) {
@@ -203,7 +264,7 @@ static __global__ void k_cloud_off(const int* off, const int64_t* orig_off, int 
 // so the host never waits between levels.
 template <typename T, int D>
 __global__ void k_roots(const int64_t* valid_off, const int64_t* orig_off, int ncloud, int small_cap, Seg<T, D>* lvl0,
-                        Seg<T, D>* small, int small_capn, BuildCtl* ctl) {
+                        Small<T, D>* small, int small_capn, BuildCtl* ctl) {
   int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= ncloud) return;
   const int b = (int)valid_off[c], e = (int)valid_off[c + 1];
@@ -220,43 +281,26 @@ __global__ void k_roots(const int64_t* valid_off, const int64_t* orig_off, int n
     g.lo[d] = Limits<T>::max();  // replaced by the tight box at a root
     g.hi[d] = Limits<T>::lowest();
   }
+  seg_clear(g);
   if (e - b > small_cap) {
+    ctl->unboxed = 1;
+    take_place(g, 0, ctl);
     lvl0[atomicAdd(&ctl->level_cnt[0], 1)] = g;
   } else {
     const int slot = atomicAdd(&ctl->nsmall, 1);
     if (slot < small_capn)
-      small[slot] = g;
+      small[slot] = small_of(g);
     else
       atomicExch(&ctl->status, 7);
   }
 }
 
+// The segment of every tile, a warp per segment.
 template <typename T, int D>
-__global__ void k_tiles(Seg<T, D>* segs, int lvl, int* tile_seg, BuildCtl* ctl) {
-  __shared__ int sh[33];
-  const int nseg = ctl->level_cnt[lvl];
-  int carry = 0;
-  for (int c0 = 0; c0 < nseg; c0 += blockDim.x) {
-    int i = c0 + threadIdx.x;
-    int nt = 0;
-    if (i < nseg) nt = div_up_dev(segs[i].e - segs[i].b, TILE);
-    int tot;
-    int ex = block_excl_scan(nt, sh, tot);
-    if (i < nseg) {
-      segs[i].tile0 = carry + ex;
-      segs[i].ntiles = nt;
-    }
-    carry += tot;
-  }
-  if (threadIdx.x == 0) {
-    ctl->n_tiles = carry;
-    ctl->rec_base[lvl] = ctl->rec_count;
-    ctl->rec_count += nseg;
-  }
-  __syncthreads();
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  for (int i = wid; i < nseg; i += nw) {
-    int t0 = segs[i].tile0, nt = segs[i].ntiles;
+__global__ void k_tiles(const Seg<T, D>* segs, int lvl, int* tile_seg, const BuildCtl* ctl) {
+  const int nseg = ctl->level_cnt[lvl], lane = threadIdx.x & 31;
+  for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < nseg; i += (gridDim.x * blockDim.x) >> 5) {
+    const int t0 = segs[i].tile0, nt = segs[i].ntiles;
     for (int t = lane; t < nt; t += 32) tile_seg[t0 + t] = i;
   }
 }
@@ -273,19 +317,6 @@ __device__ __forceinline__ void tile_at(const Seg<T, D>* segs, const int* tile_s
   end = min(start + TILE, segs[s].e);
 }
 
-template <typename T, int D>
-__global__ void k_seg_init(Seg<T, D>* segs, int lvl, const BuildCtl* ctl) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= ctl->level_cnt[lvl]) return;
-  for (int d = 0; d < D; d++) {
-    segs[i].tlo[d] = ord_t<T>(Limits<T>::max());
-    segs[i].thi[d] = ord_t<T>(Limits<T>::lowest());
-  }
-  segs[i].L1 = segs[i].L2 = 0;
-  segs[i].act = 0;
-  segs[i].G = 0;
-}
-
 template <typename T>
 __device__ __forceinline__ T warp_min(T v) {
 #pragma unroll
@@ -299,14 +330,33 @@ __device__ __forceinline__ T warp_max(T v) {
   return v;
 }
 
+// The same of ordered images, in one instruction for 32-bit ones.
+template <typename U>
+__device__ __forceinline__ U warp_min_ord(U v) {
+  if constexpr (sizeof(U) == 4)
+    return __reduce_min_sync(0xffffffffu, v);
+  else
+    return warp_min(v);
+}
+template <typename U>
+__device__ __forceinline__ U warp_max_ord(U v) {
+  if constexpr (sizeof(U) == 4)
+    return __reduce_max_sync(0xffffffffu, v);
+  else
+    return warp_max(v);
+}
+
 template <typename T, int D>
-__global__ void __launch_bounds__(BT) k_bbox(Seg<T, D>* segs, const int* tile_seg, const BuildCtl* ctl, SoA<T, D> soa) {
+__global__ void __launch_bounds__(BT) k_bbox(Seg<T, D>* segs, int lvl, const int* tile_seg, const BuildCtl* ctl,
+                                             SoA<T, D> soa) {
   __shared__ T shmn[D][BT / 32], shmx[D][BT / 32];
-  const int ntiles = ctl->n_tiles;
+  if (ctl->unboxed != lvl + 1) return;
+  const int ntiles = ctl->level_tiles[lvl];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
     int s, start, end;
     tile_at(segs, tile_seg, t, s, start, end);
+    if (segs[s].boxed) continue;  // (uniform over the block)
     T mn[D], mx[D];
 #pragma unroll
     for (int d = 0; d < D; d++) {
@@ -345,107 +395,383 @@ __global__ void __launch_bounds__(BT) k_bbox(Seg<T, D>* segs, const int* tile_se
   }
 }
 
+// A record takes its place and its parent learns of it.
 template <typename T, int D>
-__global__ void k_node(Seg<T, D>* segs, int lvl, BuildCtl* ctl, Rec<T, D>* recs, int rec_cap, int* root_rec,
-                       int max_leaf, double thr) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= ctl->level_cnt[lvl]) return;
-  Seg<T, D>& g = segs[i];
-  T tlo[D], thi[D], lo[D], hi[D];
+__device__ __forceinline__ bool link_record(const Rec<T, D>& rec, int id, int up, Rec<T, D>* recs, int rec_cap,
+                                            int* root_rec, BuildCtl* ctl) {
+  if (id >= rec_cap) {
+    atomicExch(&ctl->status, 6);
+    return false;
+  }
+  recs[id] = rec;
+  if (up < 0)
+    root_rec[-up - 1] = id;
+  else if (up & 1)
+    recs[up >> 1].right = id;
+  else
+    recs[up >> 1].left = id;
+  return true;
+}
+
+// Split decision and record of a segment whose box is known.
+template <typename T, int D>
+__device__ __forceinline__ void decide(Seg<T, D>& g, BuildCtl* ctl, Rec<T, D>* recs, int rec_cap, int* root_rec,
+                                       int max_leaf, double thr) {
+  T tlo[D], thi[D];
   for (int d = 0; d < D; d++) {
     tlo[d] = from_ord_t<T>(g.tlo[d]);
     thi[d] = from_ord_t<T>(g.thi[d]);
-    lo[d] = g.lo[d];
-    hi[d] = g.hi[d];
   }
   Rec<T, D> rec;
-  int act, sd = 0;
-  T sv = (T)0;
-  node_logic<T, D>(g.e - g.b, g.n_orig, g.parent < 0, lo, hi, tlo, thi, max_leaf, thr, rec, act, sd, sv);
+  g.sd = 0;
+  g.sv = (T)0;
+  node_logic<T, D>(g.e - g.b, g.n_orig, g.parent < 0, g.lo, g.hi, tlo, thi, max_leaf, thr, rec, g.act, g.sd, g.sv);
   rec.begin = g.b;
   rec.end = g.e;
-  const int id = ctl->rec_base[lvl] + i;
-  if (id >= rec_cap) {
-    atomicExch(&ctl->status, 6);
+  if (!link_record<T, D>(rec, g.rec, g.parent < 0 ? g.parent : 2 * g.parent + g.side, recs, rec_cap, root_rec, ctl))
     g.act = 0;
-    return;
-  }
-  recs[id] = rec;
-  if (g.parent >= 0) {
-    if (g.side == 0)
-      recs[g.parent].left = id;
-    else
-      recs[g.parent].right = id;
-  } else {
-    root_rec[-g.parent - 1] = id;
-  }
-  g.rec = id;
-  g.act = act;
-  g.sd = sd;
-  g.sv = sv;
-  for (int d = 0; d < D; d++) {
-    g.lo[d] = lo[d];
-    g.hi[d] = hi[d];
-  }
+  g.boxed = 1;
 }
 
+// The decisions that waited for k_bbox.
 template <typename T, int D>
-__global__ void __launch_bounds__(BT) k_count(Seg<T, D>* segs, const int* tile_seg, const BuildCtl* ctl, SoA<T, D> soa) {
-  __shared__ long long sh[33];
-  const int ntiles = ctl->n_tiles;
+__global__ void k_node(Seg<T, D>* segs, int lvl, BuildCtl* ctl, Rec<T, D>* recs, int rec_cap, int* root_rec,
+                       int max_leaf, double thr) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (ctl->unboxed != lvl + 1 || i >= ctl->level_cnt[lvl] || segs[i].boxed) return;
+  Seg<T, D> g = segs[i];
+  decide(g, ctl, recs, rec_cap, root_rec, max_leaf, thr);
+  segs[i] = g;
+}
+
+// One pass over a level's points: how many lie below (L1) and at or below
+// (L2) the split value, per tile how many below, which (a bit per point, for
+// the ranks), and the tight boxes of both sides, so that neither the ranks nor
+// the next level's boxes read the points again: 12 B a point in place of 24.
+// Bound by its instructions (two-sided boxes), then by loads in flight: 20M
+// points 107 us with selects for both sides, 65 with a branch.
+template <typename T, int D>
+__global__ void __launch_bounds__(BT) k_split(Seg<T, D>* segs, int lvl, const int* tile_seg, const BuildCtl* ctl,
+                                              SoA<T, D> soa, int* tile_lt, uint32_t* tile_bits) {
+  typedef typename OrdOf<T>::type U;
+  __shared__ U shb[BT / 32][4 * D];
+  __shared__ int shc[BT / 32][2];
+  const int ntiles = ctl->level_tiles[lvl];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
     int s, start, end;
     tile_at(segs, tile_seg, t, s, start, end);
     if (!segs[s].act) continue;  // (uniform over the block)
     const T sv = segs[s].sv;
-    const T* v = soa.x[segs[s].sd];
+    const int sd = segs[s].sd;
+    T lo[2][D], hi[2][D];
+#pragma unroll
+    for (int c = 0; c < 2; c++)
+#pragma unroll
+      for (int d = 0; d < D; d++) {
+        lo[c][d] = Limits<T>::max();
+        hi[c][d] = Limits<T>::lowest();
+      }
     int c1 = 0, c2 = 0;
-    for (int i = start + threadIdx.x; i < end; i += BT) {
-      T x = v[i];
-      c1 += x < sv;
-      c2 += x <= sv;
+    // a full tile needs no test of its end; the loads of SPLIT_U points are
+    // issued together
+    auto points = [&](auto full) {
+      for (int j0 = 0; j0 < TITEMS; j0 += SPLIT_U) {
+        T x[SPLIT_U][D];
+        bool in[SPLIT_U];
+#pragma unroll
+        for (int u = 0; u < SPLIT_U; u++) {
+          const int i = start + (j0 + u) * BT + threadIdx.x;
+          in[u] = decltype(full)::value || i < end;
+#pragma unroll
+          for (int d = 0; d < D; d++) x[u][d] = in[u] ? soa.x[d][i] : (T)0;
+        }
+#pragma unroll
+        for (int u = 0; u < SPLIT_U; u++) {
+          T v = x[u][0];
+#pragma unroll
+          for (int d = 1; d < D; d++) v = d == sd ? x[u][d] : v;
+          const bool below = in[u] && v < sv;
+          c2 += in[u] && v == sv;
+          if (below) {
+#pragma unroll
+            for (int d = 0; d < D; d++) {
+              lo[0][d] = min(lo[0][d], x[u][d]);
+              hi[0][d] = max(hi[0][d], x[u][d]);
+            }
+          } else if (in[u]) {
+#pragma unroll
+            for (int d = 0; d < D; d++) {
+              lo[1][d] = min(lo[1][d], x[u][d]);
+              hi[1][d] = max(hi[1][d], x[u][d]);
+            }
+          }
+          const unsigned m = __ballot_sync(0xffffffffu, below);
+          c1 += __popc(m);
+          if (lane == 0) tile_bits[(size_t)t * (TILE / 32) + (j0 + u) * (BT / 32) + wid] = m;
+        }
+      }
+    };
+    if (start + TILE <= end)
+      points(std::true_type());
+    else
+      points(std::false_type());
+    c2 = warp_sum(c2) + c1;  // (c1: the warp's already)
+#pragma unroll
+    for (int c = 0; c < 2; c++)
+#pragma unroll
+      for (int d = 0; d < D; d++) {
+        const U a = warp_min_ord(ord_t<T>(lo[c][d])), b = warp_max_ord(ord_t<T>(hi[c][d]));
+        if (lane == 0) {
+          shb[wid][c * 2 * D + d] = a;
+          shb[wid][c * 2 * D + D + d] = b;
+        }
+      }
+    if (lane == 0) {
+      shc[wid][0] = c1;
+      shc[wid][1] = c2;
     }
-    long long packed = ((long long)c2 << 32) | (long long)c1;
-    long long tot = block_sum(packed, sh);
+    __syncthreads();
+    if (threadIdx.x < 4 * D) {
+      const int c = threadIdx.x / (2 * D), r = threadIdx.x % (2 * D);
+      U v = shb[0][threadIdx.x];
+      for (int w = 1; w < BT / 32; w++) v = r < D ? min(v, shb[w][threadIdx.x]) : max(v, shb[w][threadIdx.x]);
+      if (r < D)
+        atomicMin(&segs[s].clo[c][r], v);
+      else
+        atomicMax(&segs[s].chi[c][r - D], v);
+    } else if (threadIdx.x == 4 * D) {
+      int n = 0;
+      for (int w = 0; w < BT / 32; w++) n += shc[w][0];
+      tile_lt[t] = n;
+      atomicAdd(&segs[s].L1, n);
+    } else if (threadIdx.x == 4 * D + 1) {
+      int n = 0;
+      for (int w = 0; w < BT / 32; w++) n += shc[w][1];
+      atomicAdd(&segs[s].L2, n);
+    }
+    __syncthreads();
+  }
+}
+
+// Ranks of pass 1 from the tiles' counts: left of Z = b + L1 the points not
+// below the split value are misplaced, right of it those below.  A tile on
+// one side of Z needs no second look; the one that holds Z counts its bits.
+template <typename T, int D>
+__global__ void k_ranks(Seg<T, D>* segs, int lvl, const int* tile_lt, const uint32_t* tile_bits, long long* tile_off,
+                        BuildCtl* ctl) {
+  __shared__ long long sh[33];
+  const int nseg = ctl->level_cnt[lvl];
+  for (int si = blockIdx.x; si < nseg; si += gridDim.x) {
+    Seg<T, D>& g = segs[si];
+    if (!g.act) continue;  // (uniform over the block)
+    const int b = g.b, Z = b + g.L1;
+    // points below the split value among the first Z - start of the tile that
+    // holds Z (one word per thread)
+    const int mid = g.L1 / TILE, n = g.L1 - mid * TILE;
+    int in = 0;
+    if (mid < g.ntiles && threadIdx.x <= n >> 5 && threadIdx.x < TILE / 32) {
+      const uint32_t w = tile_bits[(size_t)(g.tile0 + mid) * (TILE / 32) + threadIdx.x];
+      in = __popc(threadIdx.x < n >> 5 ? w : w & ((1u << (n & 31)) - 1u));
+    }
+    const int left = (int)block_sum((long long)in, sh);
+    long long carry = 0;
+    for (int c0 = 0; c0 < g.ntiles; c0 += blockDim.x) {
+      const int t = c0 + threadIdx.x;
+      long long v = 0;
+      if (t < g.ntiles) {
+        const int start = b + t * TILE, end = min(start + TILE, g.e), lt = tile_lt[g.tile0 + t];
+        if (end <= Z) {
+          v = end - start - lt;
+        } else if (start >= Z) {
+          v = (long long)lt << 32;
+        } else {
+          v = (n - left) + ((long long)(lt - left) << 32);
+        }
+      }
+      long long tot;
+      const long long ex = block_excl_scan(v, sh, tot);
+      if (t < g.ntiles) tile_off[g.tile0 + t] = carry + ex;
+      carry += tot;
+    }
     if (threadIdx.x == 0) {
-      atomicAdd(&segs[s].L1, (int)(tot & 0xffffffffll));
-      atomicAdd(&segs[s].L2, (int)(tot >> 32));
+      const int nbl = (int)(carry & 0xffffffffll), ngr = (int)(carry >> 32);
+      g.G = nbl;
+      if (nbl != ngr) atomicExch(&ctl->status, 1);
+      if (g.L1 != g.L2) {
+        ctl->ties = lvl + 1;
+        if (g.e - g.b > TIE_BLOCK) ctl->big = lvl + 1;
+      }
     }
   }
 }
 
-// Misplaced-element predicates of the two partition passes.
-template <typename T>
-__device__ __forceinline__ void pass_flags(int pass, int i, T x, T sv, int b, int L1, int L2, bool& bl, bool& gr) {
-  if (pass == 1) {
-    const int Z = b + L1;
-    bl = (i < Z) && !(x < sv);
-    gr = (i >= Z) && (x < sv);
-  } else {
-    const int Z = b + L2;
-    bl = (i >= b + L1) && (i < Z) && (x > sv);
-    gr = (i >= Z) && (x <= sv);
+// The positions of pass 1's misplaced points at their ranks, from the bits.
+template <typename T, int D>
+__global__ void __launch_bounds__(BT) k_place_ranks(Seg<T, D>* segs, int lvl, const int* tile_seg,
+                                                    const BuildCtl* ctl, const uint32_t* tile_bits, const long long* tile_off, int* blpos,
+                                                    int* grpos) {
+  __shared__ long long sh[33];
+  const int ntiles = ctl->level_tiles[lvl];
+  for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
+    int s, start, end;
+    tile_at(segs, tile_seg, t, s, start, end);
+    if (!segs[s].act) continue;  // (uniform over the block)
+    const int b = segs[s].b, Z = b + segs[s].L1, G = segs[s].G, size = segs[s].e - b;
+    // 16 positions per thread: half a word
+    static_assert(TITEMS == 16, "half a word of the tile's bits per thread");
+    const int i0 = start + threadIdx.x * TITEMS;
+    const unsigned below = tile_bits[(size_t)t * (TILE / 32) + (threadIdx.x >> 1)] >> (16 * (threadIdx.x & 1)) & 0xffffu;
+    const unsigned in = i0 >= end ? 0u : end - i0 >= TITEMS ? 0xffffu : (1u << (end - i0)) - 1u;
+    const unsigned left = i0 >= Z ? 0u : Z - i0 >= TITEMS ? 0xffffu : (1u << (Z - i0)) - 1u;
+    unsigned mbl = in & left & ~below, mgr = in & ~left & below;
+    const long long mine = (long long)__popc(mbl) + ((long long)__popc(mgr) << 32);
+    long long tot;
+    const long long ex = block_excl_scan(mine, sh, tot) + tile_off[t];
+    int rb = (int)(ex & 0xffffffffll), rg = (int)(ex >> 32);
+    while (mbl) {
+      const int j = __ffs(mbl) - 1;
+      mbl &= mbl - 1;
+      if (rb < size) blpos[b + rb] = i0 + j;
+      rb++;
+    }
+    while (mgr) {
+      const int j = __ffs(mgr) - 1;
+      mgr &= mgr - 1;
+      const int slot = G - 1 - rg;
+      if (slot >= 0 && slot < size) grpos[b + slot] = i0 + j;
+      rg++;
+    }
   }
+}
+
+// ---- the tie pass (PartitionIndices' second): points equal to the split
+// value move to [b + L1, b + L2).  Segments of up to TIE_BLOCK points have it
+// from one block each (k_ties), larger ones from the whole grid (k_flags,
+// k_tscan, k_scatter, k_swap), which the host launches only once a level has
+// asked for it.
+template <typename T, int D>
+__device__ __forceinline__ bool big_tie(const Seg<T, D>& g) {
+  return g.L1 != g.L2 && g.e - g.b > TIE_BLOCK;
 }
 
 template <typename T, int D>
-__global__ void __launch_bounds__(BT) k_flags(int pass, Seg<T, D>* segs, const int* tile_seg, const BuildCtl* ctl,
+__global__ void __launch_bounds__(BT) k_ties(Seg<T, D>* segs, int lvl, BuildCtl* ctl, SoA<T, D> soa, int* blpos,
+                                             int* grpos) {
+  typedef typename OrdOf<T>::type U;
+  __shared__ long long sh[33];
+  __shared__ U box[4 * D];
+  if (ctl->ties != lvl + 1) return;
+  const int nseg = ctl->level_cnt[lvl];
+  for (int si = blockIdx.x; si < nseg; si += gridDim.x) {
+    Seg<T, D>& g = segs[si];
+    if (!g.act || g.L1 == g.L2 || g.e - g.b > TIE_BLOCK) continue;  // (uniform over the block)
+    const int b = g.b, e = g.e, L1 = g.L1, Z = b + g.L2;
+    const T sv = g.sv;
+    const T* v = soa.x[g.sd];
+    long long carry = 0;
+    for (int i0 = b + L1; i0 < e; i0 += BT) {
+      const int i = i0 + threadIdx.x;
+      bool bl = false, gr = false;
+      if (i < e) {
+        const T x = v[i];
+        bl = i < Z && x > sv;
+        gr = i >= Z && x <= sv;
+      }
+      long long tot;
+      const long long ex = carry + block_excl_scan((long long)bl + ((long long)gr << 32), sh, tot);
+      if (bl) blpos[b + (int)(ex & 0xffffffffll)] = i;
+      if (gr) grpos[b + (int)(ex >> 32)] = i;  // (from the left: read from its end below)
+      carry += tot;
+    }
+    const int G = (int)(carry & 0xffffffffll);
+    if (G != (int)(carry >> 32)) {
+      if (threadIdx.x == 0) atomicExch(&ctl->status, 1);
+      continue;
+    }
+    __threadfence_block();
+    __syncthreads();
+    for (int j = threadIdx.x; j < G; j += BT) {
+      const int x = blpos[b + j], y = grpos[b + G - 1 - j];
+#pragma unroll
+      for (int d = 0; d < D; d++) {
+        const T t = soa.x[d][x];
+        soa.x[d][x] = soa.x[d][y];
+        soa.x[d][y] = t;
+      }
+      const int t = soa.id[x];
+      soa.id[x] = soa.id[y];
+      soa.id[y] = t;
+    }
+    // the children's boxes, where the ties moved the split off b + L1
+    const int at = b + num_left_rule(L1, g.L2, e - b);
+    if (at == b + L1) continue;  // (uniform over the block)
+    if (threadIdx.x < 4 * D)
+      box[threadIdx.x] = ord_t<T>((threadIdx.x / D) & 1 ? Limits<T>::lowest() : Limits<T>::max());
+    __threadfence_block();
+    __syncthreads();
+    U lo[2][D], hi[2][D];
+#pragma unroll
+    for (int c = 0; c < 2; c++)
+#pragma unroll
+      for (int d = 0; d < D; d++) {
+        lo[c][d] = ord_t<T>(Limits<T>::max());
+        hi[c][d] = ord_t<T>(Limits<T>::lowest());
+      }
+    for (int i = b + threadIdx.x; i < e; i += BT)
+#pragma unroll
+      for (int d = 0; d < D; d++) {
+        const U x = ord_t<T>(soa.x[d][i]);
+#pragma unroll
+        for (int c = 0; c < 2; c++)
+          if ((i >= at) == (c == 1)) {
+            lo[c][d] = min(lo[c][d], x);
+            hi[c][d] = max(hi[c][d], x);
+          }
+      }
+#pragma unroll
+    for (int c = 0; c < 2; c++)
+#pragma unroll
+      for (int d = 0; d < D; d++) {
+        atomicMin(&box[(2 * c) * D + d], lo[c][d]);
+        atomicMax(&box[(2 * c + 1) * D + d], hi[c][d]);
+      }
+    __syncthreads();
+    if (threadIdx.x < D) {
+      const int d = threadIdx.x;
+      for (int c = 0; c < 2; c++) {
+        g.clo[c][d] = box[(2 * c) * D + d];
+        g.chi[c][d] = box[(2 * c + 1) * D + d];
+      }
+    }
+    __syncthreads();
+  }
+}
+
+template <typename T>
+__device__ __forceinline__ void tie_flags(int i, T x, T sv, int b, int L1, int L2, bool& bl, bool& gr) {
+  const int Z = b + L2;
+  bl = (i >= b + L1) && (i < Z) && (x > sv);
+  gr = (i >= Z) && (x <= sv);
+}
+
+template <typename T, int D>
+__global__ void __launch_bounds__(BT) k_flags(Seg<T, D>* segs, int lvl, const int* tile_seg, const BuildCtl* ctl,
                                               SoA<T, D> soa, long long* tile_cnt) {
   __shared__ long long sh[33];
-  const int ntiles = ctl->n_tiles;
+  if (ctl->big != lvl + 1) return;
+  const int ntiles = ctl->level_tiles[lvl];
   for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
     int s, start, end;
     tile_at(segs, tile_seg, t, s, start, end);
     long long c = 0;
-    // the second pass moves the points equal to the split value; with none
-    // (L1 == L2, the usual case for float data) it has nothing to do
-    if (segs[s].act && !(pass == 2 && segs[s].L1 == segs[s].L2)) {
+    if (segs[s].act && big_tie(segs[s])) {
       const T sv = segs[s].sv;
       const T* v = soa.x[segs[s].sd];
       const int b = segs[s].b, L1 = segs[s].L1, L2 = segs[s].L2;
       for (int i = start + threadIdx.x; i < end; i += BT) {
         bool bl, gr;
-        pass_flags(pass, i, v[i], sv, b, L1, L2, bl, gr);
+        tie_flags(i, v[i], sv, b, L1, L2, bl, gr);
         c += (long long)bl + ((long long)gr << 32);
       }
     }
@@ -457,10 +783,11 @@ __global__ void __launch_bounds__(BT) k_flags(int pass, Seg<T, D>* segs, const i
 template <typename T, int D>
 __global__ void k_tscan(Seg<T, D>* segs, int lvl, const long long* tile_cnt, long long* tile_off, BuildCtl* ctl) {
   __shared__ long long sh[33];
+  if (ctl->big != lvl + 1) return;
   const int nseg = ctl->level_cnt[lvl];
   for (int si = blockIdx.x; si < nseg; si += gridDim.x) {
     Seg<T, D>& g = segs[si];
-    if (!g.act) continue;  // (uniform over the block)
+    if (!g.act || !big_tie(g)) continue;  // (uniform over the block)
     long long carry = 0;
     for (int c0 = 0; c0 < g.ntiles; c0 += blockDim.x) {
       int t = c0 + threadIdx.x;
@@ -479,14 +806,15 @@ __global__ void k_tscan(Seg<T, D>* segs, int lvl, const long long* tile_cnt, lon
 }
 
 template <typename T, int D>
-__global__ void __launch_bounds__(BT) k_scatter(int pass, Seg<T, D>* segs, const int* tile_seg, const BuildCtl* ctl,
+__global__ void __launch_bounds__(BT) k_scatter(Seg<T, D>* segs, int lvl, const int* tile_seg, const BuildCtl* ctl,
                                                 SoA<T, D> soa, const long long* tile_off, int* blpos, int* grpos) {
   __shared__ long long sh[33];
-  const int ntiles = ctl->n_tiles;
+  if (ctl->big != lvl + 1) return;
+  const int ntiles = ctl->level_tiles[lvl];
   for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
     int s, start, end;
     tile_at(segs, tile_seg, t, s, start, end);
-    if (!segs[s].act || (pass == 2 && segs[s].L1 == segs[s].L2)) continue;  // (uniform over the block)
+    if (!segs[s].act || !big_tie(segs[s])) continue;  // (uniform over the block)
     const T sv = segs[s].sv;
     const T* v = soa.x[segs[s].sd];
     const int b = segs[s].b, L1 = segs[s].L1, L2 = segs[s].L2, G = segs[s].G;
@@ -497,7 +825,7 @@ __global__ void __launch_bounds__(BT) k_scatter(int pass, Seg<T, D>* segs, const
       int i = i0 + j;
       if (i < end) {
         bool bl, gr;
-        pass_flags(pass, i, v[i], sv, b, L1, L2, bl, gr);
+        tie_flags(i, v[i], sv, b, L1, L2, bl, gr);
         mbl |= (unsigned)bl << j;
         mgr |= (unsigned)gr << j;
       }
@@ -522,14 +850,17 @@ __global__ void __launch_bounds__(BT) k_scatter(int pass, Seg<T, D>* segs, const
   }
 }
 
+// Swaps rank-matched pairs (tie: those of the tie pass, if the level has one).
 template <typename T, int D>
-__global__ void __launch_bounds__(BT) k_swap(Seg<T, D>* segs, const int* tile_seg, BuildCtl* ctl, SoA<T, D> soa,
-                                             const int* blpos, const int* grpos) {
-  const int ntiles = ctl->n_tiles;
+__global__ void __launch_bounds__(BT) k_swap(Seg<T, D>* segs, int lvl, bool tie, const int* tile_seg, BuildCtl* ctl,
+                                             SoA<T, D> soa, const int* blpos, const int* grpos) {
+  if (tie && ctl->big != lvl + 1) return;
+  const int ntiles = ctl->level_tiles[lvl];
   for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
     int s, start, end;
     tile_at(segs, tile_seg, t, s, start, end);
     if (!segs[s].act) continue;
+    if (tie && !big_tie(segs[s])) continue;
     const int b = segs[s].b, e = segs[s].e, G = segs[s].G;
     // pair j of this tile: j = start - b + threadIdx.x + u * BT.  Every
     // position belongs to one pair only, so the loads of SWAP_U pairs are
@@ -578,371 +909,406 @@ __global__ void __launch_bounds__(BT) k_swap(Seg<T, D>* segs, const int* tile_se
   }
 }
 
+// The children of a level's segments: a lane per segment makes them, decides
+// those that stay large, and the warp writes the map of their tiles.
 template <typename T, int D>
-__global__ void k_children(Seg<T, D>* segs, int lvl, Rec<T, D>* recs, Seg<T, D>* next, Seg<T, D>* small,
-                           int small_capn, int small_cap_pts, BuildCtl* ctl) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= ctl->level_cnt[lvl]) return;
-  const Seg<T, D>& g = segs[i];
-  if (!g.act) return;
-  const int count = g.e - g.b;
-  const int si = g.b + num_left_rule(g.L1, g.L2, count);
-  recs[g.rec].split_index = si;
-  for (int side = 0; side < 2; side++) {
-    int cb = side ? si : g.b, ce = side ? g.e : si;
-    if (cb >= ce) continue;
-    Seg<T, D> c;
-    c.b = cb;
-    c.e = ce;
-    c.parent = g.rec;
-    c.side = side;
-    c.lvl = g.lvl + 1;
-    c.rec = -1;
-    c.n_orig = g.n_orig;
-    for (int d = 0; d < D; d++) {
-      c.lo[d] = g.lo[d];
-      c.hi[d] = g.hi[d];
-    }
-    if (side == 0)
-      c.hi[g.sd] = g.sv;
-    else
-      c.lo[g.sd] = g.sv;
-    if (ce - cb > small_cap_pts) {
-      next[atomicAdd(&ctl->level_cnt[lvl + 1], 1)] = c;
-    } else {
-      const int slot = atomicAdd(&ctl->nsmall, 1);
-      if (slot < small_capn)
-        small[slot] = c;
+__global__ void k_children(Seg<T, D>* segs, int lvl, int tied, Rec<T, D>* recs, int rec_cap, Seg<T, D>* next,
+                           Small<T, D>* small, int small_capn, int small_cap_pts, int max_leaf, double thr,
+                           int* tile_seg, BuildCtl* ctl) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31;
+  // a level whose ties had no pass (tied 0: none was launched, 1: that of
+  // small segments) waits for it
+  if ((tied < 1 && ctl->ties == lvl + 1) || (tied < 2 && ctl->big == lvl + 1)) {
+    if (i == 0) ctl->stalled = lvl + 1;
+    return;
+  }
+  const int nseg = ctl->level_cnt[lvl];
+  if ((i & ~31) >= nseg) return;
+  int t0[2] = {0, 0}, nt[2] = {0, 0}, at[2] = {0, 0};
+  if (i < nseg && segs[i].act) {
+    const Seg<T, D>& g = segs[i];
+    const int count = g.e - g.b;
+    const int si = g.b + num_left_rule(g.L1, g.L2, count);
+    recs[g.rec].split_index = si;
+#pragma unroll
+    for (int side = 0; side < 2; side++) {
+      const int cb = side ? si : g.b, ce = side ? g.e : si;
+      if (cb >= ce) continue;
+      Seg<T, D> c;
+      c.b = cb;
+      c.e = ce;
+      c.parent = g.rec;
+      c.side = side;
+      c.lvl = g.lvl + 1;
+      c.rec = -1;
+      c.n_orig = g.n_orig;
+      for (int d = 0; d < D; d++) {
+        c.lo[d] = g.lo[d];
+        c.hi[d] = g.hi[d];
+      }
+      if (side == 0)
+        c.hi[g.sd] = g.sv;
       else
-        atomicExch(&ctl->status, 7);
+        c.lo[g.sd] = g.sv;
+      if (ce - cb > small_cap_pts) {
+        seg_clear(c);
+        take_place(c, lvl + 1, ctl);
+        if (si == g.b + g.L1 || !big_tie(g)) {
+          for (int d = 0; d < D; d++) {
+            c.tlo[d] = g.clo[side][d];
+            c.thi[d] = g.chi[side][d];
+          }
+          decide(c, ctl, recs, rec_cap, (int*)nullptr, max_leaf, thr);
+        } else {
+          ctl->unboxed = lvl + 2;
+        }
+        t0[side] = c.tile0;
+        nt[side] = c.ntiles;
+        at[side] = atomicAdd(&ctl->level_cnt[lvl + 1], 1);
+        next[at[side]] = c;
+      } else {
+        const int slot = atomicAdd(&ctl->nsmall, 1);
+        if (slot < small_capn)
+          small[slot] = small_of(c);
+        else
+          atomicExch(&ctl->status, 7);
+      }
     }
   }
+#pragma unroll
+  for (int side = 0; side < 2; side++)
+    for (unsigned rest = __ballot_sync(0xffffffffu, nt[side] > 0); rest; rest &= rest - 1) {
+      const int s = __ffs(rest) - 1;
+      const int a = __shfl_sync(0xffffffffu, t0[side], s), n = __shfl_sync(0xffffffffu, nt[side], s),
+                k = __shfl_sync(0xffffffffu, at[side], s);
+      for (int t = lane; t < n; t += 32) tile_seg[a + t] = k;
+    }
 }
 
-// -------------------------------------------------- per-CTA subtrees ----
+// ------------------------------------------------- per-warp subtrees ----
 template <typename T, int D>
 struct Entry {
-  int b, e, parent, side;
+  uint16_t b, e;
+  int up;  // 2 * parent record + side, or -1 - cloud for a root
   T lo[D], hi[D];
 };
 
-constexpr int SUB_THREADS = 256;
-// k_subtree nodes of at most this many points are split by one thread
+// k_subtree nodes of at most this many points are split by one lane each.
 constexpr int LANE_NODE = 32;
 
-// Finishes small segments' whole subtrees in shared memory, level by level:
-// one warp per node above LANE_NODE points, one thread per smaller node.
-// Persistent: each CTA takes segments from the small list until it is
-// exhausted.  (Splitting the first levels' few nodes with
-// the whole block instead was measured slower: a third more subtree time on
-// a 4,096-cloud forest; the warps of the SM's other CTAs already fill the
-// issue slots those levels leave idle.)
+// Finishes the subtrees of small segments in shared memory, one warp per
+// segment, level by level: every node above LANE_NODE points by the whole
+// warp (boxes and ranks by warp reductions and ballots, the split decisions of
+// all of them side by side), the others by one lane each.  A warp waits for no
+// other, so the few nodes of a segment's first levels and the uneven ones of
+// its last cost only their own warp.  Persistent: a warp takes segments from
+// the list until it is exhausted.
 template <typename T, int D>
-__global__ void __launch_bounds__(SUB_THREADS) k_subtree(const Seg<T, D>* small, SoA<T, D> soa, Rec<T, D>* recs,
-                                                         int* root_rec, int cap_pts, int cap_list, int max_leaf,
-                                                         double thr, int rec_cap, BuildCtl* ctl) {
+__global__ void __launch_bounds__(32) k_subtree(const Small<T, D>* small, SoA<T, D> soa, Rec<T, D>* recs, int* root_rec,
+                                                int cap_pts, int cap_list, int max_leaf, double thr, int rec_cap,
+                                                int small_capn, BuildCtl* ctl) {
   extern __shared__ __align__(16) unsigned char smem[];
   T* X[D];
   unsigned char* p = smem;
+#pragma unroll
   for (int d = 0; d < D; d++) {
     X[d] = (T*)p;
     p += sizeof(T) * cap_pts;
   }
   int* ID = (int*)p;
   p += sizeof(int) * cap_pts;
-  int* S = (int*)p;
-  p += sizeof(int) * cap_pts;
-  p = (unsigned char*)(((uintptr_t)p + 15) & ~(uintptr_t)15);
-  Entry<T, D>* LA0 = (Entry<T, D>*)p;
-  Entry<T, D>* LB0 = LA0 + cap_list;
-  int* cnt = (int*)(LB0 + cap_list);  // [0] nA, [1] nB, [2] base, [3] overflow, [4] item
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  Entry<T, D>* LA = (Entry<T, D>*)p;
+  p += sizeof(Entry<T, D>) * cap_list;
+  Entry<T, D>* LB = (Entry<T, D>*)p;
+  p += sizeof(Entry<T, D>) * cap_list;
+  uint16_t* S = (uint16_t*)p;
+  const int lane = threadIdx.x;
+  const unsigned FULL = 0xffffffffu;
   const unsigned lt = (1u << lane) - 1u;
-  const int nsmall = min(ctl->nsmall, INT_MAX);
+  const int nsmall = min(ctl->nsmall, small_capn);
 
   while (true) {
-    if (threadIdx.x == 0) cnt[4] = atomicAdd(&ctl->small_next, 1);
-    __syncthreads();
-    const int item = cnt[4];
-    __syncthreads();
+    int item = 0;
+    if (lane == 0) item = atomicAdd(&ctl->small_next, 1);
+    item = __shfl_sync(FULL, item, 0);
     if (item >= nsmall) break;
-    const Seg<T, D> seg = small[item];
+    const Small<T, D> seg = small[item];
     const int n = seg.e - seg.b;
-    Entry<T, D>* LA = LA0;
-    Entry<T, D>* LB = LB0;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
+    for (int i = lane; i < n; i += 32) {
+#pragma unroll
       for (int d = 0; d < D; d++) X[d][i] = soa.x[d][seg.b + i];
       ID[i] = soa.id[seg.b + i];
     }
-    if (threadIdx.x == 0) {
+    if (lane == 0) {
       Entry<T, D> r;
       r.b = 0;
-      r.e = n;
-      r.parent = seg.parent;
-      r.side = seg.side;
+      r.e = (uint16_t)n;
+      r.up = seg.up;
+#pragma unroll
       for (int d = 0; d < D; d++) {
         r.lo[d] = seg.lo[d];
         r.hi[d] = seg.hi[d];
       }
       LA[0] = r;
-      cnt[0] = 1;
-      cnt[3] = 0;
     }
-    __syncthreads();
-    int levels = 0;
-    while (true) {
-      const int nA = cnt[0];
-      if (nA == 0) break;
+    __syncwarp();
+    int nA = 1, levels = 0;
+    while (nA > 0) {
       if (levels > n + 1) {  // every level splits ranges into strictly smaller ones
-        if (threadIdx.x == 0) atomicExch(&ctl->status, 5);
+        if (lane == 0) atomicExch(&ctl->status, 5);
         break;
       }
-      __syncthreads();
-      if (threadIdx.x == 0) {
-        cnt[1] = 0;
-        cnt[2] = atomicAdd(&ctl->rec_count, nA);
-      }
-      __syncthreads();
-      const int base = cnt[2];
+      int base = 0;
+      if (lane == 0) base = atomicAdd(&ctl->rec_count, nA);
+      base = __shfl_sync(FULL, base, 0);
       levels++;
-      for (int ei = wid; ei < nA; ei += nw) {
-        Entry<T, D> en = LA[ei];
+      int nB = 0;
+      for (int e0 = 0; e0 < nA; e0 += 32) {
+        const int ei = e0 + lane;
+        Entry<T, D> en;
+        en.b = en.e = 0;
+        if (ei < nA) en = LA[ei];
         const int b = en.b, e = en.e, size = e - b;
-        if (size <= LANE_NODE) continue;  // (warp-uniform) one thread's node, below
+        const unsigned large = __ballot_sync(FULL, size > LANE_NODE);
         T mn[D], mx[D];
+#pragma unroll
         for (int d = 0; d < D; d++) {
           mn[d] = Limits<T>::max();
           mx[d] = Limits<T>::lowest();
         }
-        for (int q = b + lane; q < e; q += 32)
+        // tight boxes: of a large node by the warp, of a small one by its lane
+        for (unsigned rest = large; rest; rest &= rest - 1) {
+          const int s = __ffs(rest) - 1;
+          const int nb = __shfl_sync(FULL, b, s), ne = __shfl_sync(FULL, e, s);
+          T lo[D], hi[D];
+#pragma unroll
           for (int d = 0; d < D; d++) {
-            T v = X[d][q];
-            mn[d] = min(mn[d], v);
-            mx[d] = max(mx[d], v);
+            lo[d] = Limits<T>::max();
+            hi[d] = Limits<T>::lowest();
           }
-        for (int d = 0; d < D; d++) {
-          mn[d] = warp_min(mn[d]);
-          mx[d] = warp_max(mx[d]);
+          for (int q = nb + lane; q < ne; q += 32)
+#pragma unroll
+            for (int d = 0; d < D; d++) {
+              const T v = X[d][q];
+              lo[d] = min(lo[d], v);
+              hi[d] = max(hi[d], v);
+            }
+#pragma unroll
+          for (int d = 0; d < D; d++) {
+            lo[d] = warp_min(lo[d]);
+            hi[d] = warp_max(hi[d]);
+            if (lane == s) {
+              mn[d] = lo[d];
+              mx[d] = hi[d];
+            }
+          }
         }
+        const bool tiny = size > 0 && size <= LANE_NODE;
+        if (tiny)
+          for (int q = b; q < e; q++)
+#pragma unroll
+            for (int d = 0; d < D; d++) {
+              const T v = X[d][q];
+              mn[d] = min(mn[d], v);
+              mx[d] = max(mx[d], v);
+            }
         int act = 0, sd = 0;
         T sv = (T)0;
         const int id = base + ei;
-        if (lane == 0) {
+        if (size > 0) {
           Rec<T, D> rec;
-          node_logic<T, D>(size, seg.n_orig, en.parent < 0, en.lo, en.hi, mn, mx, max_leaf, thr, rec, act, sd, sv);
+          node_logic<T, D>(size, seg.n_orig, en.up < 0, en.lo, en.hi, mn, mx, max_leaf, thr, rec, act, sd, sv);
           rec.begin = seg.b + b;
           rec.end = seg.b + e;
-          if (id >= rec_cap) {
-            atomicExch(&ctl->status, 6);
-            act = 0;
-          } else {
-            recs[id] = rec;
-            if (en.parent >= 0) {
-              if (en.side == 0)
-                recs[en.parent].left = id;
-              else
-                recs[en.parent].right = id;
-            } else {
-              root_rec[-en.parent - 1] = id;
-            }
-          }
-          LA[ei] = en;  // keep the trimmed extent for the children
+          if (!link_record<T, D>(rec, id, en.up, recs, rec_cap, root_rec, ctl)) act = 0;
         }
-        act = __shfl_sync(0xffffffffu, act, 0);
-        if (!act) continue;
-        sd = __shfl_sync(0xffffffffu, sd, 0);
-        sv = __shfl_sync(0xffffffffu, sv, 0);
-        T* v = X[sd];
         int L1 = 0, L2 = 0;
-        for (int q0 = b; q0 < e; q0 += 32) {
-          int q = q0 + lane;
-          T x = q < e ? v[q] : sv;
-          bool in = q < e;
-          L1 += __popc(__ballot_sync(0xffffffffu, in && x < sv));
-          L2 += __popc(__ballot_sync(0xffffffffu, in && x <= sv));
-        }
-        const int half = size / 2;
-        for (int pass = 1; pass <= (L1 == L2 ? 1 : 2); pass++) {
-          const int zlo = pass == 1 ? b : b + L1;
-          const int Z = pass == 1 ? b + L1 : b + L2;
-          int G = 0;
-          for (int q0 = zlo; q0 < Z; q0 += 32) {
-            int q = q0 + lane;
-            bool f = false;
-            if (q < Z) {
-              T x = v[q];
-              f = pass == 1 ? !(x < sv) : (x > sv);
-            }
-            unsigned bal = __ballot_sync(0xffffffffu, f);
-            if (f && G + __popc(bal & lt) < half) S[b + G + __popc(bal & lt)] = q;
-            G += __popc(bal);
+        // partition of the large nodes, by the warp
+        for (unsigned rest = __ballot_sync(FULL, size > LANE_NODE && act); rest; rest &= rest - 1) {
+          const int s = __ffs(rest) - 1;
+          const int nb = __shfl_sync(FULL, b, s), ne = __shfl_sync(FULL, e, s), nd = __shfl_sync(FULL, sd, s);
+          const T nv = __shfl_sync(FULL, sv, s);
+          const T* v = X[0];
+#pragma unroll
+          for (int d = 1; d < D; d++)
+            if (d == nd) v = X[d];
+          // bits of the points below the split value: word w is lane w's
+          // (cap_pts <= 1024)
+          unsigned word = 0;
+          int c1 = 0, c2 = 0;
+          for (int q0 = nb, w = 0; q0 < ne; q0 += 32, w++) {
+            const int q = q0 + lane;
+            const bool in = q < ne;
+            const T x = in ? v[q] : nv;
+            const unsigned m = __ballot_sync(FULL, in && x < nv);
+            c1 += __popc(m);
+            c2 += __popc(__ballot_sync(FULL, in && x <= nv));
+            if (lane == w) word = m;
           }
-          int a = 0;
-          for (int q0 = Z; q0 < e; q0 += 32) {
-            int q = q0 + lane;
-            bool f = false;
-            if (q < e) {
-              T x = v[q];
-              f = pass == 1 ? (x < sv) : (x <= sv);
-            }
-            unsigned bal = __ballot_sync(0xffffffffu, f);
-            if (f) {
-              int r = a + __popc(bal & lt);
-              if (r < G && G <= half) S[b + half + (G - 1 - r)] = q;
-            }
-            a += __popc(bal);
-          }
-          if ((a != G || G > half) && lane == 0) atomicExch(&ctl->status, 2);
-          __syncwarp();
-          if (a == G && G <= half)
-            for (int j = lane; j < G; j += 32) {
-              int x = S[b + j], y = S[b + half + j];
-              for (int d = 0; d < D; d++) {
-                T t = X[d][x];
-                X[d][x] = X[d][y];
-                X[d][y] = t;
+          // pass 1: misplaced points ranked from the bits, then swapped
+          const int half = (ne - nb) / 2;
+          {
+            const int Z = nb + c1;
+            int G = 0, a = 0;
+            for (int q0 = nb, w = 0; q0 < ne; q0 += 32, w++) {
+              const int q = q0 + lane;
+              const bool below = __shfl_sync(FULL, word, w) >> lane & 1u;
+              const unsigned bl = __ballot_sync(FULL, q < Z && !below), gr = __ballot_sync(FULL, q >= Z && below);
+              if (bl >> lane & 1u) {
+                const int r = G + __popc(bl & lt);
+                if (r < half) S[nb + r] = (uint16_t)q;
               }
-              int t = ID[x];
-              ID[x] = ID[y];
-              ID[y] = t;
+              if (gr >> lane & 1u) {
+                const int r = a + __popc(gr & lt);
+                if (r < half) S[nb + half + r] = (uint16_t)q;
+              }
+              G += __popc(bl);
+              a += __popc(gr);
             }
-          __syncwarp();
-        }
-        if (lane == 0) {
-          const int si = b + num_left_rule(L1, L2, size);
-          if (id < rec_cap) recs[id].split_index = seg.b + si;
-          const Entry<T, D> par = LA[ei];
-          for (int side = 0; side < 2; side++) {
-            int cb = side ? si : b, ce = side ? e : si;
-            if (cb >= ce) continue;
-            Entry<T, D> c;
-            c.b = cb;
-            c.e = ce;
-            c.parent = id;
-            c.side = side;
-            for (int d = 0; d < D; d++) {
-              c.lo[d] = par.lo[d];
-              c.hi[d] = par.hi[d];
+            if ((a != G || G > half) && lane == 0) atomicExch(&ctl->status, 2);
+            __syncwarp();
+            if (a == G && G <= half)
+              for (int j = lane; j < G; j += 32) {
+                const int x = S[nb + j], y = S[nb + half + G - 1 - j];
+#pragma unroll
+                for (int d = 0; d < D; d++) {
+                  const T t = X[d][x];
+                  X[d][x] = X[d][y];
+                  X[d][y] = t;
+                }
+                const int t = ID[x];
+                ID[x] = ID[y];
+                ID[y] = t;
+              }
+            __syncwarp();
+          }
+          if (c1 != c2) {
+            // pass 2: points equal to the split value to [c1, c2)
+            const int Z = nb + c2;
+            int G = 0, a = 0;
+            for (int q0 = nb + c1; q0 < ne; q0 += 32) {
+              const int q = q0 + lane;
+              const T x = q < ne ? v[q] : nv;
+              const unsigned bl = __ballot_sync(FULL, q < Z && x > nv);
+              const unsigned gr = __ballot_sync(FULL, q < ne && q >= Z && x <= nv);
+              if (bl >> lane & 1u) {
+                const int r = G + __popc(bl & lt);
+                if (r < half) S[nb + r] = (uint16_t)q;
+              }
+              if (gr >> lane & 1u) {
+                const int r = a + __popc(gr & lt);
+                if (r < half) S[nb + half + r] = (uint16_t)q;
+              }
+              G += __popc(bl);
+              a += __popc(gr);
             }
-            if (side == 0)
-              c.hi[sd] = sv;
-            else
-              c.lo[sd] = sv;
-            int slot = atomicAdd(&cnt[1], 1);
-            if (slot < cap_list)
-              LB[slot] = c;
-            else
-              atomicExch(&cnt[3], 1);
+            if ((a != G || G > half) && lane == 0) atomicExch(&ctl->status, 2);
+            __syncwarp();
+            if (a == G && G <= half)
+              for (int j = lane; j < G; j += 32) {
+                const int x = S[nb + j], y = S[nb + half + G - 1 - j];
+#pragma unroll
+                for (int d = 0; d < D; d++) {
+                  const T t = X[d][x];
+                  X[d][x] = X[d][y];
+                  X[d][y] = t;
+                }
+                const int t = ID[x];
+                ID[x] = ID[y];
+                ID[y] = t;
+              }
+            __syncwarp();
+          }
+          if (lane == s) {
+            L1 = c1;
+            L2 = c2;
           }
         }
-      }
-      // nodes of at most LANE_NODE points: one thread each, with the
-      // reference's two converging cursors over shared memory (the pairs a
-      // warp forms by ranks), so that the many small nodes of the last
-      // levels do not each pay a warp's fixed per-node work
-      for (int ei = threadIdx.x; ei < nA; ei += blockDim.x) {
-        Entry<T, D> en = LA[ei];
-        const int b = en.b, e = en.e, size = e - b;
-        if (size > LANE_NODE) continue;
-        T mn[D], mx[D];
-        for (int d = 0; d < D; d++) {
-          mn[d] = Limits<T>::max();
-          mx[d] = Limits<T>::lowest();
-        }
-        for (int q = b; q < e; q++)
-          for (int d = 0; d < D; d++) {
-            const T x = X[d][q];
-            mn[d] = min(mn[d], x);
-            mx[d] = max(mx[d], x);
+        // partition of a small node by its lane, with the reference's two
+        // converging cursors (the pairs a warp forms by ranks)
+        if (tiny && act) {
+          const T* v = X[0];
+#pragma unroll
+          for (int d = 1; d < D; d++)
+            if (d == sd) v = X[d];
+          for (int q = b; q < e; q++) {
+            const T x = v[q];
+            L1 += x < sv;
+            L2 += x <= sv;
           }
-        const int id = base + ei;
-        Rec<T, D> rec;
-        int act = 0, sd = 0;
-        T sv = (T)0;
-        node_logic<T, D>(size, seg.n_orig, en.parent < 0, en.lo, en.hi, mn, mx, max_leaf, thr, rec, act, sd, sv);
-        rec.begin = seg.b + b;
-        rec.end = seg.b + e;
-        if (id >= rec_cap) {
-          atomicExch(&ctl->status, 6);
+          for (int pass = 1; pass <= (L1 == L2 ? 1 : 2); pass++) {
+            const int Z = pass == 1 ? b + L1 : b + L2;
+            int i = pass == 1 ? b : b + L1, j = e - 1;
+            while (true) {
+              while (i < Z && !(pass == 1 ? !(v[i] < sv) : (v[i] > sv))) i++;
+              while (j >= Z && !(pass == 1 ? (v[j] < sv) : (v[j] <= sv))) j--;
+              if (i >= Z || j < Z) break;
+#pragma unroll
+              for (int d = 0; d < D; d++) {
+                const T t = X[d][i];
+                X[d][i] = X[d][j];
+                X[d][j] = t;
+              }
+              const int t = ID[i];
+              ID[i] = ID[j];
+              ID[j] = t;
+              i++;
+              j--;
+            }
+          }
+        }
+        // children, in the order of their parents
+        const int si = b + (act ? num_left_rule(L1, L2, size) : 0);
+        const bool left = act && si > b, right = act && si < e;
+        if (act) recs[id].split_index = seg.b + si;
+        const unsigned ml = __ballot_sync(FULL, left), mr = __ballot_sync(FULL, right);
+        const int more = __popc(ml) + __popc(mr);
+        if (nB + more > cap_list) {
+          if (lane == 0) atomicExch(&ctl->status, 3);
+          nB = 0;
+          e0 = nA;  // (reported; the segment ends here)
           continue;
         }
-        recs[id] = rec;
-        if (en.parent >= 0) {
-          if (en.side == 0)
-            recs[en.parent].left = id;
-          else
-            recs[en.parent].right = id;
-        } else {
-          root_rec[-en.parent - 1] = id;
-        }
-        if (!act) continue;
-        const T* v = X[sd];
-        int L1 = 0, L2 = 0;
-        for (int q = b; q < e; q++) {
-          L1 += v[q] < sv;
-          L2 += v[q] <= sv;
-        }
-        for (int pass = 1; pass <= (L1 == L2 ? 1 : 2); pass++) {
-          const int Z = pass == 1 ? b + L1 : b + L2;
-          int i = pass == 1 ? b : b + L1, j = e - 1;
-          while (true) {
-            while (i < Z && !(pass == 1 ? !(v[i] < sv) : (v[i] > sv))) i++;
-            while (j >= Z && !(pass == 1 ? (v[j] < sv) : (v[j] <= sv))) j--;
-            if (i >= Z || j < Z) break;
-            for (int d = 0; d < D; d++) {
-              const T t = X[d][i];
-              X[d][i] = X[d][j];
-              X[d][j] = t;
-            }
-            const int t = ID[i];
-            ID[i] = ID[j];
-            ID[j] = t;
-            i++;
-            j--;
-          }
-        }
-        const int si = b + num_left_rule(L1, L2, size);
-        recs[id].split_index = seg.b + si;
-        for (int side = 0; side < 2; side++) {
-          const int cb = side ? si : b, ce = side ? e : si;
-          if (cb >= ce) continue;
-          Entry<T, D> c;
-          c.b = cb;
-          c.e = ce;
-          c.parent = id;
-          c.side = side;
+        int slot = nB + __popc(ml & lt) + __popc(mr & lt);
+        Entry<T, D> c;
+        c.b = (uint16_t)b;
+        c.e = (uint16_t)si;
+        c.up = 2 * id;
+        if (left) {
+#pragma unroll
           for (int d = 0; d < D; d++) {
             c.lo[d] = en.lo[d];
+            c.hi[d] = d == sd ? sv : en.hi[d];
+          }
+          LB[slot++] = c;
+        }
+        if (right) {
+          c.b = (uint16_t)si;
+          c.e = (uint16_t)e;
+          c.up = 2 * id + 1;
+#pragma unroll
+          for (int d = 0; d < D; d++) {
+            c.lo[d] = d == sd ? sv : en.lo[d];
             c.hi[d] = en.hi[d];
           }
-          if (side == 0)
-            c.hi[sd] = sv;
-          else
-            c.lo[sd] = sv;
-          const int slot = atomicAdd(&cnt[1], 1);
-          if (slot < cap_list)
-            LB[slot] = c;
-          else
-            atomicExch(&cnt[3], 1);
+          LB[slot] = c;
         }
+        nB += more;
       }
-      __syncthreads();
-      if (threadIdx.x == 0) {
-        cnt[0] = min(cnt[1], cap_list);
-        if (cnt[3]) atomicExch(&ctl->status, 3);
-      }
-      __syncthreads();
+      __syncwarp();
+      nA = nB;
       Entry<T, D>* tmp = LA;
       LA = LB;
       LB = tmp;
     }
-    __syncthreads();
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
+    __syncwarp();
+    for (int i = lane; i < n; i += 32) {
+#pragma unroll
       for (int d = 0; d < D; d++) soa.x[d][seg.b + i] = X[d][i];
       soa.id[seg.b + i] = ID[i];
     }
-    if (threadIdx.x == 0) atomicMax(&ctl->depth, seg.lvl + levels);
-    __syncthreads();
+    if (lane == 0) atomicMax(&ctl->depth, seg.lvl + levels);
+    __syncwarp();
   }
 }
 
@@ -1235,15 +1601,17 @@ static int level_grid(int device) {
   return std::max(nsm, 1) * 8;
 }
 
+// Points of the largest segment that k_subtree takes, its list capacity and
+// its shared memory: 512 float points and their lists take 15 KB, so 14 warps
+// share an SM.  (1,024 points: one level less, but 128 us in place of 80 for
+// the six segments of a 3,001-point cloud.)
 template <typename T, int D>
 int small_capacity(int max_leaf, int& cap_list, size_t& smem) {
-  const size_t budget = 72 * 1024;
-  int cap = sizeof(T) == 4 ? 2048 : 1024;
+  int cap = sizeof(T) <= 4 ? 512 : 256;
   while (true) {
     cap_list = 2 * (cap / (max_leaf + 1)) + 2;
-    smem = (sizeof(T) * D + 2 * sizeof(int)) * (size_t)cap + 16 + 2 * sizeof(Entry<T, D>) * (size_t)cap_list +
-           8 * sizeof(int);
-    if (smem <= budget || cap <= 64) break;
+    smem = (sizeof(T) * D + sizeof(int) + sizeof(uint16_t)) * (size_t)cap + 2 * sizeof(Entry<T, D>) * (size_t)cap_list;
+    if (smem <= 24 * 1024 || cap <= 64) break;
     cap /= 2;
   }
   return cap;
@@ -1311,6 +1679,76 @@ void lower_tnodes(TreeBase* tree, cudaStream_t st) {
   dev_free(tree->tnodes, st);
   tree->tnodes = out;
 }
+
+// Scratch of the grid-wide levels and the launches of one level.
+template <typename T, int D>
+struct Levels {
+  BuildBuf<int> blpos, grpos, tile_seg, tile_lt;
+  BuildBuf<uint32_t> bits;
+  BuildBuf<long long> tile_cnt, tile_off;
+  unsigned gt, gq, gs;
+  BuildCtl* ctl;
+  SoA<T, D> soa;
+  Rec<T, D>* recs;
+  int rec_cap;
+  int* root_rec;
+  int max_leaf;
+  double thr;
+  cudaStream_t st;
+
+  Levels(int64_t n, int max_tiles, int seg_cap, int device, BuildCtl* ctl_, SoA<T, D> soa_, Rec<T, D>* recs_,
+         int rec_cap_, int* root_rec_, int max_leaf_, double thr_, cudaStream_t st_)
+      : blpos(n + 1, st_), grpos(n + 1, st_), tile_seg(max_tiles, st_), tile_lt(max_tiles, st_),
+        bits((size_t)max_tiles * (TILE / 32), st_), tile_cnt(max_tiles, st_), tile_off(max_tiles, st_),
+        gt((unsigned)std::min(max_tiles, level_grid(device))), gq((unsigned)std::min(seg_cap, level_grid(device))),
+        gs((unsigned)div_up(seg_cap, 128)), ctl(ctl_), soa(soa_), recs(recs_), rec_cap(rec_cap_), root_rec(root_rec_),
+        max_leaf(max_leaf_), thr(thr_), st(st_) {}
+
+  // Boxes (where its segments' may be unknown: the roots', and those below a
+  // large segment's split that ties moved), split values and pass 1 of level
+  // lvl.
+  void split(Seg<T, D>* A, int lvl, bool boxes) {
+    if (lvl == 0) {
+      k_tiles<T, D><<<gq, 128, 0, st>>>(A, lvl, tile_seg.get(), ctl);
+      PPTKG_CHECK_LAUNCH();
+    }
+    if (boxes) {
+      k_bbox<T, D><<<gt, BT, 0, st>>>(A, lvl, tile_seg.get(), ctl, soa);
+      PPTKG_CHECK_LAUNCH();
+      k_node<T, D><<<gs, 128, 0, st>>>(A, lvl, ctl, recs, rec_cap, root_rec, max_leaf, thr);
+      PPTKG_CHECK_LAUNCH();
+    }
+    k_split<T, D><<<gt, BT, 0, st>>>(A, lvl, tile_seg.get(), ctl, soa, tile_lt.get(), bits.get());
+    PPTKG_CHECK_LAUNCH();
+    k_ranks<T, D><<<gq, 256, 0, st>>>(A, lvl, tile_lt.get(), bits.get(), tile_off.get(), ctl);
+    PPTKG_CHECK_LAUNCH();
+    k_place_ranks<T, D><<<gt, BT, 0, st>>>(A, lvl, tile_seg.get(), ctl, bits.get(), tile_off.get(), blpos.get(),
+                                           grpos.get());
+    PPTKG_CHECK_LAUNCH();
+    k_swap<T, D><<<gt, BT, 0, st>>>(A, lvl, false, tile_seg.get(), ctl, soa, blpos.get(), grpos.get());
+    PPTKG_CHECK_LAUNCH();
+  }
+  // The tie pass: of small segments (tied 1), of all (2).
+  void tie_pass(Seg<T, D>* A, int lvl, int tied) {
+    if (tied < 1) return;
+    k_ties<T, D><<<gq, BT, 0, st>>>(A, lvl, ctl, soa, blpos.get(), grpos.get());
+    PPTKG_CHECK_LAUNCH();
+    if (tied < 2) return;
+    k_flags<T, D><<<gt, BT, 0, st>>>(A, lvl, tile_seg.get(), ctl, soa, tile_cnt.get());
+    PPTKG_CHECK_LAUNCH();
+    k_tscan<T, D><<<gq, 256, 0, st>>>(A, lvl, tile_cnt.get(), tile_off.get(), ctl);
+    PPTKG_CHECK_LAUNCH();
+    k_scatter<T, D><<<gt, BT, 0, st>>>(A, lvl, tile_seg.get(), ctl, soa, tile_off.get(), blpos.get(), grpos.get());
+    PPTKG_CHECK_LAUNCH();
+    k_swap<T, D><<<gt, BT, 0, st>>>(A, lvl, true, tile_seg.get(), ctl, soa, blpos.get(), grpos.get());
+    PPTKG_CHECK_LAUNCH();
+  }
+  void children(Seg<T, D>* A, int lvl, int tied, Seg<T, D>* B, Small<T, D>* small, int small_capn, int small_cap) {
+    k_children<T, D><<<gs, 128, 0, st>>>(A, lvl, tied, recs, rec_cap, B, small, small_capn, small_cap, max_leaf, thr,
+                                         tile_seg.get(), ctl);
+    PPTKG_CHECK_LAUNCH();
+  }
+};
 
 template <typename T, int D>
 TreeBase* build_forest(const T* d_in, int64_t n, const int64_t* orig_off_h, int ncloud, int max_leaf, double thr,
@@ -1387,13 +1825,15 @@ TreeBase* build_forest(const T* d_in, int64_t n, const int64_t* orig_off_h, int 
   const int seg_cap = nv / (small_cap + 1) + 2;
   const int max_tiles = nv / TILE + seg_cap + 2;
   int small_capn = ncloud + 2 * 64 * (seg_cap + 1);
+  int64_t most = 0;  // points of the largest cloud
+  for (int c = 0; c < ncloud; c++) most = std::max(most, tree->valid_off_h[c + 1] - tree->valid_off_h[c]);
   int depth = 0;
   for (int attempt = 0; attempt < 4; attempt++, small_capn *= 4) {
     Stage st_att("build.attempt", st);
     BuildBuf<BuildCtl> ctl(1, st);
     PPTKG_CUDA(cudaMemsetAsync(ctl.get(), 0, sizeof(BuildCtl), st));
     BuildBuf<Seg<T, D>> segL[2] = {BuildBuf<Seg<T, D>>(seg_cap, st), BuildBuf<Seg<T, D>>(seg_cap, st)};
-    BuildBuf<Seg<T, D>> smallL(small_capn, st);
+    BuildBuf<Small<T, D>> smallL(small_capn, st);
     if (nv > 0) {
       k_roots<T, D><<<div_up(ncloud, 128), 128, 0, st>>>(tree->valid_off, tree->orig_off, ncloud, small_cap,
                                                           segL[0].get(), smallL.get(), small_capn, ctl.get());
@@ -1402,75 +1842,74 @@ TreeBase* build_forest(const T* d_in, int64_t n, const int64_t* orig_off_h, int 
     int levels = 0;
     {
       Stage st_levels("build.levels", st);
-      BuildBuf<int> blpos(nv + 1, st), grpos(nv + 1, st);
-      BuildBuf<int> tile_seg(max_tiles, st);
-      BuildBuf<long long> tile_cnt(max_tiles, st), tile_off(max_tiles, st);
-      const unsigned gt = (unsigned)std::min(max_tiles, level_grid(tree->device));
-      const unsigned gq = (unsigned)std::min(seg_cap, level_grid(tree->device));
-      const unsigned gs = (unsigned)div_up(seg_cap, 128);
-      int h0 = 0;
-      if (nv > 0) {
-        PPTKG_CUDA(cudaMemcpyAsync(&h0, &ctl.get()->level_cnt[0], sizeof(int), cudaMemcpyDeviceToHost, st));
-        PPTKG_CUDA(cudaStreamSynchronize(st));
-      }
-      for (int lvl = 0; h0 > 0 && lvl < MAX_LEVELS; lvl++) {
+      Levels<T, D> lv(nv, max_tiles, seg_cap, tree->device, ctl.get(), soa, recs, (int)rec_cap, tree->root_rec,
+                      max_leaf, thr, st);
+      // Points at a split value are rare in float data: the tie pass is
+      // launched only once a level has asked for it (that level's children,
+      // and so all later levels, wait for the host to notice), and then on
+      // every level until four had none.
+      int tied = 0;
+      // The host looks every fourth level of a large build; of a smaller one
+      // after four, then once the largest cloud may be down to small segments,
+      // and then every second level.  Kernels of a level without segments exit
+      // at once.
+      const bool often = nv < (1 << 21);
+      int look = 2;
+      while (look < 32 && (most >> look) > small_cap) look++;
+      for (int lvl = 0; most > small_cap && lvl < MAX_LEVELS; lvl++) {
         Seg<T, D>* A = segL[lvl & 1].get();
         Seg<T, D>* B = segL[(lvl + 1) & 1].get();
-        k_tiles<T, D><<<1, 1024, 0, st>>>(A, lvl, tile_seg.get(), ctl.get());
-        PPTKG_CHECK_LAUNCH();
-        k_seg_init<T, D><<<gs, 128, 0, st>>>(A, lvl, ctl.get());
-        PPTKG_CHECK_LAUNCH();
-        k_bbox<T, D><<<gt, BT, 0, st>>>(A, tile_seg.get(), ctl.get(), soa);
-        PPTKG_CHECK_LAUNCH();
-        k_node<T, D><<<gs, 128, 0, st>>>(A, lvl, ctl.get(), recs, (int)rec_cap, tree->root_rec, max_leaf, thr);
-        PPTKG_CHECK_LAUNCH();
-        k_count<T, D><<<gt, BT, 0, st>>>(A, tile_seg.get(), ctl.get(), soa);
-        PPTKG_CHECK_LAUNCH();
-        for (int pass = 1; pass <= 2; pass++) {
-          k_flags<T, D><<<gt, BT, 0, st>>>(pass, A, tile_seg.get(), ctl.get(), soa, tile_cnt.get());
-          PPTKG_CHECK_LAUNCH();
-          k_tscan<T, D><<<gq, 256, 0, st>>>(A, lvl, tile_cnt.get(), tile_off.get(), ctl.get());
-          PPTKG_CHECK_LAUNCH();
-          k_scatter<T, D><<<gt, BT, 0, st>>>(pass, A, tile_seg.get(), ctl.get(), soa, tile_off.get(), blpos.get(),
-                                            grpos.get());
-          PPTKG_CHECK_LAUNCH();
-          k_swap<T, D><<<gt, BT, 0, st>>>(A, tile_seg.get(), ctl.get(), soa, blpos.get(), grpos.get());
-          PPTKG_CHECK_LAUNCH();
-        }
-        k_children<T, D><<<gs, 128, 0, st>>>(A, lvl, recs, B, smallL.get(), small_capn, small_cap, ctl.get());
-        PPTKG_CHECK_LAUNCH();
+        lv.split(A, lvl, tied == 2 || lvl == 0);
+        lv.tie_pass(A, lvl, tied);
+        lv.children(A, lvl, tied, B, smallL.get(), small_capn, small_cap);
         levels = lvl + 1;
-        // the host looks at the next level's size every fourth level only;
-        // kernels of a level without segments exit at once
-        if (levels % 4 == 0) {
-          int h = 0;
-          PPTKG_CUDA(cudaMemcpyAsync(&h, &ctl.get()->level_cnt[lvl + 1], sizeof(int), cudaMemcpyDeviceToHost, st));
+        if (often ? levels == look || levels == 4 : levels % 4 == 0) {
+          if (levels == look) look += 2;
+          struct {
+            int ties, big, stalled;
+          } h = {0, 0, 0};
+          int left = 0;
+          PPTKG_CUDA(cudaMemcpyAsync(&left, &ctl.get()->level_cnt[lvl + 1], sizeof(int), cudaMemcpyDeviceToHost, st));
+          PPTKG_CUDA(cudaMemcpyAsync(&h, &ctl.get()->ties, sizeof(h), cudaMemcpyDeviceToHost, st));
           PPTKG_CUDA(cudaStreamSynchronize(st));
-          if (h == 0) break;
+          if (tied == 2 && h.big < levels - 3) tied = 1;
+          if (tied == 1 && h.ties < levels - 3) tied = 0;
+          if (h.stalled > 0) {
+            // back to the level that waits (the later ones found no segments)
+            lvl = h.stalled - 1;
+            Seg<T, D>* W = segL[lvl & 1].get();
+            Seg<T, D>* X = segL[(lvl + 1) & 1].get();
+            tied = h.big == h.stalled ? 2 : 1;
+            PPTKG_CUDA(cudaMemsetAsync(&ctl.get()->stalled, 0, sizeof(int), st));
+            lv.tie_pass(W, lvl, tied);
+            lv.children(W, lvl, tied, X, smallL.get(), small_capn, small_cap);
+            levels = lvl + 1;
+            continue;
+          }
+          if (left == 0) break;
         }
       }
     }
-    BuildCtl hctl;
-    PPTKG_CUDA(cudaMemcpyAsync(&hctl, ctl.get(), sizeof(BuildCtl), cudaMemcpyDeviceToHost, st));
-    PPTKG_CUDA(cudaStreamSynchronize(st));
-    if (hctl.status == 7) continue;  // small list too short: retry with more room
-    if (hctl.status) throw Error(E_DEVICE, "device build: partition check failed (code " + std::to_string(hctl.status) + ")");
     if (levels >= MAX_LEVELS) throw Error(E_DEVICE, "device build: more than 4096 levels of large nodes");
     depth = levels;
-    if (hctl.nsmall > 0) {
+    BuildCtl hctl;  // (its scalars)
+    {
       Stage st_sub("build.subtree", st);
       PPTKG_CUDA(cudaFuncSetAttribute(k_subtree<T, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
       int per_sm = 1, nsm = 1;
-      PPTKG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_subtree<T, D>, SUB_THREADS, smem));
+      PPTKG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_subtree<T, D>, 32, smem));
       PPTKG_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, tree->device));
-      const int grid = std::max(1, std::min(hctl.nsmall, std::max(per_sm, 1) * nsm));
-      k_subtree<T, D><<<grid, SUB_THREADS, smem, st>>>(smallL.get(), soa, recs, tree->root_rec, small_cap, cap_list,
-                                                       max_leaf, thr, (int)rec_cap, ctl.get());
+      const int grid = std::max(1, std::min(small_capn, std::max(per_sm, 1) * nsm));
+      k_subtree<T, D><<<grid, 32, smem, st>>>(smallL.get(), soa, recs, tree->root_rec, small_cap, cap_list, max_leaf,
+                                              thr, (int)rec_cap, small_capn, ctl.get());
       PPTKG_CHECK_LAUNCH();
-      PPTKG_CUDA(cudaMemcpyAsync(&hctl, ctl.get(), sizeof(BuildCtl), cudaMemcpyDeviceToHost, st));
+      PPTKG_CUDA(cudaMemcpyAsync(&hctl, ctl.get(), offsetof(BuildCtl, level_cnt), cudaMemcpyDeviceToHost, st));
       PPTKG_CUDA(cudaStreamSynchronize(st));
+      // small list too short: again with more room (the points are partitioned
+      // by now, so every pass of the second attempt finds them in place)
+      if (hctl.status == 7 && attempt < 3) continue;
       if (hctl.status)
-        throw Error(E_DEVICE, "device build: subtree check failed (code " + std::to_string(hctl.status) + ")");
+        throw Error(E_DEVICE, "device build: check failed (code " + std::to_string(hctl.status) + ")");
     }
     tree->n_recs = hctl.rec_count;
     tree->levels = levels;
@@ -1626,7 +2065,7 @@ void forest_capture_ready(TreeBase* t, cudaStream_t st) {
     throw Error(E_INVALID, "forest too large for capture mode");
   int per_sm = 1, nsm = 1;
   PPTKG_CUDA(cudaFuncSetAttribute(k_subtree<T, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  PPTKG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_subtree<T, D>, SUB_THREADS, smem));
+  PPTKG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_subtree<T, D>, 32, smem));
   PPTKG_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, t->device));
   t->cap_subgrid = std::max(per_sm, 1) * nsm;
   // capacity-sized arrays, current contents kept
@@ -1690,51 +2129,27 @@ void rebuild_forest(TreeBase* t, const T* d_in, cudaStream_t st, int* status) {
   PPTKG_CUDA(cudaMemsetAsync(ctl.get(), 0, sizeof(BuildCtl), st));
   PPTKG_CUDA(cudaMemsetAsync(t->root_rec, 0xff, sizeof(int) * ncloud, st));
   BuildBuf<Seg<T, D>> segL[2] = {BuildBuf<Seg<T, D>>(seg_cap, st), BuildBuf<Seg<T, D>>(seg_cap, st)};
-  BuildBuf<Seg<T, D>> smallL(t->cap_small, st);
+  BuildBuf<Small<T, D>> smallL(t->cap_small, st);
   k_roots<T, D><<<div_up(ncloud, 128), 128, 0, st>>>(t->valid_off, t->orig_off, ncloud, small_cap, segL[0].get(),
                                                       smallL.get(), t->cap_small, ctl.get());
   PPTKG_CHECK_LAUNCH();
   {
     // a fixed number of levels; the kernels of a level without segments
     // return at once
-    BuildBuf<int> blpos(n + 1, st), grpos(n + 1, st);
-    BuildBuf<int> tile_seg(max_tiles, st);
-    BuildBuf<long long> tile_cnt(max_tiles, st), tile_off(max_tiles, st);
-    const unsigned gt = (unsigned)std::min(max_tiles, level_grid(t->device));
-    const unsigned gq = (unsigned)std::min(seg_cap, level_grid(t->device));
-    const unsigned gs = (unsigned)div_up(seg_cap, 128);
+    Levels<T, D> lv(n, max_tiles, seg_cap, t->device, ctl.get(), soa, recs, rec_cap, t->root_rec, t->max_leaf,
+                    t->empty_split, st);
     for (int lvl = 0; lvl < t->cap_levels; lvl++) {
       Seg<T, D>* A = segL[lvl & 1].get();
       Seg<T, D>* B = segL[(lvl + 1) & 1].get();
-      k_tiles<T, D><<<1, 1024, 0, st>>>(A, lvl, tile_seg.get(), ctl.get());
-      PPTKG_CHECK_LAUNCH();
-      k_seg_init<T, D><<<gs, 128, 0, st>>>(A, lvl, ctl.get());
-      PPTKG_CHECK_LAUNCH();
-      k_bbox<T, D><<<gt, BT, 0, st>>>(A, tile_seg.get(), ctl.get(), soa);
-      PPTKG_CHECK_LAUNCH();
-      k_node<T, D><<<gs, 128, 0, st>>>(A, lvl, ctl.get(), recs, rec_cap, t->root_rec, t->max_leaf, t->empty_split);
-      PPTKG_CHECK_LAUNCH();
-      k_count<T, D><<<gt, BT, 0, st>>>(A, tile_seg.get(), ctl.get(), soa);
-      PPTKG_CHECK_LAUNCH();
-      for (int pass = 1; pass <= 2; pass++) {
-        k_flags<T, D><<<gt, BT, 0, st>>>(pass, A, tile_seg.get(), ctl.get(), soa, tile_cnt.get());
-        PPTKG_CHECK_LAUNCH();
-        k_tscan<T, D><<<gq, 256, 0, st>>>(A, lvl, tile_cnt.get(), tile_off.get(), ctl.get());
-        PPTKG_CHECK_LAUNCH();
-        k_scatter<T, D><<<gt, BT, 0, st>>>(pass, A, tile_seg.get(), ctl.get(), soa, tile_off.get(), blpos.get(),
-                                          grpos.get());
-        PPTKG_CHECK_LAUNCH();
-        k_swap<T, D><<<gt, BT, 0, st>>>(A, tile_seg.get(), ctl.get(), soa, blpos.get(), grpos.get());
-        PPTKG_CHECK_LAUNCH();
-      }
-      k_children<T, D><<<gs, 128, 0, st>>>(A, lvl, recs, B, smallL.get(), t->cap_small, small_cap, ctl.get());
-      PPTKG_CHECK_LAUNCH();
+      lv.split(A, lvl, true);
+      lv.tie_pass(A, lvl, 2);
+      lv.children(A, lvl, 2, B, smallL.get(), t->cap_small, small_cap);
     }
   }
   // the persistent subtree kernel takes the small segments; blocks without
   // work return
-  k_subtree<T, D><<<t->cap_subgrid, SUB_THREADS, smem, st>>>(smallL.get(), soa, recs, t->root_rec, small_cap, cap_list,
-                                                             t->max_leaf, t->empty_split, rec_cap, ctl.get());
+  k_subtree<T, D><<<t->cap_subgrid, 32, smem, st>>>(smallL.get(), soa, recs, t->root_rec, small_cap, cap_list,
+                                                             t->max_leaf, t->empty_split, rec_cap, t->cap_small, ctl.get());
   PPTKG_CHECK_LAUNCH();
   k_rebuild_status<<<1, 1, 0, st>>>(ctl.get(), t->cap_levels, t->tdepth, status, t->dev_meta, t->valid_off, ncloud);
   PPTKG_CHECK_LAUNCH();
