@@ -1088,15 +1088,6 @@ void with_loader(const TreeBase* t, const QuerySpec& qs, F&& f) {
   }
 }
 
-// make_order, or (small warp-per-query batches) the queries as they come,
-// their indices checked all the same.
-template <typename T, int D>
-int ordered_unless(bool as_is, const TreeBase* t, const QuerySpec& qs, DevBuf<int>& order, cudaStream_t st) {
-  if (!as_is) return make_order<T, D>(t, qs, order, st);
-  check_indices(t, qs, st);
-  return 0;
-}
-
 template <typename T, int D>
 int64_t rnear_count(const TreeBase* t, const QuerySpec& qs, double dmax, int64_t* d_off, cudaStream_t st) {
   typedef typename DistOf<T>::type DistT;
@@ -1109,7 +1100,9 @@ int64_t rnear_count(const TreeBase* t, const QuerySpec& qs, double dmax, int64_t
   PPTKG_CUDA(cudaMemsetAsync(status.get(), 0, sizeof(int), st));
   DevBuf<int> order;
   const bool warps = rnear_by_warp(t->nv, m);
-  const int mode = ordered_unless<T, D>(warps && m <= WARP_UNSORTED, t, qs, order, st);
+  // (sorted for either walk: neighbours share the ids they copy; 20k queries
+  // of 45k hits take 4.7 ms in no order, 3.3 sorted)
+  const int mode = make_order<T, D>(t, qs, order, st);
   const DistT r2 = radius2<DistT>(dmax);
   const size_t smem = QWARPS * rnear_smem_bytes<T, D>(t->tdepth);
   Stage stage("rnear_count", st);
@@ -1143,7 +1136,9 @@ void rnear_fill(const TreeBase* t, const QuerySpec& qs, double dmax, const int64
   PPTKG_CUDA(cudaMemsetAsync(status.get(), 0, sizeof(int), st));
   DevBuf<int> order;
   const bool warps = rnear_by_warp(t->nv, m);
-  const int mode = ordered_unless<T, D>(warps && m <= WARP_UNSORTED, t, qs, order, st);
+  // (sorted for either walk: neighbours share the ids they copy; 20k queries
+  // of 45k hits take 4.7 ms in no order, 3.3 sorted)
+  const int mode = make_order<T, D>(t, qs, order, st);
   const DistT r2 = radius2<DistT>(dmax);
   const size_t smem = QWARPS * rnear_smem_bytes<T, D>(t->tdepth);
   Stage stage("rnear_fill", st);
@@ -1797,7 +1792,11 @@ void normals_query(const TreeBase* t, const QuerySpec& qs_in, int k, float r, in
   // (tree order covers valid points only: rows of dropped points, none when
   // n == nv, need no separate pass)
   const bool warps = k == -1 ? rnear_by_warp(t->nv, m) : by_warp(t->nv, m, k);
-  const int mode = ordered_unless<T, 3>(warps && m <= WARP_UNSORTED, t, qs, order, st);
+  int mode = 0;
+  if (k > 0 && warps && m <= WARP_UNSORTED)
+    check_indices(t, qs, st);
+  else
+    mode = make_order<T, 3>(t, qs, order, st);
   // the radius travels as a C float (estimate_normals.cpp:264) and is cast to
   // the input type (:17-22) before being squared in the distance type
   const DistT rr = (DistT)(T)r;
