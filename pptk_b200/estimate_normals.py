@@ -13,7 +13,7 @@ import time
 import numpy as np
 
 from . import _native as N
-from ._args import as_points_2d, extract_indices
+from ._args import as_points_2d, extract_indices, extract_indices_cuda
 
 _FLOAT_CODES = {np.dtype(np.float32): 0, np.dtype(np.float64): 1}
 PRECISIONS = {"auto": N.PREC_AUTO, "fp32": N.PREC_FP32, "fp64": N.PREC_FP64}
@@ -114,13 +114,16 @@ def estimate_normals(points, k, r, subsample=None, output_eigenvalues=False, out
 
     sub = None
     if subsample is not None:
-        sub_obj = subsample.cpu().numpy() if N.is_torch_cuda(subsample) else subsample
-        sub = extract_indices(sub_obj, n)
+        on_device = use_torch and N.is_torch_cuda(subsample) and subsample.device == device
+        sub = extract_indices_cuda(subsample, n) if on_device else None
         if sub is None:
-            raise TypeError("subsample must be interpretable as specifying a subset of points")
-        if use_torch:
-            import torch
-            sub = torch.from_numpy(sub).to(device)
+            sub_obj = subsample.cpu().numpy() if N.is_torch_cuda(subsample) else subsample
+            sub = extract_indices(sub_obj, n)
+            if sub is None:
+                raise TypeError("subsample must be interpretable as specifying a subset of points")
+            if use_torch:
+                import torch
+                sub = torch.from_numpy(sub).to(device)
     m = n if sub is None else int(sub.shape[0])
 
     if precision not in PRECISIONS:

@@ -15,7 +15,7 @@ import math
 import numpy as np
 
 from . import _native as N
-from ._args import as_points_2d, cast_as_float_rounded, extract_indices
+from ._args import as_points_2d, cast_as_float_rounded, extract_indices, extract_indices_cuda
 
 _UNSET = object()
 _FLOAT_CODES = {np.dtype(np.float32): 0, np.dtype(np.float64): 1}
@@ -187,8 +187,10 @@ class _Batch:
                 self.qdtype = 0 if q.dtype == torch.float32 else 1
                 self.m = int(q.shape[0])
                 return
-            idx = extract_indices(queries.cpu().numpy(), tree.n_valid)
-            self.indices = torch.from_numpy(idx).to(queries.device)
+            idx = extract_indices_cuda(queries, tree.n_valid)
+            if idx is None:
+                idx = torch.from_numpy(extract_indices(queries.cpu().numpy(), tree.n_valid)).to(queries.device)
+            self.indices = idx
             self.m = int(idx.shape[0])
             return
         if isinstance(queries, np.ndarray) and queries.ndim == 2:
