@@ -267,6 +267,8 @@ struct WarpScratch {
   int* stack;
   PointRec<T, D>* buf;                   // 32 entries (r-near staging)
   int* log;                              // per-lane neighbour lists, lane-strided; null when unused
+  WNode<T, D>* nodes;                    // the 32 nodes of a step (kNN)
+  typename DistOf<T>::type* box;         // the packet's two boxes: [2][lo, hi][D] (kNN)
 };
 
 // A lane's query as the rest of its warp reads it during a bucket scan:
@@ -490,16 +492,21 @@ __device__ bool wide_knn(const TreeView<T, D>& tv, int root, const DistT* q, int
   }
   const unsigned far = __reduce_max_sync(FULL, jump > 0.f ? __float_as_uint(jump) : 0u);
   const int cut = far ? __ffs(__ballot_sync(FULL, jump > 0.f && __float_as_uint(jump) == far)) - 1 : 32;
-  DistT plo[2][D], phi[2][D];
+  // (in shared memory: a step reads them as broadcasts, and the lists need
+  // the registers)
 #pragma unroll
   for (int b = 0; b < 2; b++) {
     const bool in = active && (lane >= cut) == (b == 1);
 #pragma unroll
     for (int d = 0; d < D; d++) {
-      plo[b][d] = lanes_min(in ? q[d] : (DistT)INFINITY);
-      phi[b][d] = lanes_max(in ? q[d] : (DistT)-INFINITY);
+      const DistT lo = lanes_min(in ? q[d] : (DistT)INFINITY), hi = lanes_max(in ? q[d] : (DistT)-INFINITY);
+      if (lane == 0) {
+        ws.box[2 * D * b + d] = lo;
+        ws.box[2 * D * b + D + d] = hi;
+      }
     }
   }
+  __syncwarp();
   auto reach = [&]() {
     const DistT w = top.worst() < r2 ? top.worst() : r2;
     return __reduce_max_sync(FULL, active && w >= (DistT)0 ? __float_as_uint(float_above(w)) : 0u);
@@ -521,30 +528,27 @@ __device__ bool wide_knn(const TreeView<T, D>& tv, int root, const DistT* q, int
     bool hit = lane < cnt && w.cnt != 0;
     unsigned md = 0;
     if (hit && started) {
-      md = __float_as_uint(fminf(packet_min_dist2<T, DistT, D>(w.lo, w.hi, plo[0], phi[0]),
-                                 packet_min_dist2<T, DistT, D>(w.lo, w.hi, plo[1], phi[1])));
+      md = __float_as_uint(fminf(packet_min_dist2<T, DistT, D>(w.lo, w.hi, ws.box, ws.box + D),
+                                 packet_min_dist2<T, DistT, D>(w.lo, w.hi, ws.box + 2 * D, ws.box + 3 * D)));
       hit = md <= rmax && !(at + lane >= h0 && at + lane < h1);
     }
     unsigned hm = __ballot_sync(FULL, hit);
     if (hm) {
       if (__any_sync(FULL, hit && w.cnt > 0)) {
         // leaf ranges, nearest first, until none is within reach
+        __syncwarp();
+        if (hit) ws.nodes[lane] = w;
+        __syncwarp();
         do {
           const unsigned near = __reduce_min_sync(FULL, hit ? md : 0xffffffffu);
           if (near > rmax) break;
           const int s = __ffs(__ballot_sync(FULL, hit && md == near)) - 1;
           if (lane == s) hit = false;
           hm &= ~(1u << s);
-          T lo[D], hi[D];
-#pragma unroll
-          for (int d = 0; d < D; d++) {
-            lo[d] = __shfl_sync(FULL, w.lo[d], s);
-            hi[d] = __shfl_sync(FULL, w.hi[d], s);
-          }
-          const int begin = __shfl_sync(FULL, w.begin, s), n = __shfl_sync(FULL, w.cnt, s);
-          const bool mine = need(box_min_dist2<T, DistT, D>(lo, hi, q));
+          const WNode<T, D> leaf = ws.nodes[s];
+          const bool mine = need(box_min_dist2<T, DistT, D>(leaf.lo, leaf.hi, q));
           if (__any_sync(FULL, mine)) {
-            scan(begin, n, mine);
+            scan(leaf.begin, leaf.cnt, mine);
             rmax = reach();
           }
         } while (hm);

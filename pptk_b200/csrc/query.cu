@@ -71,12 +71,13 @@ __device__ __forceinline__ WarpScratch<T, D> rnear_scratch(int depth) {
   return ws;
 }
 
-// kNN walks: the queries, the stack, and (normals) `logcap` list slots per lane.
+// kNN walks: the queries, the stack, a step's nodes, the packet's boxes, and
+// (normals) `logcap` list slots per lane.
 template <typename T, int D>
 __host__ __device__ __forceinline__ size_t warp_smem_bytes(int stack, int logcap = 0) {
   typedef typename DistOf<T>::type DistT;
-  return stage_bytes<T, D>() + (((size_t)stack * sizeof(int2) + 15) & ~(size_t)15) +
-         (size_t)logcap * 32 * 4;
+  return stage_bytes<T, D>() + (((size_t)stack * sizeof(int2) + 15) & ~(size_t)15) + 32 * sizeof(WNode<T, D>) +
+         ((4 * D * sizeof(DistT) + 15) & ~(size_t)15) + (size_t)logcap * 32 * 4;
 }
 
 template <typename T, int D>
@@ -90,12 +91,16 @@ __device__ __forceinline__ WarpScratch<T, D> warp_scratch(int stack, int logcap 
   base += stage_bytes<T, D>();
   ws.stack = (int*)base;
   base += ((size_t)stack * sizeof(int2) + 15) & ~(size_t)15;
+  ws.nodes = (WNode<T, D>*)base;
+  base += 32 * sizeof(WNode<T, D>);
+  ws.box = (DistT*)base;
+  base += (4 * D * sizeof(DistT) + 15) & ~(size_t)15;
   ws.log = logcap ? (int*)base : nullptr;
   return ws;
 }
 
 // Candidate-log capacity per lane of the normals kernel.
-__host__ __device__ constexpr int normals_logcap(int kmax) { return 2 * kmax; }
+__host__ __device__ constexpr int normals_logcap(int kmax) { return kmax; }
 
 // ------------------------------------------------------------- loaders ----
 // Query i is row i of a user array.
@@ -516,10 +521,23 @@ int make_order(const TreeBase* t, const QuerySpec& qs, DevBuf<int>& order, cudaS
 }
 
 // ----------------------------------------------------------------- kNN ----
+// warm_mult of a batch of m queries on nv points: one more where packets
+// span over 256 tree positions and lists are short.  Their queries' walks
+// share less, so candidates found before them save more (1M scattered
+// queries, k = 16: 2.35 -> 2.10 ms; queries in tree order: 31.8 -> 32.7).
+inline int warm_window(int64_t nv, int64_t m, int kmax) {
+  return g_tune_warm_mult.load() + (kmax <= 16 && 32 * nv > 256 * m ? 1 : 0);
+}
+
 // Blocks per SM the kNN kernel is compiled for: float top-k lists of up to
-// 16 entries fit 96 registers (5 blocks of 128 threads); larger lists keep
-// the compiler's register count.
-constexpr int knn_min_blocks(int kmax, int dist_bytes) { return (dist_bytes == 4 && kmax <= 16) ? 5 : (dist_bytes == 4 && kmax <= 32) ? 4 : 1; }
+// 16 entries run in 80 registers (6 blocks of 128 threads; spills of 200 B
+// cost less than the sixth block gives: 1M scattered queries 2.54 ms at 5
+// blocks, 2.35 at 6, 2.34 at 7, all-point normals 34.1 / 31.8 / 33.3), of up
+// to 32 in 128 (5 blocks spill 780 B: 56.7 against 54.1 ms of kNN k = 32);
+// larger lists keep the compiler's register count.
+constexpr int knn_min_blocks(int kmax, int dist_bytes) {
+  return (dist_bytes == 4 && kmax <= 16) ? 6 : (dist_bytes == 4 && kmax <= 32) ? 4 : 1;
+}
 
 template <typename T, int D, int KMAX, typename L>
 __global__ void __launch_bounds__(QTHREADS, knn_min_blocks(KMAX, sizeof(typename DistOf<T>::type))) k_knn(TreeView<T, D> tv, L ld, const int* order, int order_mode, int m,
@@ -573,7 +591,7 @@ void launch_knn(const TreeBase* t, L ld, const int* order, int mode, int m, int 
   k_knn<T, D, KMAX, L><<<div_up(m, QTHREADS), QTHREADS, smem, st>>>(view_of<T, D>(t), ld, order, mode, m, k, r2,
                                                                       d_idx, d_cnt, status, fm,
                                                                       g_tune_warm_bound.load() != 0,
-                                                                      g_tune_warm_mult.load());
+                                                                      warm_window(t->nv, m, KMAX));
   PPTKG_CHECK_LAUNCH();
 }
 
@@ -1231,9 +1249,11 @@ __device__ __forceinline__ void write_invalid(int row, int num_eigen, T* evecs, 
   if (sizes) sizes[row] = 0;
 }
 
-// Blocks per SM that the register budget of a normals kernel aims for: the
-// top-k list takes 2 (float) or 3 (double) registers per slot.
+// Blocks per SM that the register budget of a normals kernel aims for: that
+// of the kNN kernel for float lists of up to 16 entries, otherwise the top-k
+// list's 2 (float) or 3 (double) registers per slot and some for the rest.
 constexpr int normals_min_blocks(int kmax, int dist_bytes, int prec) {
+  if (dist_bytes == 4 && kmax <= 16 && prec == PREC_FP32) return knn_min_blocks(kmax, dist_bytes);
   const int need = kmax * (dist_bytes == 4 ? 2 : 3) + (prec == PREC_FP32 ? 64 : 72);
   const int b = 65536 / (QTHREADS * need);
   return b < 1 ? 1 : (b > 8 ? 8 : b);
@@ -1648,7 +1668,7 @@ void launch_normals(const TreeBase* t, L ld, const int* order, int mode, int m, 
         cudaFuncSetAttribute(k_normals<T, KMAX, L, PREC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   k_normals<T, KMAX, L, PREC><<<div_up(m, QTHREADS), QTHREADS, smem, st>>>(
       view_of<T, 3>(t), ld, order, mode, m, k, r2, num_eigen, gap_thr, ev, ew, sz, fix, nfix, status, fm,
-      g_tune_warm_bound.load() != 0, g_tune_warm_mult.load(), kidx, kcnt);
+      g_tune_warm_bound.load() != 0, warm_window(t->nv, m, KMAX), kidx, kcnt);
   PPTKG_CHECK_LAUNCH();
 }
 
@@ -2085,11 +2105,12 @@ void multi_tables(const TreeBase* const* trees, int ntrees, const int64_t* rows,
 
 // A stand-in tree carrying the batch-wide traversal bounds for the launch
 // helpers (which size shared memory from the tree they are given).
-static TreeBase* bounds_tree(int depth, int n_nodes, int wlevels) {
+static TreeBase* bounds_tree(int depth, int n_nodes, int wlevels, int64_t nv) {
   TreeBase* b = new TreeBase();
   b->tdepth = depth;
   b->n_tnodes = n_nodes;
   b->wlevels = wlevels;
+  b->nv = nv;
   return b;
 }
 
@@ -2143,7 +2164,7 @@ void multi_knn(const TreeBase* const* trees, int ntrees, const void* d_q, int qd
       qs.m = rows[g + 1] - rows[g];
       return qs;
     }, st, true);
-  std::unique_ptr<TreeBase> bt(bounds_tree(mt.depth, mt.n_nodes, mt.wlevels));
+  std::unique_ptr<TreeBase> bt(bounds_tree(mt.depth, mt.n_nodes, mt.wlevels, mt.nv));
   DevBuf<int> status(1, st);
   PPTKG_CUDA(cudaMemsetAsync(status.get(), 0, sizeof(int), st));
   const DistT r2 = radius2<DistT>(dmax);
@@ -2183,7 +2204,7 @@ void multi_normals(const TreeBase* const* trees, int ntrees, const int32_t* d_id
       qs.exclude_self = false;
       return qs;
     }, st);
-  std::unique_ptr<TreeBase> bt(bounds_tree(mt.depth, mt.n_nodes, mt.wlevels));
+  std::unique_ptr<TreeBase> bt(bounds_tree(mt.depth, mt.n_nodes, mt.wlevels, mt.nv));
   DevBuf<int> status(1, st);
   PPTKG_CUDA(cudaMemsetAsync(status.get(), 0, sizeof(int), st));
   const DistT rr = (DistT)(T)r;
