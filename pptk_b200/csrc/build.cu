@@ -5,7 +5,7 @@
 // The reference builds depth first; every node only permutes the indices of
 // its own range, so building all nodes of a level at once gives the same
 // permutation.  Nodes with more than `small_cap` points are processed by
-// grid-wide kernels over 4096-point tiles; smaller subtrees are finished by
+// grid-wide kernels over tiles of points; smaller subtrees are finished by
 // one warp each, entirely in shared memory.
 //
 // The reference partition (PartitionIndices, kdtree-impl.h:192-246) is two
@@ -25,9 +25,13 @@ namespace pptkg {
 
 constexpr int BT = 256;     // threads per tile block
 constexpr int SWAP_U = 4;   // pairs a k_swap thread has in flight
-constexpr int SPLIT_U = 8;  // points a k_split thread has in flight
-constexpr int TILE = 4096;  // points per tile
-constexpr int TITEMS = TILE / BT;
+constexpr int SPLIT_U = 4;  // points a k_split thread has in flight
+// Points per tile of a level: 4,096, or 1,024 in builds of less than 4M
+// points, whose levels would otherwise leave SMs without a tile (200k points:
+// 49 tiles, a level's pass over them 15 us against 7).  A multiple of
+// SPLIT_U x BT, at most 16 x BT.
+inline int tile_points(int64_t n) { return n < ((int64_t)1 << 22) ? 1024 : 4096; }
+static_assert(1024 % (SPLIT_U * BT) == 0 && 4096 <= 16 * BT, "tiles are whole steps of a block, 16 points a thread");
 
 template <typename T, int D>
 struct Seg {
@@ -75,6 +79,7 @@ struct BuildCtl {
   int big;      // 1 + the last level with such points in a segment too large for one block
   int stalled;  // 1 + the level that waits for a tie pass that the host has not launched
   int unboxed;  // 1 + the last level with segments whose box is not known
+  int tile;     // points per tile
   int level_cnt[MAX_LEVELS + 1];    // large segments per level
   int level_tiles[MAX_LEVELS + 1];  // their tiles
 };
@@ -223,8 +228,8 @@ __device__ __forceinline__ void seg_clear(Seg<T, D>& g) {
 
 // A large segment takes its tiles and its record.
 template <typename T, int D>
-__device__ __forceinline__ void take_place(Seg<T, D>& g, int lvl, BuildCtl* ctl) {
-  g.ntiles = div_up_dev(g.e - g.b, TILE);
+__device__ __forceinline__ void take_place(Seg<T, D>& g, int lvl, int tile, BuildCtl* ctl) {
+  g.ntiles = div_up_dev(g.e - g.b, tile);
   g.tile0 = atomicAdd(&ctl->level_tiles[lvl], g.ntiles);
   g.rec = atomicAdd(&ctl->rec_count, 1);
 }
@@ -263,9 +268,10 @@ static __global__ void k_cloud_off(const int* off, const int64_t* orig_off, int 
 // launched with upper-bound grids and read the live counts from the device,
 // so the host never waits between levels.
 template <typename T, int D>
-__global__ void k_roots(const int64_t* valid_off, const int64_t* orig_off, int ncloud, int small_cap, Seg<T, D>* lvl0,
-                        Small<T, D>* small, int small_capn, BuildCtl* ctl) {
+__global__ void k_roots(const int64_t* valid_off, const int64_t* orig_off, int ncloud, int small_cap, int tile,
+                        Seg<T, D>* lvl0, Small<T, D>* small, int small_capn, BuildCtl* ctl) {
   int c = blockIdx.x * blockDim.x + threadIdx.x;
+  if (c == 0) ctl->tile = tile;
   if (c >= ncloud) return;
   const int b = (int)valid_off[c], e = (int)valid_off[c + 1];
   if (e <= b) return;
@@ -284,7 +290,7 @@ __global__ void k_roots(const int64_t* valid_off, const int64_t* orig_off, int n
   seg_clear(g);
   if (e - b > small_cap) {
     ctl->unboxed = 1;
-    take_place(g, 0, ctl);
+    take_place(g, 0, tile, ctl);
     lvl0[atomicAdd(&ctl->level_cnt[0], 1)] = g;
   } else {
     const int slot = atomicAdd(&ctl->nsmall, 1);
@@ -310,11 +316,11 @@ __global__ void k_tiles(const Seg<T, D>* segs, int lvl, int* tile_seg, const Bui
 // capture-mode rebuild) costs a few hundred idle blocks, not one per tile of
 // the largest level.
 template <typename T, int D>
-__device__ __forceinline__ void tile_at(const Seg<T, D>* segs, const int* tile_seg, int t, int& s, int& start,
+__device__ __forceinline__ void tile_at(const Seg<T, D>* segs, const int* tile_seg, int t, int tile, int& s, int& start,
                                         int& end) {
   s = tile_seg[t];
-  start = segs[s].b + (t - segs[s].tile0) * TILE;
-  end = min(start + TILE, segs[s].e);
+  start = segs[s].b + (t - segs[s].tile0) * tile;
+  end = min(start + tile, segs[s].e);
 }
 
 template <typename T>
@@ -351,11 +357,11 @@ __global__ void __launch_bounds__(BT) k_bbox(Seg<T, D>* segs, int lvl, const int
                                              SoA<T, D> soa) {
   __shared__ T shmn[D][BT / 32], shmx[D][BT / 32];
   if (ctl->unboxed != lvl + 1) return;
-  const int ntiles = ctl->level_tiles[lvl];
+  const int ntiles = ctl->level_tiles[lvl], tile = ctl->tile;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
     int s, start, end;
-    tile_at(segs, tile_seg, t, s, start, end);
+    tile_at(segs, tile_seg, t, tile, s, start, end);
     if (segs[s].boxed) continue;  // (uniform over the block)
     T mn[D], mx[D];
 #pragma unroll
@@ -456,11 +462,11 @@ __global__ void __launch_bounds__(BT) k_split(Seg<T, D>* segs, int lvl, const in
   typedef typename OrdOf<T>::type U;
   __shared__ U shb[BT / 32][4 * D];
   __shared__ int shc[BT / 32][2];
-  const int ntiles = ctl->level_tiles[lvl];
+  const int ntiles = ctl->level_tiles[lvl], tile = ctl->tile;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
     int s, start, end;
-    tile_at(segs, tile_seg, t, s, start, end);
+    tile_at(segs, tile_seg, t, tile, s, start, end);
     if (!segs[s].act) continue;  // (uniform over the block)
     const T sv = segs[s].sv;
     const int sd = segs[s].sd;
@@ -476,7 +482,7 @@ __global__ void __launch_bounds__(BT) k_split(Seg<T, D>* segs, int lvl, const in
     // a full tile needs no test of its end; the loads of SPLIT_U points are
     // issued together
     auto points = [&](auto full) {
-      for (int j0 = 0; j0 < TITEMS; j0 += SPLIT_U) {
+      for (int j0 = 0; j0 < tile / BT; j0 += SPLIT_U) {
         T x[SPLIT_U][D];
         bool in[SPLIT_U];
 #pragma unroll
@@ -508,11 +514,11 @@ __global__ void __launch_bounds__(BT) k_split(Seg<T, D>* segs, int lvl, const in
           }
           const unsigned m = __ballot_sync(0xffffffffu, below);
           c1 += __popc(m);
-          if (lane == 0) tile_bits[(size_t)t * (TILE / 32) + (j0 + u) * (BT / 32) + wid] = m;
+          if (lane == 0) tile_bits[(size_t)t * (tile / 32) + (j0 + u) * (BT / 32) + wid] = m;
         }
       }
     };
-    if (start + TILE <= end)
+    if (start + tile <= end)
       points(std::true_type());
     else
       points(std::false_type());
@@ -561,17 +567,17 @@ template <typename T, int D>
 __global__ void k_ranks(Seg<T, D>* segs, int lvl, const int* tile_lt, const uint32_t* tile_bits, long long* tile_off,
                         BuildCtl* ctl) {
   __shared__ long long sh[33];
-  const int nseg = ctl->level_cnt[lvl];
+  const int nseg = ctl->level_cnt[lvl], tile = ctl->tile;
   for (int si = blockIdx.x; si < nseg; si += gridDim.x) {
     Seg<T, D>& g = segs[si];
     if (!g.act) continue;  // (uniform over the block)
     const int b = g.b, Z = b + g.L1;
     // points below the split value among the first Z - start of the tile that
     // holds Z (one word per thread)
-    const int mid = g.L1 / TILE, n = g.L1 - mid * TILE;
+    const int mid = g.L1 / tile, n = g.L1 - mid * tile;
     int in = 0;
-    if (mid < g.ntiles && threadIdx.x <= n >> 5 && threadIdx.x < TILE / 32) {
-      const uint32_t w = tile_bits[(size_t)(g.tile0 + mid) * (TILE / 32) + threadIdx.x];
+    if (mid < g.ntiles && threadIdx.x <= n >> 5 && threadIdx.x < tile / 32) {
+      const uint32_t w = tile_bits[(size_t)(g.tile0 + mid) * (tile / 32) + threadIdx.x];
       in = __popc(threadIdx.x < n >> 5 ? w : w & ((1u << (n & 31)) - 1u));
     }
     const int left = (int)block_sum((long long)in, sh);
@@ -580,7 +586,7 @@ __global__ void k_ranks(Seg<T, D>* segs, int lvl, const int* tile_lt, const uint
       const int t = c0 + threadIdx.x;
       long long v = 0;
       if (t < g.ntiles) {
-        const int start = b + t * TILE, end = min(start + TILE, g.e), lt = tile_lt[g.tile0 + t];
+        const int start = b + t * tile, end = min(start + tile, g.e), lt = tile_lt[g.tile0 + t];
         if (end <= Z) {
           v = end - start - lt;
         } else if (start >= Z) {
@@ -612,18 +618,19 @@ __global__ void __launch_bounds__(BT) k_place_ranks(Seg<T, D>* segs, int lvl, co
                                                     const BuildCtl* ctl, const uint32_t* tile_bits, const long long* tile_off, int* blpos,
                                                     int* grpos) {
   __shared__ long long sh[33];
-  const int ntiles = ctl->level_tiles[lvl];
+  const int ntiles = ctl->level_tiles[lvl], tile = ctl->tile;
   for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
     int s, start, end;
-    tile_at(segs, tile_seg, t, s, start, end);
+    tile_at(segs, tile_seg, t, tile, s, start, end);
     if (!segs[s].act) continue;  // (uniform over the block)
     const int b = segs[s].b, Z = b + segs[s].L1, G = segs[s].G, size = segs[s].e - b;
-    // 16 positions per thread: half a word
-    static_assert(TITEMS == 16, "half a word of the tile's bits per thread");
-    const int i0 = start + threadIdx.x * TITEMS;
-    const unsigned below = tile_bits[(size_t)t * (TILE / 32) + (threadIdx.x >> 1)] >> (16 * (threadIdx.x & 1)) & 0xffffu;
-    const unsigned in = i0 >= end ? 0u : end - i0 >= TITEMS ? 0xffffu : (1u << (end - i0)) - 1u;
-    const unsigned left = i0 >= Z ? 0u : Z - i0 >= TITEMS ? 0xffffu : (1u << (Z - i0)) - 1u;
+    // tile / BT positions per thread (4 or 16): a part of a word
+    const int items = tile / BT, bit0 = threadIdx.x * items;
+    const int i0 = start + bit0;
+    const unsigned all = (1u << items) - 1u;
+    const unsigned below = tile_bits[(size_t)t * (tile / 32) + (bit0 >> 5)] >> (bit0 & 31) & all;
+    const unsigned in = i0 >= end ? 0u : end - i0 >= items ? all : (1u << (end - i0)) - 1u;
+    const unsigned left = i0 >= Z ? 0u : Z - i0 >= items ? all : (1u << (Z - i0)) - 1u;
     unsigned mbl = in & left & ~below, mgr = in & ~left & below;
     const long long mine = (long long)__popc(mbl) + ((long long)__popc(mgr) << 32);
     long long tot;
@@ -760,10 +767,10 @@ __global__ void __launch_bounds__(BT) k_flags(Seg<T, D>* segs, int lvl, const in
                                               SoA<T, D> soa, long long* tile_cnt) {
   __shared__ long long sh[33];
   if (ctl->big != lvl + 1) return;
-  const int ntiles = ctl->level_tiles[lvl];
+  const int ntiles = ctl->level_tiles[lvl], tile = ctl->tile;
   for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
     int s, start, end;
-    tile_at(segs, tile_seg, t, s, start, end);
+    tile_at(segs, tile_seg, t, tile, s, start, end);
     long long c = 0;
     if (segs[s].act && big_tie(segs[s])) {
       const T sv = segs[s].sv;
@@ -810,18 +817,17 @@ __global__ void __launch_bounds__(BT) k_scatter(Seg<T, D>* segs, int lvl, const 
                                                 SoA<T, D> soa, const long long* tile_off, int* blpos, int* grpos) {
   __shared__ long long sh[33];
   if (ctl->big != lvl + 1) return;
-  const int ntiles = ctl->level_tiles[lvl];
+  const int ntiles = ctl->level_tiles[lvl], tile = ctl->tile;
   for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
     int s, start, end;
-    tile_at(segs, tile_seg, t, s, start, end);
+    tile_at(segs, tile_seg, t, tile, s, start, end);
     if (!segs[s].act || !big_tie(segs[s])) continue;  // (uniform over the block)
     const T sv = segs[s].sv;
     const T* v = soa.x[segs[s].sd];
     const int b = segs[s].b, L1 = segs[s].L1, L2 = segs[s].L2, G = segs[s].G;
-    const int i0 = start + threadIdx.x * TITEMS;
+    const int items = tile / BT, i0 = start + threadIdx.x * items;
     unsigned mbl = 0, mgr = 0;
-#pragma unroll
-    for (int j = 0; j < TITEMS; j++) {
+    for (int j = 0; j < items; j++) {
       int i = i0 + j;
       if (i < end) {
         bool bl, gr;
@@ -835,8 +841,7 @@ __global__ void __launch_bounds__(BT) k_scatter(Seg<T, D>* segs, int lvl, const 
     long long ex = block_excl_scan(mine, sh, tot) + tile_off[t];
     int rb = (int)(ex & 0xffffffffll), rg = (int)(ex >> 32);
     const int size = segs[s].e - b;
-#pragma unroll
-    for (int j = 0; j < TITEMS; j++) {
+    for (int j = 0; j < items; j++) {
       if (mbl >> j & 1) {
         if (rb < size) blpos[b + rb] = i0 + j;
         rb++;
@@ -855,10 +860,10 @@ template <typename T, int D>
 __global__ void __launch_bounds__(BT) k_swap(Seg<T, D>* segs, int lvl, bool tie, const int* tile_seg, BuildCtl* ctl,
                                              SoA<T, D> soa, const int* blpos, const int* grpos) {
   if (tie && ctl->big != lvl + 1) return;
-  const int ntiles = ctl->level_tiles[lvl];
+  const int ntiles = ctl->level_tiles[lvl], tile = ctl->tile;
   for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
     int s, start, end;
-    tile_at(segs, tile_seg, t, s, start, end);
+    tile_at(segs, tile_seg, t, tile, s, start, end);
     if (!segs[s].act) continue;
     if (tie && !big_tie(segs[s])) continue;
     const int b = segs[s].b, e = segs[s].e, G = segs[s].G;
@@ -909,31 +914,31 @@ __global__ void __launch_bounds__(BT) k_swap(Seg<T, D>* segs, int lvl, bool tie,
   }
 }
 
-// The children of a level's segments: a lane per segment makes them, decides
-// those that stay large, and the warp writes the map of their tiles.
+// The children of a level's segments: a lane per child makes it and decides
+// it if it stays large, and the warp writes the map of the tiles.  (Bound by
+// the decisions' serial arithmetic: both children on one lane took 24 us for
+// the 400 segments of a 200k-point build's last level.)
 template <typename T, int D>
 __global__ void k_children(Seg<T, D>* segs, int lvl, int tied, Rec<T, D>* recs, int rec_cap, Seg<T, D>* next,
                            Small<T, D>* small, int small_capn, int small_cap_pts, int max_leaf, double thr,
                            int* tile_seg, BuildCtl* ctl) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31;
+  const int c0 = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31;
+  const int i = c0 >> 1, side = c0 & 1;
   // a level whose ties had no pass (tied 0: none was launched, 1: that of
   // small segments) waits for it
   if ((tied < 1 && ctl->ties == lvl + 1) || (tied < 2 && ctl->big == lvl + 1)) {
-    if (i == 0) ctl->stalled = lvl + 1;
+    if (c0 == 0) ctl->stalled = lvl + 1;
     return;
   }
   const int nseg = ctl->level_cnt[lvl];
-  if ((i & ~31) >= nseg) return;
-  int t0[2] = {0, 0}, nt[2] = {0, 0}, at[2] = {0, 0};
+  if ((c0 & ~31) >> 1 >= nseg) return;
+  int t0 = 0, nt = 0, at = 0;
   if (i < nseg && segs[i].act) {
     const Seg<T, D>& g = segs[i];
-    const int count = g.e - g.b;
-    const int si = g.b + num_left_rule(g.L1, g.L2, count);
-    recs[g.rec].split_index = si;
-#pragma unroll
-    for (int side = 0; side < 2; side++) {
-      const int cb = side ? si : g.b, ce = side ? g.e : si;
-      if (cb >= ce) continue;
+    const int si = g.b + num_left_rule(g.L1, g.L2, g.e - g.b);
+    if (side == 0) recs[g.rec].split_index = si;
+    const int cb = side ? si : g.b, ce = side ? g.e : si;
+    if (cb < ce) {
       Seg<T, D> c;
       c.b = cb;
       c.e = ce;
@@ -943,16 +948,12 @@ __global__ void k_children(Seg<T, D>* segs, int lvl, int tied, Rec<T, D>* recs, 
       c.rec = -1;
       c.n_orig = g.n_orig;
       for (int d = 0; d < D; d++) {
-        c.lo[d] = g.lo[d];
-        c.hi[d] = g.hi[d];
+        c.lo[d] = side == 1 && d == g.sd ? g.sv : g.lo[d];
+        c.hi[d] = side == 0 && d == g.sd ? g.sv : g.hi[d];
       }
-      if (side == 0)
-        c.hi[g.sd] = g.sv;
-      else
-        c.lo[g.sd] = g.sv;
       if (ce - cb > small_cap_pts) {
         seg_clear(c);
-        take_place(c, lvl + 1, ctl);
+        take_place(c, lvl + 1, ctl->tile, ctl);
         if (si == g.b + g.L1 || !big_tie(g)) {
           for (int d = 0; d < D; d++) {
             c.tlo[d] = g.clo[side][d];
@@ -962,10 +963,10 @@ __global__ void k_children(Seg<T, D>* segs, int lvl, int tied, Rec<T, D>* recs, 
         } else {
           ctl->unboxed = lvl + 2;
         }
-        t0[side] = c.tile0;
-        nt[side] = c.ntiles;
-        at[side] = atomicAdd(&ctl->level_cnt[lvl + 1], 1);
-        next[at[side]] = c;
+        t0 = c.tile0;
+        nt = c.ntiles;
+        at = atomicAdd(&ctl->level_cnt[lvl + 1], 1);
+        next[at] = c;
       } else {
         const int slot = atomicAdd(&ctl->nsmall, 1);
         if (slot < small_capn)
@@ -975,14 +976,12 @@ __global__ void k_children(Seg<T, D>* segs, int lvl, int tied, Rec<T, D>* recs, 
       }
     }
   }
-#pragma unroll
-  for (int side = 0; side < 2; side++)
-    for (unsigned rest = __ballot_sync(0xffffffffu, nt[side] > 0); rest; rest &= rest - 1) {
-      const int s = __ffs(rest) - 1;
-      const int a = __shfl_sync(0xffffffffu, t0[side], s), n = __shfl_sync(0xffffffffu, nt[side], s),
-                k = __shfl_sync(0xffffffffu, at[side], s);
-      for (int t = lane; t < n; t += 32) tile_seg[a + t] = k;
-    }
+  for (unsigned rest = __ballot_sync(0xffffffffu, nt > 0); rest; rest &= rest - 1) {
+    const int s = __ffs(rest) - 1;
+    const int a = __shfl_sync(0xffffffffu, t0, s), n = __shfl_sync(0xffffffffu, nt, s),
+              k = __shfl_sync(0xffffffffu, at, s);
+    for (int t = lane; t < n; t += 32) tile_seg[a + t] = k;
+  }
 }
 
 // ------------------------------------------------- per-warp subtrees ----
@@ -1372,11 +1371,15 @@ __global__ void k_tfill(const Rec<T, D>* recs, int n_recs, const int* flag, cons
 template <typename T, int D>
 __global__ void k_troots(const Rec<T, D>* recs, const int* root_rec, const int64_t* valid_off, int ncloud,
                          const int* flag, const int* tid, int nt, TNode<T, D>* nodes, int* root_tnode,
-                         const int* nt_dev = nullptr) {
+                         double* box = nullptr) {
   int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= ncloud) return;
-  if (nt_dev) nt = *nt_dev;  // the node count on the device
   const int r = root_rec[c];
+  if (box && c == 0)  // the first cloud's box
+    for (int d = 0; d < D; d++) {
+      box[d] = r >= 0 ? (double)recs[r].lo[d] : 0.0;
+      box[4 + d] = r >= 0 ? (double)recs[r].hi[d] : 0.0;
+    }
   TNode<T, D> t;
   for (int k = 0; k < 2; k++)
     for (int d = 0; d < D; d++) {
@@ -1680,12 +1683,40 @@ void lower_tnodes(TreeBase* tree, cudaStream_t st) {
   tree->tnodes = out;
 }
 
-// Scratch of the grid-wide levels and the launches of one level.
+// k_subtree's grid: the warps that the shared memory of a device's SMs holds
+// (its dynamic part stays below the 48 KB that need no opt-in).
+static int subtree_grid(size_t smem, int device) {
+  int nsm = 148, per_sm = 228 * 1024;
+  PPTKG_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device));
+  PPTKG_CUDA(cudaDeviceGetAttribute(&per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, device));
+  return std::max(nsm, 1) * std::max(1, std::min(32, (int)(per_sm / (smem + 1024))));
+}
+
+// A stretch of a scratch block, handed out piece by piece (base null: only
+// measured).
+struct Carve {
+  char* base;
+  size_t at = 0;
+  template <typename V>
+  V* take(size_t n) {
+    V* p = base ? reinterpret_cast<V*>(base + at) : nullptr;
+    at += (n * sizeof(V) + 255) & ~(size_t)255;
+    return p;
+  }
+};
+
+// Scratch of a build's levels, one block of device memory (an allocation of
+// its own for each of the eleven arrays took 30 us of a small build), and the
+// launches of one level.
 template <typename T, int D>
 struct Levels {
-  BuildBuf<int> blpos, grpos, tile_seg, tile_lt;
-  BuildBuf<uint32_t> bits;
-  BuildBuf<long long> tile_cnt, tile_off;
+  BuildBuf<char> block;
+  Seg<T, D>* seg[2];
+  Small<T, D>* small;
+  int small_capn, small_cap;
+  int *blpos, *grpos, *tile_seg, *tile_lt;
+  uint32_t* bits;
+  long long *tile_cnt, *tile_off;
   unsigned gt, gq, gs;
   BuildCtl* ctl;
   SoA<T, D> soa;
@@ -1696,56 +1727,74 @@ struct Levels {
   double thr;
   cudaStream_t st;
 
-  Levels(int64_t n, int max_tiles, int seg_cap, int device, BuildCtl* ctl_, SoA<T, D> soa_, Rec<T, D>* recs_,
-         int rec_cap_, int* root_rec_, int max_leaf_, double thr_, cudaStream_t st_)
-      : blpos(n + 1, st_), grpos(n + 1, st_), tile_seg(max_tiles, st_), tile_lt(max_tiles, st_),
-        bits((size_t)max_tiles * (TILE / 32), st_), tile_cnt(max_tiles, st_), tile_off(max_tiles, st_),
+  void carve(Carve c, int64_t n, int tile, int max_tiles, int seg_cap, size_t* bytes) {
+    ctl = c.take<BuildCtl>(1);
+    for (auto& x : seg) x = c.take<Seg<T, D>>(seg_cap);
+    small = c.take<Small<T, D>>(small_capn);
+    blpos = c.take<int>(n + 1);
+    grpos = c.take<int>(n + 1);
+    tile_seg = c.take<int>(max_tiles);
+    tile_lt = c.take<int>(max_tiles);
+    bits = c.take<uint32_t>((size_t)max_tiles * (tile / 32));
+    tile_cnt = c.take<long long>(max_tiles);
+    tile_off = c.take<long long>(max_tiles);
+    if (bytes) *bytes = c.at;
+  }
+  Levels(int64_t n, int tile, int max_tiles, int seg_cap, int small_capn_, int small_cap_, int device, SoA<T, D> soa_,
+         Rec<T, D>* recs_, int rec_cap_, int* root_rec_, int max_leaf_, double thr_, cudaStream_t st_)
+      : small_capn(small_capn_), small_cap(small_cap_),
         gt((unsigned)std::min(max_tiles, level_grid(device))), gq((unsigned)std::min(seg_cap, level_grid(device))),
-        gs((unsigned)div_up(seg_cap, 128)), ctl(ctl_), soa(soa_), recs(recs_), rec_cap(rec_cap_), root_rec(root_rec_),
-        max_leaf(max_leaf_), thr(thr_), st(st_) {}
+        gs((unsigned)div_up(seg_cap, 128)), soa(soa_), recs(recs_), rec_cap(rec_cap_), root_rec(root_rec_),
+        max_leaf(max_leaf_), thr(thr_), st(st_) {
+    size_t bytes = 0;
+    carve(Carve{nullptr}, n, tile, max_tiles, seg_cap, &bytes);
+    block.alloc(bytes, st);
+    carve(Carve{block.get()}, n, tile, max_tiles, seg_cap, nullptr);
+    PPTKG_CUDA(cudaMemsetAsync(ctl, 0, sizeof(BuildCtl), st));
+  }
 
   // Boxes (where its segments' may be unknown: the roots', and those below a
   // large segment's split that ties moved), split values and pass 1 of level
   // lvl.
   void split(Seg<T, D>* A, int lvl, bool boxes) {
     if (lvl == 0) {
-      k_tiles<T, D><<<gq, 128, 0, st>>>(A, lvl, tile_seg.get(), ctl);
+      k_tiles<T, D><<<gq, 128, 0, st>>>(A, lvl, tile_seg, ctl);
       PPTKG_CHECK_LAUNCH();
     }
     if (boxes) {
-      k_bbox<T, D><<<gt, BT, 0, st>>>(A, lvl, tile_seg.get(), ctl, soa);
+      k_bbox<T, D><<<gt, BT, 0, st>>>(A, lvl, tile_seg, ctl, soa);
       PPTKG_CHECK_LAUNCH();
       k_node<T, D><<<gs, 128, 0, st>>>(A, lvl, ctl, recs, rec_cap, root_rec, max_leaf, thr);
       PPTKG_CHECK_LAUNCH();
     }
-    k_split<T, D><<<gt, BT, 0, st>>>(A, lvl, tile_seg.get(), ctl, soa, tile_lt.get(), bits.get());
+    k_split<T, D><<<gt, BT, 0, st>>>(A, lvl, tile_seg, ctl, soa, tile_lt, bits);
     PPTKG_CHECK_LAUNCH();
-    k_ranks<T, D><<<gq, 256, 0, st>>>(A, lvl, tile_lt.get(), bits.get(), tile_off.get(), ctl);
+    k_ranks<T, D><<<gq, 256, 0, st>>>(A, lvl, tile_lt, bits, tile_off, ctl);
     PPTKG_CHECK_LAUNCH();
-    k_place_ranks<T, D><<<gt, BT, 0, st>>>(A, lvl, tile_seg.get(), ctl, bits.get(), tile_off.get(), blpos.get(),
-                                           grpos.get());
+    k_place_ranks<T, D><<<gt, BT, 0, st>>>(A, lvl, tile_seg, ctl, bits, tile_off, blpos,
+                                           grpos);
     PPTKG_CHECK_LAUNCH();
-    k_swap<T, D><<<gt, BT, 0, st>>>(A, lvl, false, tile_seg.get(), ctl, soa, blpos.get(), grpos.get());
+    k_swap<T, D><<<gt, BT, 0, st>>>(A, lvl, false, tile_seg, ctl, soa, blpos, grpos);
     PPTKG_CHECK_LAUNCH();
   }
   // The tie pass: of small segments (tied 1), of all (2).
   void tie_pass(Seg<T, D>* A, int lvl, int tied) {
     if (tied < 1) return;
-    k_ties<T, D><<<gq, BT, 0, st>>>(A, lvl, ctl, soa, blpos.get(), grpos.get());
+    k_ties<T, D><<<gq, BT, 0, st>>>(A, lvl, ctl, soa, blpos, grpos);
     PPTKG_CHECK_LAUNCH();
     if (tied < 2) return;
-    k_flags<T, D><<<gt, BT, 0, st>>>(A, lvl, tile_seg.get(), ctl, soa, tile_cnt.get());
+    k_flags<T, D><<<gt, BT, 0, st>>>(A, lvl, tile_seg, ctl, soa, tile_cnt);
     PPTKG_CHECK_LAUNCH();
-    k_tscan<T, D><<<gq, 256, 0, st>>>(A, lvl, tile_cnt.get(), tile_off.get(), ctl);
+    k_tscan<T, D><<<gq, 256, 0, st>>>(A, lvl, tile_cnt, tile_off, ctl);
     PPTKG_CHECK_LAUNCH();
-    k_scatter<T, D><<<gt, BT, 0, st>>>(A, lvl, tile_seg.get(), ctl, soa, tile_off.get(), blpos.get(), grpos.get());
+    k_scatter<T, D><<<gt, BT, 0, st>>>(A, lvl, tile_seg, ctl, soa, tile_off, blpos, grpos);
     PPTKG_CHECK_LAUNCH();
-    k_swap<T, D><<<gt, BT, 0, st>>>(A, lvl, true, tile_seg.get(), ctl, soa, blpos.get(), grpos.get());
+    k_swap<T, D><<<gt, BT, 0, st>>>(A, lvl, true, tile_seg, ctl, soa, blpos, grpos);
     PPTKG_CHECK_LAUNCH();
   }
-  void children(Seg<T, D>* A, int lvl, int tied, Seg<T, D>* B, Small<T, D>* small, int small_capn, int small_cap) {
-    k_children<T, D><<<gs, 128, 0, st>>>(A, lvl, tied, recs, rec_cap, B, small, small_capn, small_cap, max_leaf, thr,
-                                         tile_seg.get(), ctl);
+  void children(Seg<T, D>* A, int lvl, int tied, Seg<T, D>* B) {
+    k_children<T, D><<<2 * gs, 128, 0, st>>>(A, lvl, tied, recs, rec_cap, B, small, small_capn, small_cap, max_leaf, thr,
+                                         tile_seg, ctl);
     PPTKG_CHECK_LAUNCH();
   }
 };
@@ -1823,27 +1872,24 @@ TreeBase* build_forest(const T* d_in, int64_t n, const int64_t* orig_off_h, int 
 
   // large segments per level are disjoint and above small_cap points
   const int seg_cap = nv / (small_cap + 1) + 2;
-  const int max_tiles = nv / TILE + seg_cap + 2;
+  const int max_tiles = nv / tile_points(n) + seg_cap + 2;
   int small_capn = ncloud + 2 * 64 * (seg_cap + 1);
   int64_t most = 0;  // points of the largest cloud
   for (int c = 0; c < ncloud; c++) most = std::max(most, tree->valid_off_h[c + 1] - tree->valid_off_h[c]);
   int depth = 0;
   for (int attempt = 0; attempt < 4; attempt++, small_capn *= 4) {
     Stage st_att("build.attempt", st);
-    BuildBuf<BuildCtl> ctl(1, st);
-    PPTKG_CUDA(cudaMemsetAsync(ctl.get(), 0, sizeof(BuildCtl), st));
-    BuildBuf<Seg<T, D>> segL[2] = {BuildBuf<Seg<T, D>>(seg_cap, st), BuildBuf<Seg<T, D>>(seg_cap, st)};
-    BuildBuf<Small<T, D>> smallL(small_capn, st);
+    Levels<T, D> lv(nv, tile_points(n), max_tiles, seg_cap, small_capn, small_cap, tree->device, soa, recs, (int)rec_cap,
+                    tree->root_rec, max_leaf, thr, st);
+    BuildCtl* ctl = lv.ctl;
     if (nv > 0) {
       k_roots<T, D><<<div_up(ncloud, 128), 128, 0, st>>>(tree->valid_off, tree->orig_off, ncloud, small_cap,
-                                                          segL[0].get(), smallL.get(), small_capn, ctl.get());
+                                                          tile_points(n), lv.seg[0], lv.small, small_capn, ctl);
       PPTKG_CHECK_LAUNCH();
     }
     int levels = 0;
     {
       Stage st_levels("build.levels", st);
-      Levels<T, D> lv(nv, max_tiles, seg_cap, tree->device, ctl.get(), soa, recs, (int)rec_cap, tree->root_rec,
-                      max_leaf, thr, st);
       // Points at a split value are rare in float data: the tie pass is
       // launched only once a level has asked for it (that level's children,
       // and so all later levels, wait for the host to notice), and then on
@@ -1857,11 +1903,11 @@ TreeBase* build_forest(const T* d_in, int64_t n, const int64_t* orig_off_h, int 
       int look = 2;
       while (look < 32 && (most >> look) > small_cap) look++;
       for (int lvl = 0; most > small_cap && lvl < MAX_LEVELS; lvl++) {
-        Seg<T, D>* A = segL[lvl & 1].get();
-        Seg<T, D>* B = segL[(lvl + 1) & 1].get();
+        Seg<T, D>* A = lv.seg[lvl & 1];
+        Seg<T, D>* B = lv.seg[(lvl + 1) & 1];
         lv.split(A, lvl, tied == 2 || lvl == 0);
         lv.tie_pass(A, lvl, tied);
-        lv.children(A, lvl, tied, B, smallL.get(), small_capn, small_cap);
+        lv.children(A, lvl, tied, B);
         levels = lvl + 1;
         if (often ? levels == look || levels == 4 : levels % 4 == 0) {
           if (levels == look) look += 2;
@@ -1869,20 +1915,20 @@ TreeBase* build_forest(const T* d_in, int64_t n, const int64_t* orig_off_h, int 
             int ties, big, stalled;
           } h = {0, 0, 0};
           int left = 0;
-          PPTKG_CUDA(cudaMemcpyAsync(&left, &ctl.get()->level_cnt[lvl + 1], sizeof(int), cudaMemcpyDeviceToHost, st));
-          PPTKG_CUDA(cudaMemcpyAsync(&h, &ctl.get()->ties, sizeof(h), cudaMemcpyDeviceToHost, st));
+          PPTKG_CUDA(cudaMemcpyAsync(&left, &ctl->level_cnt[lvl + 1], sizeof(int), cudaMemcpyDeviceToHost, st));
+          PPTKG_CUDA(cudaMemcpyAsync(&h, &ctl->ties, sizeof(h), cudaMemcpyDeviceToHost, st));
           PPTKG_CUDA(cudaStreamSynchronize(st));
           if (tied == 2 && h.big < levels - 3) tied = 1;
           if (tied == 1 && h.ties < levels - 3) tied = 0;
           if (h.stalled > 0) {
             // back to the level that waits (the later ones found no segments)
             lvl = h.stalled - 1;
-            Seg<T, D>* W = segL[lvl & 1].get();
-            Seg<T, D>* X = segL[(lvl + 1) & 1].get();
+            Seg<T, D>* W = lv.seg[lvl & 1];
+            Seg<T, D>* X = lv.seg[(lvl + 1) & 1];
             tied = h.big == h.stalled ? 2 : 1;
-            PPTKG_CUDA(cudaMemsetAsync(&ctl.get()->stalled, 0, sizeof(int), st));
+            PPTKG_CUDA(cudaMemsetAsync(&ctl->stalled, 0, sizeof(int), st));
             lv.tie_pass(W, lvl, tied);
-            lv.children(W, lvl, tied, X, smallL.get(), small_capn, small_cap);
+            lv.children(W, lvl, tied, X);
             levels = lvl + 1;
             continue;
           }
@@ -1895,15 +1941,11 @@ TreeBase* build_forest(const T* d_in, int64_t n, const int64_t* orig_off_h, int 
     BuildCtl hctl;  // (its scalars)
     {
       Stage st_sub("build.subtree", st);
-      PPTKG_CUDA(cudaFuncSetAttribute(k_subtree<T, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-      int per_sm = 1, nsm = 1;
-      PPTKG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_subtree<T, D>, 32, smem));
-      PPTKG_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, tree->device));
-      const int grid = std::max(1, std::min(small_capn, std::max(per_sm, 1) * nsm));
-      k_subtree<T, D><<<grid, 32, smem, st>>>(smallL.get(), soa, recs, tree->root_rec, small_cap, cap_list, max_leaf,
-                                              thr, (int)rec_cap, small_capn, ctl.get());
+      const int grid = std::max(1, std::min(small_capn, subtree_grid(smem, tree->device)));
+      k_subtree<T, D><<<grid, 32, smem, st>>>(lv.small, soa, recs, tree->root_rec, small_cap, cap_list, max_leaf,
+                                              thr, (int)rec_cap, small_capn, ctl);
       PPTKG_CHECK_LAUNCH();
-      PPTKG_CUDA(cudaMemcpyAsync(&hctl, ctl.get(), offsetof(BuildCtl, level_cnt), cudaMemcpyDeviceToHost, st));
+      PPTKG_CUDA(cudaMemcpyAsync(&hctl, ctl, offsetof(BuildCtl, level_cnt), cudaMemcpyDeviceToHost, st));
       PPTKG_CUDA(cudaStreamSynchronize(st));
       // small list too short: again with more room (the points are partitioned
       // by now, so every pass of the second attempt finds them in place)
@@ -1945,19 +1987,6 @@ TreeBase* build_forest(const T* d_in, int64_t n, const int64_t* orig_off_h, int 
     make_tnodes<T, D>(tree.get(), bucket, st);
   }
 
-  Stage st_root("build.root", st);
-  Rec<T, D> r0;
-  int root0 = -1;
-  PPTKG_CUDA(cudaMemcpyAsync(&root0, tree->root_rec, sizeof(int), cudaMemcpyDeviceToHost, st));
-  PPTKG_CUDA(cudaStreamSynchronize(st));
-  if (root0 >= 0) {
-    PPTKG_CUDA(cudaMemcpyAsync(&r0, (Rec<T, D>*)tree->recs + root0, sizeof(r0), cudaMemcpyDeviceToHost, st));
-    PPTKG_CUDA(cudaStreamSynchronize(st));
-    for (int d = 0; d < D; d++) {
-      tree->root_lo[d] = (double)r0.lo[d];
-      tree->root_hi[d] = (double)r0.hi[d];
-    }
-  }
   if constexpr (std::is_integral<T>::value) lower_points<T, D>(tree.get(), st);
   return tree.release();
 }
@@ -1979,6 +2008,7 @@ void make_tnodes(TreeBase* tree, int bucket, cudaStream_t st) {
   const int nr = tree->n_recs;
   const Rec<T, D>* recs = (const Rec<T, D>*)tree->recs;
   BuildBuf<int> flag(nr + 1, st), tid(nr + 1, st);
+  BuildBuf<double> boxbuf(8, st);
   int nt = 0, n_wide = 0;
   wide_begin<T, D>(tree, nr, st);
   PPTKG_CUDA(cudaMemcpyAsync(&n_wide, tree->wrank + (int64_t)tree->wlevels * tree->wwords, sizeof(int),
@@ -2007,14 +2037,20 @@ void make_tnodes(TreeBase* tree, int bucket, cudaStream_t st) {
   }
   k_troots<T, D><<<div_up(tree->ncloud, 128), 128, 0, st>>>(recs, tree->root_rec, tree->valid_off, tree->ncloud,
                                                             nr > 0 ? flag.get() : nullptr, tid.get(), nt, nodes,
-                                                            tree->root_tnode);
+                                                            tree->root_tnode, boxbuf.get());
   PPTKG_CHECK_LAUNCH();
+  double box[8];
+  PPTKG_CUDA(cudaMemcpyAsync(box, boxbuf.get(), sizeof(box), cudaMemcpyDeviceToHost, st));
   tree->root_tnode_h.resize(tree->ncloud);
   PPTKG_CUDA(cudaMemcpyAsync(tree->root_tnode_h.data(), tree->root_tnode, sizeof(int) * tree->ncloud,
                              cudaMemcpyDeviceToHost, st));
   if (!tree->capture) tree->tdepth = tree->depth + 2;
   if constexpr (std::is_integral<T>::value) lower_tnodes<T, D>(tree, st);
   PPTKG_CUDA(cudaStreamSynchronize(st));
+  for (int d = 0; d < D; d++) {
+    tree->root_lo[d] = box[d];
+    tree->root_hi[d] = box[4 + d];
+  }
 }
 
 #ifndef PPTKG_BUILD_INT
@@ -2063,11 +2099,7 @@ void forest_capture_ready(TreeBase* t, cudaStream_t st) {
   t->cap_tnodes = std::min<int64_t>(t->cap_recs, 2 * live_tnodes + 4096) + t->ncloud;
   if (t->cap_recs > INT32_MAX / 2 || t->cap_tnodes > INT32_MAX / 2)
     throw Error(E_INVALID, "forest too large for capture mode");
-  int per_sm = 1, nsm = 1;
-  PPTKG_CUDA(cudaFuncSetAttribute(k_subtree<T, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  PPTKG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_subtree<T, D>, 32, smem));
-  PPTKG_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, t->device));
-  t->cap_subgrid = std::max(per_sm, 1) * nsm;
+  t->cap_subgrid = subtree_grid(smem, t->device);
   // capacity-sized arrays, current contents kept
   auto grow = [&](void** p, size_t have, size_t want) {
     void* q = nullptr;
@@ -2124,34 +2156,31 @@ void rebuild_forest(TreeBase* t, const T* d_in, cudaStream_t st, int* status) {
   const int rec_cap = (int)t->cap_recs;
   Rec<T, D>* recs = (Rec<T, D>*)t->recs;
   const int seg_cap = (int)(n / (small_cap + 1) + 2);
-  const int max_tiles = (int)(n / TILE) + seg_cap + 2;
-  BuildBuf<BuildCtl> ctl(1, st);
-  PPTKG_CUDA(cudaMemsetAsync(ctl.get(), 0, sizeof(BuildCtl), st));
+  const int max_tiles = (int)(n / tile_points(n)) + seg_cap + 2;
+  Levels<T, D> lv(n, tile_points(n), max_tiles, seg_cap, t->cap_small, small_cap, t->device, soa, recs, rec_cap, t->root_rec,
+                  t->max_leaf, t->empty_split, st);
+  BuildCtl* ctl = lv.ctl;
   PPTKG_CUDA(cudaMemsetAsync(t->root_rec, 0xff, sizeof(int) * ncloud, st));
-  BuildBuf<Seg<T, D>> segL[2] = {BuildBuf<Seg<T, D>>(seg_cap, st), BuildBuf<Seg<T, D>>(seg_cap, st)};
-  BuildBuf<Small<T, D>> smallL(t->cap_small, st);
-  k_roots<T, D><<<div_up(ncloud, 128), 128, 0, st>>>(t->valid_off, t->orig_off, ncloud, small_cap, segL[0].get(),
-                                                      smallL.get(), t->cap_small, ctl.get());
+  k_roots<T, D><<<div_up(ncloud, 128), 128, 0, st>>>(t->valid_off, t->orig_off, ncloud, small_cap, tile_points(n),
+                                                      lv.seg[0],                                                      lv.small, t->cap_small, ctl);
   PPTKG_CHECK_LAUNCH();
   {
     // a fixed number of levels; the kernels of a level without segments
     // return at once
-    Levels<T, D> lv(n, max_tiles, seg_cap, t->device, ctl.get(), soa, recs, rec_cap, t->root_rec, t->max_leaf,
-                    t->empty_split, st);
     for (int lvl = 0; lvl < t->cap_levels; lvl++) {
-      Seg<T, D>* A = segL[lvl & 1].get();
-      Seg<T, D>* B = segL[(lvl + 1) & 1].get();
+      Seg<T, D>* A = lv.seg[lvl & 1];
+      Seg<T, D>* B = lv.seg[(lvl + 1) & 1];
       lv.split(A, lvl, true);
       lv.tie_pass(A, lvl, 2);
-      lv.children(A, lvl, 2, B, smallL.get(), t->cap_small, small_cap);
+      lv.children(A, lvl, 2, B);
     }
   }
   // the persistent subtree kernel takes the small segments; blocks without
   // work return
-  k_subtree<T, D><<<t->cap_subgrid, 32, smem, st>>>(smallL.get(), soa, recs, t->root_rec, small_cap, cap_list,
-                                                             t->max_leaf, t->empty_split, rec_cap, t->cap_small, ctl.get());
+  k_subtree<T, D><<<t->cap_subgrid, 32, smem, st>>>(lv.small, soa, recs, t->root_rec, small_cap, cap_list,
+                                                             t->max_leaf, t->empty_split, rec_cap, t->cap_small, ctl);
   PPTKG_CHECK_LAUNCH();
-  k_rebuild_status<<<1, 1, 0, st>>>(ctl.get(), t->cap_levels, t->tdepth, status, t->dev_meta, t->valid_off, ncloud);
+  k_rebuild_status<<<1, 1, 0, st>>>(ctl, t->cap_levels, t->tdepth, status, t->dev_meta, t->valid_off, ncloud);
   PPTKG_CHECK_LAUNCH();
   // tree-ordered points and the forward map
   if (n > 0) {
@@ -2162,7 +2191,7 @@ void rebuild_forest(TreeBase* t, const T* d_in, cudaStream_t st, int* status) {
   }
   // traversal hierarchy over the live records
   BuildBuf<int> tflag(rec_cap + 1, st), tid(rec_cap + 1, st);
-  const int* nrec_dev = &ctl.get()->rec_count;
+  const int* nrec_dev = &ctl->rec_count;
   k_tflag<T, D><<<div_up(rec_cap, 256), 256, 0, st>>>(recs, rec_cap, t->bucket, tflag.get(), nrec_dev);
   PPTKG_CHECK_LAUNCH();
   exclusive_scan<int, int>(tflag.get(), tid.get(), rec_cap, tid.get() + rec_cap, st);
