@@ -522,7 +522,7 @@ __device__ bool wide_knn(const TreeView<T, D>& tv, int root, const DistT* q, int
   bool started = false;
   int at = h0, cnt = h1 - h0;  // nodes of this step, one per lane
   WNode<T, D> w;
-  if (lane < cnt) w = tv.wide[at + lane];
+  if (lane < cnt) w = tv.wnode(at + lane);
   while (true) {
     if (++steps > tv.n_wide + 1) return false;
     bool hit = lane < cnt && w.cnt != 0;
@@ -578,18 +578,18 @@ __device__ bool wide_knn(const TreeView<T, D>& tv, int root, const DistT* q, int
         continue;
       }
       found = true;
-      const WNode<T, D> up = tv.wide[node];
+      const WNode<T, D> up = tv.wnode(node);
       // (its first children are on their way while its own box is tested)
       at = up.begin + from;
       cnt = -up.cnt - from;
-      if (lane < cnt) w = tv.wide[at + lane];
+      if (lane < cnt) w = tv.wnode(at + lane);
       if (from == 0 && !__any_sync(FULL, need(box_min_dist2<T, DistT, D>(up.lo, up.hi, q)))) found = false;
     }
     __syncwarp();
     if (!found) break;
     if (!started) {
       started = true;
-      const WNode<T, D> up = tv.wide[root];
+      const WNode<T, D> up = tv.wnode(root);
       if (up.cnt >= 0) {  // the tree is one leaf range
         at = root;
         cnt = 1;
@@ -597,7 +597,7 @@ __device__ bool wide_knn(const TreeView<T, D>& tv, int root, const DistT* q, int
         at = up.begin;
         cnt = -up.cnt;
       }
-      if (lane < cnt) w = tv.wide[at + lane];
+      if (lane < cnt) w = tv.wnode(at + lane);
     }
     if (cnt > 32) {
       if (sp >= tv.wstack) return false;
@@ -741,7 +741,7 @@ __device__ __forceinline__ bool warp_knn(const TreeView<T, D>& tv, int root, con
   bool started = home < 0;
   int at = started ? root : home, cnt = 1;
   WNode<T, D> w;
-  if (lane < cnt) w = tv.wide[at + lane];
+  if (lane < cnt) w = tv.wnode(at + lane);
   while (true) {
     if (++steps > tv.n_wide + 1) return false;
     bool hit = lane < cnt && w.cnt != 0 && !(started && at + lane == home);
@@ -804,7 +804,7 @@ __device__ __forceinline__ bool warp_knn(const TreeView<T, D>& tv, int root, con
       started = true;
       at = root;
       cnt = 1;
-      if (lane == 0) w = tv.wide[root];
+      if (lane == 0) w = tv.wnode(root);
       continue;
     }
     // the topmost entry still within reach (32 are looked at together)
@@ -827,8 +827,8 @@ __device__ __forceinline__ bool warp_knn(const TreeView<T, D>& tv, int root, con
     }
     __syncwarp();
     if (node < 0) break;
-    at = tv.wide[node].begin + from;
-    cnt = -tv.wide[node].cnt - from;
+    at = tv.wnode(node).begin + from;
+    cnt = -tv.wnode(node).cnt - from;
     if (cnt > 32) {
       if (sp >= tv.wstack) return false;
       if (lane == 0) stk[sp] = make_int2(~node, from + 32);
@@ -836,7 +836,7 @@ __device__ __forceinline__ bool warp_knn(const TreeView<T, D>& tv, int root, con
       __syncwarp();
       cnt = 32;
     }
-    if (lane < cnt) w = tv.wide[at + lane];
+    if (lane < cnt) w = tv.wnode(at + lane);
   }
   return true;
 }

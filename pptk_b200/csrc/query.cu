@@ -742,6 +742,12 @@ struct StatusWord {
 // at slot `m0` of the processing order; hd / hp hold one heap per slot.
 constexpr int BIG_STACK = 128;
 
+// (the per-lane walk's stack; k of 65 to 256 is refused alike, so that the
+// trees a call takes do not depend on which walk answers it)
+static void check_depth(const TreeBase* t) {
+  if (t->tdepth > BIG_STACK) throw Error(E_UNSUPPORTED, "k > 64 on a tree deeper than 128 levels");
+}
+
 // POS: write tree positions (through the tree's index map) to chunk rows
 // (for the normal pass) instead of original indices to query rows.
 template <typename T, int D, typename L, bool POS>
@@ -768,7 +774,6 @@ template <typename T, int D, typename L>
 void launch_knn_big(const TreeBase* t, L ld, const int* order, int mode, int m, int k, typename DistOf<T>::type r2,
                     int32_t* d_idx, int32_t* d_cnt, int* status, cudaStream_t st) {
   typedef typename DistOf<T>::type DistT;
-  if (t->tdepth > BIG_STACK) throw Error(E_UNSUPPORTED, "k > 256 on a tree deeper than 128 levels");
   const size_t per_query = (size_t)k * (sizeof(DistT) + sizeof(int));
   const int chunk = (int)std::max<size_t>(1, std::min<size_t>((size_t)m, ((size_t)2 << 30) / per_query));
   DevBuf<DistT> hd((size_t)chunk * k, st);
@@ -788,6 +793,7 @@ void knn_query(const TreeBase* t, const QuerySpec& qs, int k, double dmax, int32
   if (k < 1) throw Error(E_INVALID, "k must be positive");
   const int m = (int)qs.m;
   if (m <= 0) return;
+  if (k > KNN_MAX_K) check_depth(t);
   DevBuf<int> status(1, st);
   PPTKG_CUDA(cudaMemsetAsync(status.get(), 0, sizeof(int), st));
   const bool warps = by_warp(t->nv, m, k);
@@ -919,8 +925,8 @@ __device__ __forceinline__ bool warp_rnear_walk(const TreeView<T, D>& tv, int ro
     int first = 0, kids = 0;
     bool hit = false, whole = false;
     if (fresh ? lane < cnt : (todo >> lane & 1u)) {
-      const WNode<T, D> w = tv.wide[at + lane];
-      span = tv.wspan[at + lane];
+      const WNode<T, D> w = tv.wnode(at + lane);
+      span = tv.wspan_of(at + lane);
       first = w.begin;
       kids = w.cnt > 0 ? 0 : -w.cnt;
       if (fresh) {
@@ -1776,7 +1782,7 @@ void normals_big(const TreeBase* t, L ld, const int* order, int mode, int m, int
                  int num_eigen, T* ev, T* ew, int32_t* sz, int* status, cudaStream_t st) {
   typedef typename DistOf<T>::type DistT;
   const bool heaps = k > WARP_MAX_K;
-  if (heaps && t->tdepth > BIG_STACK) throw Error(E_UNSUPPORTED, "k > 256 on a tree deeper than 128 levels");
+  check_depth(t);
   const size_t per_query = (size_t)k * (sizeof(DistT) + 2 * sizeof(int)) + sizeof(int);
   const int chunk = (int)std::max<size_t>(1, std::min<size_t>((size_t)m, ((size_t)2 << 30) / per_query));
   DevBuf<DistT> hd(heaps ? (size_t)chunk * k : 0, st);

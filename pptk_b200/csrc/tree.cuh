@@ -120,6 +120,8 @@ struct TreeView {
   __device__ __forceinline__ int id_at(int i) const { return ids[checked(i, pts_cap, 1)]; }
   __device__ __forceinline__ int pos_of(const int32_t* map, int o) const { return map[checked(o, n_in, 2)]; }
   __device__ __forceinline__ int node_index(int i) const { return checked(i, n_nodes, 3); }
+  __device__ __forceinline__ const WNode<T, D>& wnode(int i) const { return wide[checked(i, n_wide, 3)]; }
+  __device__ __forceinline__ int2 wspan_of(int i) const { return wspan[checked(i, n_wide, 3)]; }
   // the wide hierarchy's node of level j that holds tree position p
   __device__ __forceinline__ int wide_of(int j, int p) const {
     const int c = checked(p, pts_cap, 1), w = j * wwords + (c >> 5);
