@@ -1,11 +1,12 @@
-// Warp-packet k-d tree traversal for kNN and r-near queries.
+// k-d tree traversals for kNN and r-near queries.
 //
-// A warp carries 32 queries that are close in tree order (queries are sorted
-// by the tree position of the point or of the bucket they fall in), so the
-// packet walks one shared path: each node is one broadcast load, the two
-// children are tested per lane, and a child is entered when any lane can
-// still improve its result there.  Leaf buckets are staged in shared memory
-// with one coalesced 16 B load per lane and then read back as broadcasts.
+// kNN: a warp carries a packet of 32 queries that are close in tree order
+// (queries are sorted by the tree position of the point or of the bucket they
+// fall in), or answers one query with all its lanes; both walk the wide
+// hierarchy, a node's children one per lane.  r-near packets walk the binary
+// hierarchy: each node is one broadcast load, the two children are tested per
+// lane, and leaf buckets are staged in shared memory with one coalesced 16 B
+// load per lane and read back as broadcasts.
 //
 // Distances follow the reference exactly (kdtree-impl.h:331-339): per-axis
 // (point - query) in the distance type, squared, summed in axis order, each
@@ -131,7 +132,6 @@ struct TopK<KMAX, float> {
     for (int j = 0; j < KMAX; j++)
       if (j < k && s[j] > key) s[j] = key;
   }
-  __device__ __forceinline__ void reserve(int) {}
   __device__ __forceinline__ bool valid(int j) const { return s[j] < lim && (unsigned)s[j] != 0xffffffffu; }
   __device__ __forceinline__ int id(int j) const { return (int)(unsigned)(s[j] & 0xffffffffull); }
   // Slot j sorts before the key (0, id0) of a point at distance 0.
@@ -221,7 +221,6 @@ struct TopK<KMAX, double> {
         p[j] = 0x7fffffff;
       }
   }
-  __device__ __forceinline__ void reserve(int) {}
   __device__ __forceinline__ bool valid(int j) const { return p[j] >= 0 && p[j] != 0x7fffffff && d[j] >= 0.0; }
   __device__ __forceinline__ int id(int j) const { return p[j]; }
   __device__ __forceinline__ bool below_zero(int j, int id0) const { return d[j] == 0.0 && p[j] < id0; }
@@ -848,8 +847,7 @@ __device__ __forceinline__ bool warp_knn(const TreeView<T, D>& tv, int root, con
 // Every point whose distance is within the query's final bound is offered.
 // Requires tv.depth <= LSTACK (the caller checks); false on a corrupt tree.
 template <int LSTACK, typename T, int D, typename DistT, typename Top>
-__device__ bool lane_knn(const TreeView<T, D>& tv, const DistT* q, int own, bool active, DistT r2, Top& top,
-                         int wlo = 0, int wn = 0) {
+__device__ bool lane_knn(const TreeView<T, D>& tv, const DistT* q, int own, bool active, DistT r2, Top& top) {
   if (!active) return true;
   int sref[LSTACK], scnt[LSTACK];
   DistT smd[LSTACK];
@@ -870,13 +868,13 @@ __device__ bool lane_knn(const TreeView<T, D>& tv, const DistT* q, int own, bool
       }
 #pragma unroll
       for (int j = 0; j < 4; j++)
-        if (d2[j] <= top.worst() && d2[j] < r2 && p + j != own && (unsigned)(p + j - wlo) >= (unsigned)wn)
+        if (d2[j] <= top.worst() && d2[j] < r2 && p + j != own)
           top.offer(d2[j], r[j].id);
     }
     for (; p < end; p++) {
       const PointRec<T, D> r = tv.pt(p);
       const DistT d2 = point_dist2<T, DistT, D>(r.c, q);
-      if (d2 <= top.worst() && d2 < r2 && p != own && (unsigned)(p - wlo) >= (unsigned)wn) top.offer(d2, r.id);
+      if (d2 <= top.worst() && d2 < r2 && p != own) top.offer(d2, r.id);
     }
   };
   int cur = tv.root, visits = 0;

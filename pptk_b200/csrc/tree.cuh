@@ -2,7 +2,7 @@
 //
 // The build reproduces the reference tree exactly (pptk/kdtree/src/
 // kdtree-impl.h:248-329, 773-818): the same point permutation, the same
-// split and empty-split ("trim") nodes.  It leaves three products in HBM:
+// split and empty-split ("trim") nodes.  It leaves these products in HBM:
 //
 //  * PointRec[nv]  -- the valid points in tree order, each with its original
 //                     index (the reference's points_ + reverse_indices_,
@@ -13,7 +13,10 @@
 //  * TNode[n_tnodes] -- the traversal hierarchy: the reference tree cut at
 //                     nodes of at most `bucket` points, each node holding both
 //                     children's tight boxes, so one 64 B broadcast load per
-//                     warp decides both children.
+//                     warp decides both children (r-near packets, the
+//                     descent that locates queries, k > 256);
+//  * WNode[n_wide] -- the same tree cut every four levels or so, for the walks
+//                     that test a node's children one per lane.
 //
 // The traversal only needs boxes that contain their points: every result is
 // decided by point distances computed exactly as the reference does, so the
