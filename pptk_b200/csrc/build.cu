@@ -961,6 +961,18 @@ __global__ void k_children(Seg<T, D>* segs, int lvl, int tied, Rec<T, D>* recs, 
           }
           decide(c, ctl, recs, rec_cap, (int*)nullptr, max_leaf, thr);
         } else {
+          // decided by k_node once k_bbox knows its box; until then, and for
+          // good below the last level of a rebuild, its record is a leaf that
+          // no other record refers to (the passes over all records read it)
+          Rec<T, D> rec;
+          rec.begin = cb;
+          rec.end = ce;
+          rec.split_dim = -1;
+          rec.split_index = rec.left = rec.right = -1;
+          rec.ntrim = 0;
+          for (int d = 0; d < D; d++) rec.lo[d] = rec.hi[d] = (T)0;
+          rec.split_val = (T)0;
+          if (c.rec < rec_cap) recs[c.rec] = rec;
           ctl->unboxed = lvl + 2;
         }
         t0 = c.tile0;
