@@ -18,6 +18,7 @@
 #include <vector>
 
 #include "build.cuh"
+#include "build_nodes.cuh"
 #include "profile.cuh"
 #include "util.cuh"
 
@@ -52,16 +53,6 @@ struct Seg {
   int G;
   int tile0, ntiles;
   int boxed;  // tlo / thi are known (from the parent)
-};
-
-// A segment for k_subtree.
-template <typename T, int D>
-struct Small {
-  int b, e;
-  int up;  // 2 * parent record + side, or -1 - cloud
-  int lvl;
-  long long n_orig;
-  T lo[D], hi[D];
 };
 
 // Ties of segments of at most this many points are moved by one block.
@@ -200,8 +191,9 @@ __device__ __forceinline__ Small<T, D> small_of(const Seg<T, D>& g) {
   Small<T, D> s;
   s.b = g.b;
   s.e = g.e;
-  s.up = g.parent < 0 ? g.parent : 2 * g.parent + g.side;
-  s.lvl = g.lvl;
+  s.parent = g.parent;
+  s.lvl = (int16_t)g.lvl;
+  s.side = (int16_t)g.side;
   s.n_orig = g.n_orig;
   for (int d = 0; d < D; d++) {
     s.lo[d] = g.lo[d];
@@ -403,19 +395,19 @@ __global__ void __launch_bounds__(BT) k_bbox(Seg<T, D>* segs, int lvl, const int
 
 // A record takes its place and its parent learns of it.
 template <typename T, int D>
-__device__ __forceinline__ bool link_record(const Rec<T, D>& rec, int id, int up, Rec<T, D>* recs, int rec_cap,
-                                            int* root_rec, BuildCtl* ctl) {
+__device__ __forceinline__ bool link_record(const Rec<T, D>& rec, int id, int parent, int side, Rec<T, D>* recs,
+                                            int rec_cap, int* root_rec, BuildCtl* ctl) {
   if (id >= rec_cap) {
     atomicExch(&ctl->status, 6);
     return false;
   }
   recs[id] = rec;
-  if (up < 0)
-    root_rec[-up - 1] = id;
-  else if (up & 1)
-    recs[up >> 1].right = id;
+  if (parent < 0)
+    root_rec[-parent - 1] = id;
+  else if (side)
+    recs[parent].right = id;
   else
-    recs[up >> 1].left = id;
+    recs[parent].left = id;
   return true;
 }
 
@@ -434,8 +426,7 @@ __device__ __forceinline__ void decide(Seg<T, D>& g, BuildCtl* ctl, Rec<T, D>* r
   node_logic<T, D>(g.e - g.b, g.n_orig, g.parent < 0, g.lo, g.hi, tlo, thi, max_leaf, thr, rec, g.act, g.sd, g.sv);
   rec.begin = g.b;
   rec.end = g.e;
-  if (!link_record<T, D>(rec, g.rec, g.parent < 0 ? g.parent : 2 * g.parent + g.side, recs, rec_cap, root_rec, ctl))
-    g.act = 0;
+  if (!link_record<T, D>(rec, g.rec, g.parent, g.side, recs, rec_cap, root_rec, ctl)) g.act = 0;
   g.boxed = 1;
 }
 
@@ -997,13 +988,6 @@ __global__ void k_children(Seg<T, D>* segs, int lvl, int tied, Rec<T, D>* recs, 
 }
 
 // ------------------------------------------------- per-warp subtrees ----
-template <typename T, int D>
-struct Entry {
-  uint16_t b, e;
-  int up;  // 2 * parent record + side, or -1 - cloud for a root
-  T lo[D], hi[D];
-};
-
 // k_subtree nodes of at most this many points are split by one lane each.
 constexpr int LANE_NODE = 32;
 
@@ -1054,7 +1038,8 @@ __global__ void __launch_bounds__(32) k_subtree(const Small<T, D>* small, SoA<T,
       Entry<T, D> r;
       r.b = 0;
       r.e = (uint16_t)n;
-      r.up = seg.up;
+      r.parent = seg.parent;
+      r.side = (uint16_t)seg.side;
 #pragma unroll
       for (int d = 0; d < D; d++) {
         r.lo[d] = seg.lo[d];
@@ -1128,10 +1113,10 @@ __global__ void __launch_bounds__(32) k_subtree(const Small<T, D>* small, SoA<T,
         const int id = base + ei;
         if (size > 0) {
           Rec<T, D> rec;
-          node_logic<T, D>(size, seg.n_orig, en.up < 0, en.lo, en.hi, mn, mx, max_leaf, thr, rec, act, sd, sv);
+          node_logic<T, D>(size, seg.n_orig, en.parent < 0, en.lo, en.hi, mn, mx, max_leaf, thr, rec, act, sd, sv);
           rec.begin = seg.b + b;
           rec.end = seg.b + e;
-          if (!link_record<T, D>(rec, id, en.up, recs, rec_cap, root_rec, ctl)) act = 0;
+          if (!link_record<T, D>(rec, id, en.parent, en.side, recs, rec_cap, root_rec, ctl)) act = 0;
         }
         int L1 = 0, L2 = 0;
         // partition of the large nodes, by the warp
@@ -1284,7 +1269,8 @@ __global__ void __launch_bounds__(32) k_subtree(const Small<T, D>* small, SoA<T,
         Entry<T, D> c;
         c.b = (uint16_t)b;
         c.e = (uint16_t)si;
-        c.up = 2 * id;
+        c.parent = id;
+        c.side = 0;
         if (left) {
 #pragma unroll
           for (int d = 0; d < D; d++) {
@@ -1296,7 +1282,7 @@ __global__ void __launch_bounds__(32) k_subtree(const Small<T, D>* small, SoA<T,
         if (right) {
           c.b = (uint16_t)si;
           c.e = (uint16_t)e;
-          c.up = 2 * id + 1;
+          c.side = 1;
 #pragma unroll
           for (int d = 0; d < D; d++) {
             c.lo[d] = d == sd ? sv : en.lo[d];
