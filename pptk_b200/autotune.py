@@ -12,8 +12,8 @@ Five settings shape every kNN / normal traversal; none changes a result:
 * ``topk_min``: the k-tiling of the register top-k lists (their compile-time
   capacity, at least the smallest of 4/8/16/32/64 that holds k);
 * ``warm_mult``: the width of the warm-start window of full-capacity float
-  lists, in multiples of k (2 is best for queries in tree order; 3 was
-  faster for scattered kNN queries on the 20M scene).
+  lists, in multiples of k, one more for short lists of scattered queries
+  (2 is best for queries in tree order).
 
 ``tune`` times a caller-supplied workload on a sample: the full grid of
 bucket x lane_span first, then one pass over each further knob with the

@@ -9,6 +9,7 @@
 #include "normals.cuh"
 #include "profile.cuh"
 #include "query.cuh"
+#include "rules.cuh"
 #include "util.cuh"
 
 namespace pptkg {
@@ -521,14 +522,6 @@ int make_order(const TreeBase* t, const QuerySpec& qs, DevBuf<int>& order, cudaS
 }
 
 // ----------------------------------------------------------------- kNN ----
-// warm_mult of a batch of m queries on nv points: one more where packets
-// span over 256 tree positions and lists are short.  Their queries' walks
-// share less, so candidates found before them save more (1M scattered
-// queries, k = 16: 2.35 -> 2.10 ms; queries in tree order: 31.8 -> 32.7).
-inline int warm_window(int64_t nv, int64_t m, int kmax) {
-  return g_tune_warm_mult.load() + (kmax <= 16 && 32 * nv > 256 * m ? 1 : 0);
-}
-
 // Blocks per SM the kNN kernel is compiled for: float top-k lists of up to
 // 16 entries run in 80 registers (6 blocks of 128 threads; spills of 200 B
 // cost less than the sixth block gives: 1M scattered queries 2.54 ms at 5
@@ -591,7 +584,7 @@ void launch_knn(const TreeBase* t, L ld, const int* order, int mode, int m, int 
   k_knn<T, D, KMAX, L><<<div_up(m, QTHREADS), QTHREADS, smem, st>>>(view_of<T, D>(t), ld, order, mode, m, k, r2,
                                                                       d_idx, d_cnt, status, fm,
                                                                       g_tune_warm_bound.load() != 0,
-                                                                      warm_window(t->nv, m, KMAX));
+                                                                      warm_window(g_tune_warm_mult.load(), t->nv, m, KMAX));
   PPTKG_CHECK_LAUNCH();
 }
 
@@ -1674,7 +1667,7 @@ void launch_normals(const TreeBase* t, L ld, const int* order, int mode, int m, 
         cudaFuncSetAttribute(k_normals<T, KMAX, L, PREC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   k_normals<T, KMAX, L, PREC><<<div_up(m, QTHREADS), QTHREADS, smem, st>>>(
       view_of<T, 3>(t), ld, order, mode, m, k, r2, num_eigen, gap_thr, ev, ew, sz, fix, nfix, status, fm,
-      g_tune_warm_bound.load() != 0, warm_window(t->nv, m, KMAX), kidx, kcnt);
+      g_tune_warm_bound.load() != 0, warm_window(g_tune_warm_mult.load(), t->nv, m, KMAX), kidx, kcnt);
   PPTKG_CHECK_LAUNCH();
 }
 
