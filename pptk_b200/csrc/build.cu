@@ -4,9 +4,10 @@
 //
 // The reference builds depth first; every node only permutes the indices of
 // its own range, so building all nodes of a level at once gives the same
-// permutation.  Nodes with more than `small_cap` points are processed by
-// grid-wide kernels over tiles of points; smaller subtrees are finished by
-// one warp each, entirely in shared memory.
+// permutation.  Nodes with more than mid_capacity() points are processed by
+// grid-wide kernels over tiles of points; those of up to that many are split
+// by one block each, in shared memory, until small_capacity() points are left,
+// and subtrees of those are finished by one warp each.
 //
 // The reference partition (PartitionIndices, kdtree-impl.h:192-246) is two
 // Hoare passes with converging cursors.  Each pass pairs the j-th misplaced
@@ -58,12 +59,14 @@ struct Seg {
 // Ties of segments of at most this many points are moved by one block.
 constexpr int TIE_BLOCK = 8192;
 
-constexpr int MAX_LEVELS = 4096;  // grid-wide levels (segments above small_cap points)
+constexpr int MAX_LEVELS = 4096;  // grid-wide levels
 
 struct BuildCtl {
   int status;
   int nsmall;
   int small_next;
+  int nmid;
+  int mid_next;
   int rec_count;
   int depth;
   int ties;     // 1 + the last level with points at a split value
@@ -202,6 +205,24 @@ __device__ __forceinline__ Small<T, D> small_of(const Seg<T, D>& g) {
   return s;
 }
 
+// Segments that the grid-wide levels leave: to k_block (`mid`, above small_cap
+// points) and k_subtree (`small`).
+template <typename T, int D>
+struct Lists {
+  Small<T, D>*mid, *small;
+  int mid_capn, small_capn, mid_cap, small_cap;
+};
+
+template <typename T, int D>
+__device__ __forceinline__ void hand_on(const Small<T, D>& s, const Lists<T, D>& to, BuildCtl* ctl) {
+  const bool mid = s.e - s.b > to.small_cap;
+  const int slot = atomicAdd(mid ? &ctl->nmid : &ctl->nsmall, 1);
+  if (slot < (mid ? to.mid_capn : to.small_capn))
+    (mid ? to.mid : to.small)[slot] = s;
+  else
+    atomicExch(&ctl->status, 7);
+}
+
 template <typename T, int D>
 __device__ __forceinline__ void seg_clear(Seg<T, D>& g) {
   for (int d = 0; d < D; d++) {
@@ -260,8 +281,8 @@ static __global__ void k_cloud_off(const int* off, const int64_t* orig_off, int 
 // launched with upper-bound grids and read the live counts from the device,
 // so the host never waits between levels.
 template <typename T, int D>
-__global__ void k_roots(const int64_t* valid_off, const int64_t* orig_off, int ncloud, int small_cap, int tile,
-                        Seg<T, D>* lvl0, Small<T, D>* small, int small_capn, BuildCtl* ctl) {
+__global__ void k_roots(const int64_t* valid_off, const int64_t* orig_off, int ncloud, int tile, Seg<T, D>* lvl0,
+                        Lists<T, D> to, BuildCtl* ctl) {
   int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c == 0) ctl->tile = tile;
   if (c >= ncloud) return;
@@ -280,16 +301,12 @@ __global__ void k_roots(const int64_t* valid_off, const int64_t* orig_off, int n
     g.hi[d] = Limits<T>::lowest();
   }
   seg_clear(g);
-  if (e - b > small_cap) {
+  if (e - b > to.mid_cap) {
     ctl->unboxed = 1;
     take_place(g, 0, tile, ctl);
     lvl0[atomicAdd(&ctl->level_cnt[0], 1)] = g;
   } else {
-    const int slot = atomicAdd(&ctl->nsmall, 1);
-    if (slot < small_capn)
-      small[slot] = small_of(g);
-    else
-      atomicExch(&ctl->status, 7);
+    hand_on(small_of(g), to, ctl);
   }
 }
 
@@ -911,8 +928,7 @@ __global__ void __launch_bounds__(BT) k_swap(Seg<T, D>* segs, int lvl, bool tie,
 // the 400 segments of a 200k-point build's last level.)
 template <typename T, int D>
 __global__ void k_children(Seg<T, D>* segs, int lvl, int tied, Rec<T, D>* recs, int rec_cap, Seg<T, D>* next,
-                           Small<T, D>* small, int small_capn, int small_cap_pts, int max_leaf, double thr,
-                           int* tile_seg, BuildCtl* ctl) {
+                           Lists<T, D> to, int max_leaf, double thr, int* tile_seg, BuildCtl* ctl) {
   const int c0 = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31;
   const int i = c0 >> 1, side = c0 & 1;
   // a level whose ties had no pass (tied 0: none was launched, 1: that of
@@ -942,7 +958,7 @@ __global__ void k_children(Seg<T, D>* segs, int lvl, int tied, Rec<T, D>* recs, 
         c.lo[d] = side == 1 && d == g.sd ? g.sv : g.lo[d];
         c.hi[d] = side == 0 && d == g.sd ? g.sv : g.hi[d];
       }
-      if (ce - cb > small_cap_pts) {
+      if (ce - cb > to.mid_cap) {
         seg_clear(c);
         take_place(c, lvl + 1, ctl->tile, ctl);
         if (si == g.b + g.L1 || !big_tie(g)) {
@@ -971,11 +987,7 @@ __global__ void k_children(Seg<T, D>* segs, int lvl, int tied, Rec<T, D>* recs, 
         at = atomicAdd(&ctl->level_cnt[lvl + 1], 1);
         next[at] = c;
       } else {
-        const int slot = atomicAdd(&ctl->nsmall, 1);
-        if (slot < small_capn)
-          small[slot] = small_of(c);
-        else
-          atomicExch(&ctl->status, 7);
+        hand_on(small_of(c), to, ctl);
       }
     }
   }
@@ -984,6 +996,245 @@ __global__ void k_children(Seg<T, D>* segs, int lvl, int tied, Rec<T, D>* recs, 
     const int a = __shfl_sync(0xffffffffu, t0, s), n = __shfl_sync(0xffffffffu, nt, s),
               k = __shfl_sync(0xffffffffu, at, s);
     for (int t = lane; t < n; t += 32) tile_seg[a + t] = k;
+  }
+}
+
+// --------------------------------------------- per-block segments ----
+// Points of a warp's word whose bits are set, counted before every word: the
+// words of a segment of up to 2,048 points, two per lane.
+struct WordScan {
+  int a0, a1, total;
+  __device__ __forceinline__ WordScan(const uint32_t* bits, int words) {
+    const int lane = threadIdx.x & 31;
+    const int c0 = lane < words ? __popc(bits[lane]) : 0, c1 = lane + 32 < words ? __popc(bits[lane + 32]) : 0;
+    const int i0 = warp_incl_scan(c0), t0 = __shfl_sync(0xffffffffu, i0, 31);
+    const int i1 = warp_incl_scan(c1) + t0;
+    a0 = i0 - c0;
+    a1 = i1 - c1;
+    total = __shfl_sync(0xffffffffu, i1, 31);
+  }
+  // bits set before word w (the same in every lane)
+  __device__ __forceinline__ int before(int w) const { return __shfl_sync(0xffffffffu, w < 32 ? a0 : a1, w & 31); }
+};
+
+// Splits segments of small_cap to mid_cap points, one block each in shared
+// memory, down to small_cap points, which go to the list of k_subtree.  A
+// node's partition takes its ranks from a bit per point: a misplaced point's
+// rank is the number of set (or clear) bits before it.  Persistent: a block
+// takes segments from the list until it is exhausted.
+//
+// As grid-wide levels these segments cost a chain of launches per level for a
+// few thousand points, and a cloud of long chains (a few points split off at a
+// time) one chain of launches per split.  us a build with k_subtree taking
+// 2,048 points / with levels down to 512 / so: 600 points 261 / 305 / 241,
+// 1,000 277 / 336 / 267, 3,000 in chains 3540 / 4618 / 2016, 200k with ties
+// 938 / 1023 / 895, 5M 3300 / 2971 / 2668.  A few blocks' serial splits bound
+// the small ones, the levels above the large ones.
+template <typename T, int D>
+__global__ void __launch_bounds__(BT, 4) k_block(SoA<T, D> soa, Rec<T, D>* recs, int rec_cap, int* root_rec,
+                                              Lists<T, D> to, int max_leaf, double thr, BuildCtl* ctl) {
+  typedef typename OrdOf<T>::type U;
+  constexpr int WARPS = BT / 32, TODO = 4;
+  extern __shared__ __align__(16) unsigned char smem[];
+  __shared__ Small<T, D> todo[TODO];  // (disjoint, above small_cap points each: at most three)
+  __shared__ U box[WARPS][2 * D];
+  __shared__ uint32_t bits[64];
+  __shared__ int le[WARPS];
+  // (the box as values in shared memory: ptxas 12.9 does not come back from the
+  // int16, 3-d kernel where the deciding lane converts it itself)
+  __shared__ T s_sv, tight[2 * D];
+  __shared__ int s_item, s_todo, s_act, s_sd, s_rec;
+  T* X[D];
+  unsigned char* p = smem;
+#pragma unroll
+  for (int d = 0; d < D; d++) {
+    X[d] = (T*)p;
+    p += sizeof(T) * to.mid_cap;
+  }
+  int* ID = (int*)p;
+  p += sizeof(int) * to.mid_cap;
+  uint16_t* S = (uint16_t*)p;
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  const unsigned FULL = 0xffffffffu, lt = (1u << lane) - 1u;
+  const int nmid = min(ctl->nmid, to.mid_capn);
+  // swaps the first G pairs of S[at ..] and, from its end, S[at + half ..]
+  auto swap = [&](int at, int half, int G) {
+    __syncthreads();
+    for (int j = tid; j < G; j += BT) {
+      const int x = S[at + j], y = S[at + half + G - 1 - j];
+#pragma unroll
+      for (int d = 0; d < D; d++) {
+        const T t = X[d][x];
+        X[d][x] = X[d][y];
+        X[d][y] = t;
+      }
+      const int t = ID[x];
+      ID[x] = ID[y];
+      ID[y] = t;
+    }
+    __syncthreads();
+  };
+
+  while (true) {
+    if (tid == 0) s_item = atomicAdd(&ctl->mid_next, 1);
+    __syncthreads();
+    if (s_item >= nmid) break;
+    const int base = to.mid[s_item].b, n = to.mid[s_item].e - base;
+    for (int i = tid; i < n; i += BT) {
+#pragma unroll
+      for (int d = 0; d < D; d++) X[d][i] = soa.x[d][base + i];
+      ID[i] = soa.id[base + i];
+    }
+    if (tid == 0) {
+      todo[0] = to.mid[s_item];
+      s_todo = 1;
+    }
+    __syncthreads();
+    for (int nodes = 0; s_todo > 0; nodes++) {
+      const int cur = s_todo - 1;
+      const int b = todo[cur].b - base, e = todo[cur].e - base, words = (e - b + 31) >> 5;
+      // tight box
+      T mn[D], mx[D];
+#pragma unroll
+      for (int d = 0; d < D; d++) {
+        mn[d] = Limits<T>::max();
+        mx[d] = Limits<T>::lowest();
+      }
+      for (int i = b + tid; i < e; i += BT)
+#pragma unroll
+        for (int d = 0; d < D; d++) {
+          const T v = X[d][i];
+          mn[d] = min(mn[d], v);
+          mx[d] = max(mx[d], v);
+        }
+#pragma unroll
+      for (int d = 0; d < D; d++) {
+        const U lo = warp_min_ord(ord_t<T>(mn[d])), hi = warp_max_ord(ord_t<T>(mx[d]));
+        if (lane == 0) {
+          box[wid][d] = lo;
+          box[wid][D + d] = hi;
+        }
+      }
+      __syncthreads();
+      if (wid == 0) {
+        if (lane < 2 * D) {
+          U v = box[0][lane];
+          for (int w = 1; w < WARPS; w++) v = lane < D ? min(v, box[w][lane]) : max(v, box[w][lane]);
+          tight[lane] = from_ord_t<T>(v);
+        }
+        __syncwarp();
+        if (lane == 0) {
+          Small<T, D> g = todo[cur];
+          Rec<T, D> rec;
+          int act = 0, sd = 0;
+          T sv = (T)0;
+          node_logic<T, D>(e - b, g.n_orig, g.parent < 0, g.lo, g.hi, tight, tight + D, max_leaf, thr, rec, act, sd, sv);
+          rec.begin = g.b;
+          rec.end = g.e;
+          const int id = atomicAdd(&ctl->rec_count, 1);
+          if (!link_record<T, D>(rec, id, g.parent, g.side, recs, rec_cap, root_rec, ctl)) act = 0;
+          if (nodes >= n) {  // every split leaves fewer points
+            atomicExch(&ctl->status, 5);
+            act = 0;
+          }
+          atomicMax(&ctl->depth, g.lvl + 1);
+          todo[cur] = g;  // (its extent is trimmed)
+          s_act = act;
+          s_sd = sd;
+          s_sv = sv;
+          s_rec = id;
+          if (!act) s_todo = cur;
+        }
+      }
+      __syncthreads();
+      if (!s_act) continue;
+      const T sv = s_sv;
+      const T* v = X[0];
+#pragma unroll
+      for (int d = 1; d < D; d++)
+        if (d == s_sd) v = X[d];
+      // a bit per point: below the split value
+      int c2 = 0;
+      for (int w = wid; w < words; w += WARPS) {
+        const int q = b + 32 * w + lane;
+        const bool in = q < e;
+        const T x = in ? v[q] : sv;
+        const unsigned m = __ballot_sync(FULL, in && x < sv);
+        c2 += __popc(__ballot_sync(FULL, in && x <= sv));
+        if (lane == 0) bits[w] = m;
+      }
+      if (lane == 0) le[wid] = c2;
+      __syncthreads();
+      const int half = (e - b) / 2;
+      int L1, L2 = 0;
+      {
+        const WordScan scan(bits, words);
+        L1 = scan.total;
+        for (int w = 0; w < WARPS; w++) L2 += le[w];
+        const int zw = L1 >> 5;  // points below the split value among the first L1
+        const int first = zw < words ? scan.before(zw) + __popc(bits[zw] & ((1u << (L1 & 31)) - 1u)) : L1;
+        for (int w = wid; w < words; w += WARPS) {
+          const unsigned m = bits[w];
+          const int q = 32 * w + lane, r = scan.before(w) + __popc(m & lt);
+          if (m >> lane & 1u) {
+            if (q >= L1) S[b + half + r - first] = (uint16_t)(b + q);
+          } else if (q < L1) {
+            S[b + q - r] = (uint16_t)(b + q);
+          }
+        }
+        swap(b, half, L1 - first);
+      }
+      if (L1 != L2) {
+        // the tie pass: points equal to the split value to [b + L1, b + L2)
+        for (int w = wid; w < words; w += WARPS) {
+          const int q = 32 * w + lane;
+          const T x = b + q < e ? v[b + q] : sv;
+          const unsigned m = __ballot_sync(FULL, b + q < e && q >= L1 && (q < L2 ? x > sv : x <= sv));
+          if (lane == 0) bits[w] = m;
+        }
+        __syncthreads();
+        const WordScan scan(bits, words);
+        const int zw = L2 >> 5;
+        const int G = zw < words ? scan.before(zw) + __popc(bits[zw] & ((1u << (L2 & 31)) - 1u)) : scan.total;
+        for (int w = wid; w < words; w += WARPS) {
+          const unsigned m = bits[w];
+          const int q = 32 * w + lane, r = scan.before(w) + __popc(m & lt);
+          if (m >> lane & 1u) S[q < L2 ? b + r : b + half + r - G] = (uint16_t)(b + q);
+        }
+        swap(b, half, G);
+      }
+      if (tid == 0) {
+        const Small<T, D> g = todo[cur];
+        const int at = g.b + num_left_rule(L1, L2, e - b);
+        recs[s_rec].split_index = at;
+        int left = cur;
+        for (int side = 0; side < 2; side++) {
+          Small<T, D> c = g;
+          c.b = side ? at : g.b;
+          c.e = side ? g.e : at;
+          if (c.b >= c.e) continue;
+          c.parent = s_rec;
+          c.side = (int16_t)side;
+          c.lvl = (int16_t)(g.lvl + 1);
+#pragma unroll
+          for (int d = 0; d < D; d++)
+            if (d == s_sd) (side ? c.lo[d] : c.hi[d]) = sv;
+          if (c.e - c.b <= to.small_cap)
+            hand_on(c, to, ctl);
+          else if (left < TODO)
+            todo[left++] = c;
+          else
+            atomicExch(&ctl->status, 3);
+        }
+        s_todo = left;
+      }
+      __syncthreads();
+    }
+    for (int i = tid; i < n; i += BT) {
+#pragma unroll
+      for (int d = 0; d < D; d++) soa.x[d][base + i] = X[d][i];
+      soa.id[base + i] = ID[i];
+    }
   }
 }
 
@@ -1595,6 +1846,32 @@ void make_wide(TreeBase* t, cudaStream_t st) {
 }
 
 // ------------------------------------------------------------ host side ----
+// Points of the largest segment that k_block takes; larger ones go through
+// grid-wide levels.  The levels planned for rebuilds count those: this size
+// decides which trees a capture-ready forest takes, so it does not follow
+// k_block's needs (2,048 float points are 37 KB of shared memory, six blocks
+// per SM).  Fewer where leaves of one to three points make more records.
+template <typename T, int D>
+int mid_capacity(int max_leaf) {
+  int cap = sizeof(T) == 4 ? 2048 : 1024;
+  while (cap > 64 && (sizeof(T) * D + 8) * (size_t)cap + 4 * (8 + sizeof(T) * D) * (size_t)(2 * (cap / (max_leaf + 1)) + 2) > 72 * 1024 - 48)
+    cap /= 2;
+  return cap;
+}
+
+template <typename T, int D>
+constexpr size_t block_smem(int cap) {
+  return (sizeof(T) * D + sizeof(int) + sizeof(uint16_t)) * (size_t)cap;
+}
+
+// k_block's grid: the blocks that the shared memory of a device's SMs holds.
+static int block_grid(size_t smem, int device) {
+  int nsm = 148, per_sm = 228 * 1024;
+  PPTKG_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device));
+  PPTKG_CUDA(cudaDeviceGetAttribute(&per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, device));
+  return std::max(nsm, 1) * std::max(1, std::min(8, (int)(per_sm / (smem + 3 * 1024))));
+}
+
 // Grid of the grid-stride level kernels: eight 256-thread blocks per SM.
 static int level_grid(int device) {
   int nsm = 148;
@@ -1612,7 +1889,7 @@ int small_capacity(int max_leaf, int& cap_list, size_t& smem) {
   while (true) {
     cap_list = 2 * (cap / (max_leaf + 1)) + 2;
     smem = (sizeof(T) * D + sizeof(int) + sizeof(uint16_t)) * (size_t)cap + 2 * sizeof(Entry<T, D>) * (size_t)cap_list;
-    if (smem <= 24 * 1024 || cap <= 64) break;
+    if ((smem <= 24 * 1024 && cap <= mid_capacity<T, D>(max_leaf)) || cap <= 64) break;
     cap /= 2;
   }
   return cap;
@@ -1690,6 +1967,14 @@ static int subtree_grid(size_t smem, int device) {
   return std::max(nsm, 1) * std::max(1, std::min(32, (int)(per_sm / (smem + 1024))));
 }
 
+// Segments above small_capacity() points that n points can have at a time.
+template <typename T, int D>
+int mid_segments(int64_t n, int max_leaf) {
+  int cap_list;
+  size_t smem;
+  return (int)(n / (small_capacity<T, D>(max_leaf, cap_list, smem) + 1) + 2);
+}
+
 // A stretch of a scratch block, handed out piece by piece (base null: only
 // measured).
 struct Carve {
@@ -1710,12 +1995,14 @@ template <typename T, int D>
 struct Levels {
   BuildBuf<char> block;
   Seg<T, D>* seg[2];
-  Small<T, D>* small;
-  int small_capn, small_cap;
+  Lists<T, D> lists;
+  int cap_list;  // of k_subtree's node lists
+  size_t smem;   // its shared memory
   int *blpos, *grpos, *tile_seg, *tile_lt;
   uint32_t* bits;
   long long *tile_cnt, *tile_off;
   unsigned gt, gq, gs;
+  int tile, device;
   BuildCtl* ctl;
   SoA<T, D> soa;
   Rec<T, D>* recs;
@@ -1725,10 +2012,11 @@ struct Levels {
   double thr;
   cudaStream_t st;
 
-  void carve(Carve c, int64_t n, int tile, int max_tiles, int seg_cap, size_t* bytes) {
+  void carve(Carve c, int64_t n, int max_tiles, int seg_cap, size_t* bytes) {
     ctl = c.take<BuildCtl>(1);
     for (auto& x : seg) x = c.take<Seg<T, D>>(seg_cap);
-    small = c.take<Small<T, D>>(small_capn);
+    lists.mid = c.take<Small<T, D>>(lists.mid_capn);
+    lists.small = c.take<Small<T, D>>(lists.small_capn);
     blpos = c.take<int>(n + 1);
     grpos = c.take<int>(n + 1);
     tile_seg = c.take<int>(max_tiles);
@@ -1738,17 +2026,42 @@ struct Levels {
     tile_off = c.take<long long>(max_tiles);
     if (bytes) *bytes = c.at;
   }
-  Levels(int64_t n, int tile, int max_tiles, int seg_cap, int small_capn_, int small_cap_, int device, SoA<T, D> soa_,
-         Rec<T, D>* recs_, int rec_cap_, int* root_rec_, int max_leaf_, double thr_, cudaStream_t st_)
-      : small_capn(small_capn_), small_cap(small_cap_),
-        gt((unsigned)std::min(max_tiles, level_grid(device))), gq((unsigned)std::min(seg_cap, level_grid(device))),
-        gs((unsigned)div_up(seg_cap, 128)), soa(soa_), recs(recs_), rec_cap(rec_cap_), root_rec(root_rec_),
-        max_leaf(max_leaf_), thr(thr_), st(st_) {
+  // Of a build of at most n points of tree `t` (of n_in input rows).
+  Levels(const TreeBase* t, int64_t n, int64_t n_in, int small_capn, SoA<T, D> soa_, Rec<T, D>* recs_, int rec_cap_,
+         cudaStream_t st_)
+      : tile(tile_points(n_in)), device(t->device), soa(soa_), recs(recs_), rec_cap(rec_cap_), root_rec(t->root_rec),
+        max_leaf(t->max_leaf), thr(t->empty_split), st(st_) {
+    lists.mid_cap = mid_capacity<T, D>(max_leaf);
+    lists.small_cap = small_capacity<T, D>(max_leaf, cap_list, smem);
+    // segments of a list or level are disjoint
+    lists.mid_capn = mid_segments<T, D>(n, max_leaf);
+    lists.small_capn = small_capn;
+    const int seg_cap = (int)(n / (lists.mid_cap + 1) + 2);
+    const int max_tiles = (int)(n / tile) + seg_cap + 2;
+    gt = (unsigned)std::min(max_tiles, level_grid(device));
+    gq = (unsigned)std::min(seg_cap, level_grid(device));
+    gs = (unsigned)div_up(seg_cap, 128);
     size_t bytes = 0;
-    carve(Carve{nullptr}, n, tile, max_tiles, seg_cap, &bytes);
+    carve(Carve{nullptr}, n, max_tiles, seg_cap, &bytes);
     block.alloc(bytes, st);
-    carve(Carve{block.get()}, n, tile, max_tiles, seg_cap, nullptr);
+    carve(Carve{block.get()}, n, max_tiles, seg_cap, nullptr);
     PPTKG_CUDA(cudaMemsetAsync(ctl, 0, sizeof(BuildCtl), st));
+  }
+  void roots(const int64_t* valid_off, const int64_t* orig_off, int ncloud) {
+    k_roots<T, D><<<div_up(ncloud, 128), 128, 0, st>>>(valid_off, orig_off, ncloud, tile, seg[0], lists, ctl);
+    PPTKG_CHECK_LAUNCH();
+  }
+  // What the grid-wide levels leave, in a cloud of up to `most` points.
+  void finish(int64_t most) {
+    if (most > lists.small_cap) {
+      const size_t bytes = block_smem<T, D>(lists.mid_cap);
+      k_block<T, D><<<std::min(lists.mid_capn, block_grid(bytes, device)), BT, bytes, st>>>(
+          soa, recs, rec_cap, root_rec, lists, max_leaf, thr, ctl);
+      PPTKG_CHECK_LAUNCH();
+    }
+    k_subtree<T, D><<<std::max(1, std::min(lists.small_capn, subtree_grid(smem, device))), 32, smem, st>>>(
+        lists.small, soa, recs, root_rec, lists.small_cap, cap_list, max_leaf, thr, rec_cap, lists.small_capn, ctl);
+    PPTKG_CHECK_LAUNCH();
   }
 
   // Boxes (where its segments' may be unknown: the roots', and those below a
@@ -1791,8 +2104,7 @@ struct Levels {
     PPTKG_CHECK_LAUNCH();
   }
   void children(Seg<T, D>* A, int lvl, int tied, Seg<T, D>* B) {
-    k_children<T, D><<<2 * gs, 128, 0, st>>>(A, lvl, tied, recs, rec_cap, B, small, small_capn, small_cap, max_leaf, thr,
-                                         tile_seg, ctl);
+    k_children<T, D><<<2 * gs, 128, 0, st>>>(A, lvl, tied, recs, rec_cap, B, lists, max_leaf, thr, tile_seg, ctl);
     PPTKG_CHECK_LAUNCH();
   }
 };
@@ -1858,9 +2170,6 @@ TreeBase* build_forest(const T* d_in, int64_t n, const int64_t* orig_off_h, int 
   off.release();
   st_prep.reset();
 
-  int cap_list;
-  size_t smem;
-  const int small_cap = small_capacity<T, D>(max_leaf, cap_list, smem);
   // a binary tree over nv points has at most 2 nv - 1 records
   const size_t rec_cap = 2 * (size_t)nv + 64;
   std::unique_ptr<Stage> st_scr(new Stage("build.scratch", st));
@@ -1868,23 +2177,16 @@ TreeBase* build_forest(const T* d_in, int64_t n, const int64_t* orig_off_h, int 
   Rec<T, D>* recs = recbuf.get();
   st_scr.reset();
 
-  // large segments per level are disjoint and above small_cap points
-  const int seg_cap = nv / (small_cap + 1) + 2;
-  const int max_tiles = nv / tile_points(n) + seg_cap + 2;
-  int small_capn = ncloud + 2 * 64 * (seg_cap + 1);
+  const int mid_cap = mid_capacity<T, D>(max_leaf);
+  int small_capn = ncloud + 2 * 64 * (mid_segments<T, D>(nv, max_leaf) + 1);
   int64_t most = 0;  // points of the largest cloud
   for (int c = 0; c < ncloud; c++) most = std::max(most, tree->valid_off_h[c + 1] - tree->valid_off_h[c]);
   int depth = 0;
   for (int attempt = 0; attempt < 4; attempt++, small_capn *= 4) {
     Stage st_att("build.attempt", st);
-    Levels<T, D> lv(nv, tile_points(n), max_tiles, seg_cap, small_capn, small_cap, tree->device, soa, recs, (int)rec_cap,
-                    tree->root_rec, max_leaf, thr, st);
+    Levels<T, D> lv(tree.get(), nv, n, small_capn, soa, recs, (int)rec_cap, st);
     BuildCtl* ctl = lv.ctl;
-    if (nv > 0) {
-      k_roots<T, D><<<div_up(ncloud, 128), 128, 0, st>>>(tree->valid_off, tree->orig_off, ncloud, small_cap,
-                                                          tile_points(n), lv.seg[0], lv.small, small_capn, ctl);
-      PPTKG_CHECK_LAUNCH();
-    }
+    if (nv > 0) lv.roots(tree->valid_off, tree->orig_off, ncloud);
     int levels = 0;
     {
       Stage st_levels("build.levels", st);
@@ -1894,13 +2196,13 @@ TreeBase* build_forest(const T* d_in, int64_t n, const int64_t* orig_off_h, int 
       // every level until four had none.
       int tied = 0;
       // The host looks every fourth level of a large build; of a smaller one
-      // after four, then once the largest cloud may be down to small segments,
-      // and then every second level.  Kernels of a level without segments exit
+      // after four, then once the largest cloud may be down to k_block's size
+      // or to leaves, and then every second level.  Kernels of a level without segments exit
       // at once.
       const bool often = nv < (1 << 21);
       int look = 2;
-      while (look < 32 && (most >> look) > small_cap) look++;
-      for (int lvl = 0; most > small_cap && lvl < MAX_LEVELS; lvl++) {
+      while (look < 32 && (most >> look) > std::max(mid_cap, max_leaf)) look++;
+      for (int lvl = 0; most > mid_cap && lvl < MAX_LEVELS; lvl++) {
         Seg<T, D>* A = lv.seg[lvl & 1];
         Seg<T, D>* B = lv.seg[(lvl + 1) & 1];
         lv.split(A, lvl, tied == 2 || lvl == 0);
@@ -1939,10 +2241,7 @@ TreeBase* build_forest(const T* d_in, int64_t n, const int64_t* orig_off_h, int 
     BuildCtl hctl;  // (its scalars)
     {
       Stage st_sub("build.subtree", st);
-      const int grid = std::max(1, std::min(small_capn, subtree_grid(smem, tree->device)));
-      k_subtree<T, D><<<grid, 32, smem, st>>>(lv.small, soa, recs, tree->root_rec, small_cap, cap_list, max_leaf,
-                                              thr, (int)rec_cap, small_capn, ctl);
-      PPTKG_CHECK_LAUNCH();
+      lv.finish(most);
       PPTKG_CUDA(cudaMemcpyAsync(&hctl, ctl, offsetof(BuildCtl, level_cnt), cudaMemcpyDeviceToHost, st));
       PPTKG_CUDA(cudaStreamSynchronize(st));
       // small list too short: again with more room (the points are partitioned
@@ -2076,17 +2375,13 @@ template <typename T, int D>
 void forest_capture_ready(TreeBase* t, cudaStream_t st) {
   if (t->capture) return;
   if (t->rec_dtype != F32 && t->rec_dtype != F64) throw Error(E_TYPE, "capture mode needs float32 or float64 points");
-  int cap_list;
-  size_t smem;
-  const int small_cap = small_capacity<T, D>(t->max_leaf, cap_list, smem);
   const int64_t n = t->n;
   t->cap_levels = std::min(t->levels + 8, MAX_LEVELS);
-  const int64_t seg_cap = n / (small_cap + 1) + 2;
-  // small segments: at most two children of every large segment of every
-  // level, plus the clouds' roots
-  const int64_t small = 2 * (int64_t)t->cap_levels * (seg_cap + 1) + t->ncloud + 64;
-  if (small > INT32_MAX) throw Error(E_INVALID, "forest too large for capture mode");
-  t->cap_small = (int)small;
+  // small segments: at most two children of every larger segment of every
+  // level (the planned depth is tdepth + 8), plus the clouds' roots; they are
+  // disjoint
+  const int64_t small = 2 * (int64_t)(t->tdepth + 8) * (mid_segments<T, D>(n, t->max_leaf) + 1) + t->ncloud + 64;
+  t->cap_small = (int)std::min<int64_t>(small, n + t->ncloud + 64);
   // records and traversal nodes: twice the first build's counts (a tree
   // over n points has at most 2n - 1 records); a rebuild that needs more
   // stops with code 21
@@ -2097,7 +2392,6 @@ void forest_capture_ready(TreeBase* t, cudaStream_t st) {
   t->cap_tnodes = std::min<int64_t>(t->cap_recs, 2 * live_tnodes + 4096) + t->ncloud;
   if (t->cap_recs > INT32_MAX / 2 || t->cap_tnodes > INT32_MAX / 2)
     throw Error(E_INVALID, "forest too large for capture mode");
-  t->cap_subgrid = subtree_grid(smem, t->device);
   // capacity-sized arrays, current contents kept
   auto grow = [&](void** p, size_t have, size_t want) {
     void* q = nullptr;
@@ -2148,20 +2442,14 @@ void rebuild_forest(TreeBase* t, const T* d_in, cudaStream_t st, int* status) {
   }
   flag.release();
   off.release();
-  int cap_list;
-  size_t smem;
-  const int small_cap = small_capacity<T, D>(t->max_leaf, cap_list, smem);
   const int rec_cap = (int)t->cap_recs;
   Rec<T, D>* recs = (Rec<T, D>*)t->recs;
-  const int seg_cap = (int)(n / (small_cap + 1) + 2);
-  const int max_tiles = (int)(n / tile_points(n)) + seg_cap + 2;
-  Levels<T, D> lv(n, tile_points(n), max_tiles, seg_cap, t->cap_small, small_cap, t->device, soa, recs, rec_cap, t->root_rec,
-                  t->max_leaf, t->empty_split, st);
+  int64_t most = 0;  // points that the largest cloud may have
+  for (int c = 0; c < ncloud; c++) most = std::max(most, t->orig_off_h[c + 1] - t->orig_off_h[c]);
+  Levels<T, D> lv(t, n, n, t->cap_small, soa, recs, rec_cap, st);
   BuildCtl* ctl = lv.ctl;
   PPTKG_CUDA(cudaMemsetAsync(t->root_rec, 0xff, sizeof(int) * ncloud, st));
-  k_roots<T, D><<<div_up(ncloud, 128), 128, 0, st>>>(t->valid_off, t->orig_off, ncloud, small_cap, tile_points(n),
-                                                      lv.seg[0],                                                      lv.small, t->cap_small, ctl);
-  PPTKG_CHECK_LAUNCH();
+  lv.roots(t->valid_off, t->orig_off, ncloud);
   {
     // a fixed number of levels; the kernels of a level without segments
     // return at once
@@ -2173,11 +2461,9 @@ void rebuild_forest(TreeBase* t, const T* d_in, cudaStream_t st, int* status) {
       lv.children(A, lvl, 2, B);
     }
   }
-  // the persistent subtree kernel takes the small segments; blocks without
-  // work return
-  k_subtree<T, D><<<t->cap_subgrid, 32, smem, st>>>(lv.small, soa, recs, t->root_rec, small_cap, cap_list,
-                                                             t->max_leaf, t->empty_split, rec_cap, t->cap_small, ctl);
-  PPTKG_CHECK_LAUNCH();
+  // the persistent kernels take the smaller segments; blocks without work
+  // return
+  lv.finish(most);
   k_rebuild_status<<<1, 1, 0, st>>>(ctl, t->cap_levels, t->tdepth, status, t->dev_meta, t->valid_off, ncloud);
   PPTKG_CHECK_LAUNCH();
   // tree-ordered points and the forward map

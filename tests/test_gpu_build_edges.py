@@ -1,9 +1,73 @@
-"""Builds and in-place rebuilds at the edges of their capacities.  Every
-accepted tree must be the reference's (from the CPU oracle)."""
+"""Builds and in-place rebuilds at the edges of their capacities: chains of
+thousands of levels, the second attempt of a build whose list of small
+segments overflowed, and rebuilds that need other shapes of tree than the
+first build's.  Every accepted tree must be the reference's (from the CPU
+oracle)."""
 import numpy as np
 import pytest
 
 pytestmark = pytest.mark.gpu
+
+
+def _is_reference_tree(t, o):
+    assert np.array_equal(t.reverse_indices(), o.reverse_indices())
+    assert np.array_equal(t.ref_nodes(), o.nodes())
+
+
+def _axis_chains(per_axis, lowest=1e-300):
+    """Points on the axes from 1e300 down by factors of 2.05 (float64): every midpoint split
+    takes one point off."""
+    v = 10.0 ** (300 - np.log10(2.05) * np.arange(per_axis))
+    assert v[-1] > lowest
+    p = np.zeros((3 * per_axis, 3))
+    for d in range(3):
+        p[d * per_axis:(d + 1) * per_axis, d] = v
+    return p
+
+
+def test_more_than_4096_levels_of_large_segments(gpu, port):
+    # 4,800 levels, 4,544 of them with a segment above the subtree kernel's 256
+    # float64 points
+    P = _axis_chains(1600)[np.random.default_rng(0).permutation(4800)]
+    _is_reference_tree(gpu.kdtree._build(P), port.PortTree(P))
+
+
+def _rebuilt(first, second, off, maxleafsize=10):
+    import torch
+    from pptk_b200 import ragged
+    f = ragged.Forest(torch.from_numpy(first).cuda(), off, maxleafsize=maxleafsize)
+    f.capture_ready()
+    f.rebuild(torch.from_numpy(second).cuda())
+    return f
+
+
+def _are_reference_trees(f, P, off, port, maxleafsize=10):
+    rev = f.reverse_indices()
+    for c in range(0, len(off) - 1, max(1, (len(off) - 1) // 50)):
+        o = port.PortTree(P[off[c]:off[c + 1]], maxleafsize=maxleafsize)
+        assert np.array_equal(rev[off[c]:off[c + 1]] - off[c], o.reverse_indices()), c
+        assert np.array_equal(f.ref_nodes(c), o.nodes()), c
+
+
+def _chain_to_copies(rng, n, chain, copies):
+    """Half a box of points, and in the other half powers of two along an axis
+    down to copies of one point."""
+    p = rng.random((n, 3))
+    p[:, 0] = 0.5 + 0.5 * p[:, 0]
+    p[:chain + copies] = (0.0, 0.25, 0.25)
+    p[:chain, 0] = 0.25 * 2.0 ** -np.arange(chain)
+    return p
+
+
+@pytest.mark.parametrize("dtype,copies", [(np.float32, 700), (np.float64, 400)])
+def test_rebuild_with_segments_below_the_planned_levels(gpu, port, dtype, copies):
+    # a tree of 14 levels where 19 are planned for, but with 700 (400) points
+    # in one segment three levels below the last grid-wide one
+    rng = np.random.default_rng(0)
+    off = np.array([0, 3000, 6000])
+    A = rng.random((6000, 3)).astype(dtype)
+    B = np.concatenate([_chain_to_copies(rng, 3000, 24, copies) for _ in range(2)]).astype(dtype)
+    _are_reference_trees(_rebuilt(A, B, off), B, off, port)
 
 
 def test_refused_rebuild_leaves_every_record_readable(gpu):
