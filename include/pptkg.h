@@ -299,11 +299,13 @@ PPTKG_API int64_t pptkg_launch_count(void);
 
 /* Run-time tuning (no reference counterpart; set by the autotuner,
  * pptk_b200/autotune.py).  Settings are process-wide and read at launch.
- *   "lane_span": kNN and normal batches whose 32-query packets would span
- *     more than this many tree positions on average (a third of it for
- *     k > 16) run one warp per query, as do batches of at most 65,536
- *     queries (-1: packets only, up to k = 64).  Default 1024.  Results do
- *     not depend on it.
+ *   "lane_span": kNN and normal batches too small to fill the GPU with
+ *     32-query packets, or whose packets would span too many tree positions,
+ *     run one warp per query.  1024 (default): the measured line between the
+ *     two, which depends on k, the type, the sizes and whether the queries
+ *     come in tree order; other values scale it (smaller: more batches run
+ *     one warp per query), 0: all do, -1: none with k of up to 64.  Results
+ *     do not depend on it.
  *   "rnear_warp_queries": pptkg_rnear_count / pptkg_rnear_fill calls, and
  *     normals over r-near neighbourhoods (k = -1), with at most this many
  *     queries, or whose packets would span more than 512 tree positions,

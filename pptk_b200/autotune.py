@@ -4,9 +4,9 @@ Five settings shape every kNN / normal traversal; none changes a result:
 
 * the leaf bucket size of the traversal hierarchy (``set_bucket`` on a tree
   or forest): larger buckets mean fewer node visits and more candidates;
-* ``lane_span`` (``pptkg_tune_set``): batches whose 32-query packets would
-  span more tree positions than this on average run one warp per query
-  instead -- the warps-per-query choice of the kNN walks;
+* ``lane_span`` (``pptkg_tune_set``): which batches run one warp per query
+  instead of 32-query packets -- the warps-per-query choice of the kNN walks
+  (1024: the measured line, smaller: more batches, 0: all, -1: none);
 * ``warm_bound``: whether the warm-started lists also take the seed bound of
   a wider window of tree-order neighbours;
 * ``topk_min``: the k-tiling of the register top-k lists (their compile-time

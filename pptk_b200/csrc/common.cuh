@@ -45,9 +45,8 @@ enum Status {
 extern std::atomic<long long> g_launches;
 
 // Run-time tuning knobs (pptkg_tune_set / pptkg_tune_get), read at launch.
-//  lane_span: kNN and normal batches whose 32-query packets would span more
-//    than this many tree positions on average run one warp per query, as do
-//    small batches (-1: never).
+//  lane_span: which kNN and normal batches run one warp per query (by_warp):
+//    1024 the measured line, smaller values more of them, 0 all, -1 none.
 extern std::atomic<int> g_tune_lane_span;
 //  rnear_warp_queries: r-near batches of at most this many queries, or too
 //    scattered for packets, run one warp per query (0: never).

@@ -9,7 +9,6 @@
 #include "normals.cuh"
 #include "profile.cuh"
 #include "query.cuh"
-#include "rules.cuh"
 #include "util.cuh"
 
 namespace pptkg {
@@ -479,6 +478,12 @@ static __global__ void k_place(const int* key, int m, int shift, int* cursor, in
   if (i < m) order[atomicAdd(&cursor[key[i] >> shift], 1)] = i;
 }
 
+// What a single tree's batch needs before its queries are in tree order.
+static BatchOrder batch_order(const TreeBase* t, const QuerySpec& qs) {
+  if (qs.pts) return BatchOrder::points;
+  return !qs.idx && qs.m == t->nv && t->n == t->nv ? BatchOrder::tree : BatchOrder::rows;
+}
+
 // Builds a processing order in which queries near each other in the tree are
 // adjacent (counting sort on the tree position key).  Returns the order mode.
 //
@@ -492,7 +497,7 @@ int make_order(const TreeBase* t, const QuerySpec& qs, DevBuf<int>& order, cudaS
   const int m = (int)qs.m;
   const int nv = (int)t->nv;
   if (m <= 0) return 0;
-  if (!qs.pts && !qs.idx && m == nv && t->n == t->nv) return 2;  // all points, tree order
+  if (batch_order(t, qs) == BatchOrder::tree) return 2;  // all points
   const bool locate = qs.pts && (anchors || m >= 2048);
   DevBuf<int> keybuf((locate && anchors) || (!locate && m < 2048) ? 0 : m, st);
   int* key = locate && anchors ? anchors : keybuf.get();
@@ -630,29 +635,9 @@ __global__ void __launch_bounds__(QTHREADS) k_knn_warp(TreeView<T, D> tv, L ld, 
   if (out_cnt && lane == 0) out_cnt[row] = n;
 }
 
-// Largest k of the warp lists.
-constexpr int WARP_MAX_K = 256;
-// Warp-per-query batches above this size are sorted by tree position first.
-constexpr int WARP_UNSORTED = 65536;
-
-// Whether a batch of m queries on trees of nv points runs one warp per query
-// in place of 32-query packets: beyond the packets' lists (k > 64) always;
-// otherwise a batch too small to fill the GPU with packets, or whose packets
-// would span more than lane_span tree positions on average (a third of it
-// for lists of more than 16, whose insertions packets pay for more dearly).
-// us, packets / warps, points of a scene in no order:
-//   k = 16, 2M points:  30k 375 / 166, 60k 376 / 269, 100k 418 / 375, 200k 543 / 636
-//   k = 16, 20M points: 60k 860 / 305, 200k 1075 / 750, 400k 1483 / 1365, 700k 2040 / 2249
-//   k = 32, 2M points:  60k 629 / 327, 200k 969 / 836, 400k 1526 / 1550
-//   k = 32, 20M points: 200k 1864 / 974, 1M 4703 / 4157, 2M 7743 / 8065
-//   normals, k = 16, 2M points: 10k 432 / 117, 60k 368 / 276, 100k 438 / 510
-inline bool by_warp(int64_t nv, int64_t m, int k) {
-  if (k > WARP_MAX_K) return false;
-  if (k > KNN_MAX_K) return true;
-  const int span = g_tune_lane_span.load();
-  if (span < 0) return false;
-  const int f = k > 16 ? 3 : 1;
-  return m <= 65536 || 32 * f * nv > m * span;
+template <typename T>
+bool by_warp(int64_t nv, int64_t m, int k, Answer a, BatchOrder order) {
+  return by_warp(nv, m, k, std::is_same<typename DistOf<T>::type, double>::value, a, order, g_tune_lane_span.load());
 }
 
 template <typename T, int D, typename L, bool POS>
@@ -789,8 +774,9 @@ void knn_query(const TreeBase* t, const QuerySpec& qs, int k, double dmax, int32
   if (k > KNN_MAX_K) check_depth(t);
   DevBuf<int> status(1, st);
   PPTKG_CUDA(cudaMemsetAsync(status.get(), 0, sizeof(int), st));
-  const bool warps = by_warp(t->nv, m, k);
-  const bool sorted = !warps || m > WARP_UNSORTED;
+  const BatchOrder kind = batch_order(t, qs);
+  const bool warps = by_warp<T>(t->nv, m, k, Answer::knn, kind);
+  const bool sorted = !warps || kind == BatchOrder::tree || m > warp_unsorted(kind);
   DevBuf<int> order, anchors(qs.pts && sorted ? m : 0, st);
   int mode = 0;
   if (sorted)
@@ -1810,9 +1796,12 @@ void normals_query(const TreeBase* t, const QuerySpec& qs_in, int k, float r, in
   DevBuf<int> order;
   // (tree order covers valid points only: rows of dropped points, none when
   // n == nv, need no separate pass)
-  const bool warps = k == -1 ? rnear_by_warp(t->nv, m) : by_warp(t->nv, m, k);
+  const BatchOrder kind = batch_order(t, qs);
+  const bool warps = k == -1 ? rnear_by_warp(t->nv, m) : by_warp<T>(t->nv, m, k, Answer::normals, kind);
   int mode = 0;
-  if (k > 0 && warps && m <= WARP_UNSORTED)
+  // (long lists of warps gain nothing from tree order: k = 64, double, 40k
+  // points 602 us as they come, 657 in tree order; k = 16 240 and 232)
+  if (k > 0 && warps && (kind != BatchOrder::tree || k > 16) && m <= warp_unsorted(kind))
     check_indices(t, qs, st);
   else
     mode = make_order<T, 3>(t, qs, order, st);
@@ -1967,7 +1956,7 @@ void forest_knn(const TreeBase* t, int k, double dmax, bool exclude_self, int32_
   const DistT r2 = radius2<DistT>(dmax);
   Stage stage("forest.knn", st);
   auto run = [&](auto ld) {
-    if (by_warp(n_slots, n_slots, k))
+    if (by_warp<T>(n_slots / t->ncloud, n_slots, k, Answer::knn, BatchOrder::tree))
       launch_knn_warp<T, D, decltype(ld), false>(t, ld, nullptr, 0, 0, (int)n_slots, k, r2, d_idx, d_cnt,
                                                  status.get(), st, fm);
     else
@@ -2009,20 +1998,22 @@ void forest_normals(const TreeBase* t, int k, float r, int num_eigen, int precis
   const DistT rr = (DistT)(T)r;
   const DistT r2 = rr * rr;
   int prec = precision == PREC_AUTO ? (sizeof(T) == 4 ? PREC_FP32 : PREC_FP64) : precision;
+  const bool warps = by_warp<T>(n_slots / t->ncloud, n_slots, k, d_idx ? Answer::both : Answer::normals,
+                                BatchOrder::tree);
   if (d_idx) {
     // one walk for the self kNN (the list excludes the query point) and
     // the normal (the query point put back in)
     Stage stage("forest.knn_normals", st);
     dispatch_normals<T, IndexQueries<3, true>>(t, IndexQueries<3, true>{nullptr, t->fwd}, nullptr, 0, (int)n_slots,
                                                k, r2, num_eigen, prec, gap_thr, d_evecs, d_evals, d_sizes,
-                                               status.get(), st, by_warp(n_slots, n_slots, k), fm, d_idx, d_cnt);
+                                               status.get(), st, warps, fm, d_idx, d_cnt);
     status.check(st, "forest kNN + normals");
     return;
   }
   Stage stage("forest.normals", st);
   dispatch_normals<T, IndexQueries<3, false>>(t, IndexQueries<3, false>{nullptr, t->fwd}, nullptr, 0, (int)n_slots,
                                               k, r2, num_eigen, prec, gap_thr, d_evecs, d_evals, d_sizes, status.get(),
-                                              st, by_warp(n_slots, n_slots, k), fm);
+                                              st, warps, fm);
   status.check(st, "forest normals");
 }
 
@@ -2154,8 +2145,8 @@ void multi_knn(const TreeBase* const* trees, int ntrees, const void* d_q, int qd
   multi_tables<T, D>(trees, ntrees, rows, mt, st);
   if (mt.n_slots == 0) return;
   const size_t qbytes = (qdtype == F64 ? sizeof(double) : sizeof(float)) * D;
-  const bool warps = by_warp(mt.nv, rows[ntrees], k);
-  if (!warps || rows[ntrees] > WARP_UNSORTED)
+  const bool warps = by_warp<T>(mt.nv, rows[ntrees], k, Answer::knn, BatchOrder::points);
+  if (!warps || rows[ntrees] > warp_unsorted(BatchOrder::points))
     multi_order<T, D>(trees, ntrees, rows, mt, [&](int g) {
       QuerySpec qs;
       qs.pts = (const char*)d_q + rows[g] * qbytes;
@@ -2194,8 +2185,8 @@ void multi_normals(const TreeBase* const* trees, int ntrees, const int32_t* d_id
   if (mt.n_slots == 0) return;
   // query indices are checked against their own tree's rows by the kernels
   // (status 4); the ordering pass maps bad ones to the end of the order
-  const bool warps = by_warp(mt.nv, rows[ntrees], k);
-  if (!warps || rows[ntrees] > WARP_UNSORTED)
+  const bool warps = by_warp<T>(mt.nv, rows[ntrees], k, Answer::normals, BatchOrder::rows);
+  if (!warps || rows[ntrees] > warp_unsorted(BatchOrder::rows))
     multi_order<T, 3>(trees, ntrees, rows, mt, [&](int g) {
       QuerySpec qs;
       qs.idx = d_idx + rows[g];
@@ -2267,7 +2258,8 @@ static void normals_noalloc_k(const TreeBase* t, const int32_t* idx, int m, int 
   typedef IndexQueries<3, false> L;
   L ld{idx, t->fwd};
   const int mode = (!idx && m == t->nv && t->n == t->nv) ? 2 : 0;
-  const bool warps = by_warp(t->nv, m, k);
+  // (rows stay in their order: there is no memory to sort them in)
+  const bool warps = mode == 2 ? by_warp<T>(t->nv, m, k, Answer::normals, BatchOrder::tree) : g_tune_lane_span.load() >= 0;
   int* status = scratch;
   int* nfix = scratch + 1;
   int* fix = scratch + NOALLOC_QUEUE_OFFSET;

@@ -1,6 +1,7 @@
 // Host entry points of the query kernels (kNN, r-near, normals).
 #pragma once
 
+#include "rules.cuh"
 #include "tree.cuh"
 
 namespace pptkg {
@@ -16,8 +17,6 @@ struct QuerySpec {
   // index queries exclude the query point itself (the reference's *Self forms)
   bool exclude_self = true;
 };
-
-constexpr int KNN_MAX_K = 64;
 
 template <typename T, int D>
 void knn_query(const TreeBase* t, const QuerySpec& qs, int k, double dmax, int32_t* d_idx, int32_t* d_cnt,

@@ -179,7 +179,7 @@ struct TreeBase {
   // depth) are those of the last direct build or forest_sync; dev_meta
   // holds the device's {nv, n_recs, depth, 0} of the last rebuild.
   bool capture = false;
-  int cap_levels = 0, cap_small = 0, cap_subgrid = 0;
+  int cap_levels = 0, cap_small = 0;
   int64_t cap_recs = 0, cap_tnodes = 0;
   int64_t* dev_meta = nullptr;
   size_t device_bytes() const;
