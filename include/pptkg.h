@@ -238,8 +238,9 @@ PPTKG_API int pptkg_forest_knn_normals(const pptkg_tree* forest, int k, float r,
  * set, so that rebuild, pptkg_forest_knn and pptkg_forest_normals can be
  * captured together; the trees equal those pptkg_forest_build gives for the
  * new coordinates.  The capacities are the first build's tree levels + 8
- * and twice its records and traversal nodes; sink code 20 (more levels) or
- * 21 (more records), without a sink PPTKG_E_UNSUPPORTED, means the
+ * and twice its records and traversal nodes (the wide hierarchy's nodes
+ * follow from these); sink code 20 (more levels) or 21 (more records or
+ * traversal nodes), without a sink PPTKG_E_UNSUPPORTED, means the
  * coordinates need more than that: the trees of that pass are not the
  * reference trees and the forest must be built again.  Host-side reads
  * (pptkg_forest_info, pptkg_tree_info, ref nodes, save) synchronise the

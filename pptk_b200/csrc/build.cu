@@ -1792,6 +1792,15 @@ void wide_begin(TreeBase* t, int n_recs, cudaStream_t st, const int* n_dev = nul
   exclusive_scan<NodeWord, int>((const NodeWord*)t->wbits, t->wrank, levels * words, t->wrank + levels * words, st);
 }
 
+// Wide nodes that a rebuild within the capacities of records and traversal
+// nodes can have: on every level one per cloud and one more per record that
+// the level divides.  Those have two children, as half of all records have at
+// most; above the first level they are of more than `bucket` points and so are
+// traversal nodes.
+static int wide_capacity(const TreeBase* t) {
+  return (int)std::min<int64_t>(INT32_MAX / 2, t->cap_recs / 2 + t->ncloud + (t->wlevels - 1) * t->cap_tnodes);
+}
+
 template <typename T, int D>
 void wide_alloc(TreeBase* t, int n_wide, cudaStream_t st) {
   if (t->wide) dev_free(t->wide, st);
@@ -2317,9 +2326,11 @@ void make_tnodes(TreeBase* tree, int bucket, cudaStream_t st) {
     PPTKG_CUDA(cudaMemcpyAsync(&nt, tid.get() + nr, sizeof(int), cudaMemcpyDeviceToHost, st));
   }
   PPTKG_CUDA(cudaStreamSynchronize(st));
-  // (a capture-ready forest keeps at least the capacity it has)
-  wide_alloc<T, D>(tree, tree->capture ? std::max(n_wide, tree->n_wide) : n_wide, st);
-  wide_fill<T, D>(tree, nr, tree->capture, st);
+  // (a capture-ready forest's follows below from its traversal nodes' capacity)
+  if (!tree->capture) {
+    wide_alloc<T, D>(tree, n_wide, st);
+    wide_fill<T, D>(tree, nr, false, st);
+  }
   TNode<T, D>* nodes = nullptr;
   // a capture-ready forest keeps the capacity that its rebuilds fill
   const int64_t cap = tree->capture ? std::max<int64_t>(tree->cap_tnodes, (int64_t)nt + tree->ncloud)
@@ -2328,6 +2339,10 @@ void make_tnodes(TreeBase* tree, int bucket, cudaStream_t st) {
   PPTKG_CUDA(dev_malloc((void**)&nodes, (size_t)cap * sizeof(TNode<T, D>), st));
   tree->tnodes = nodes;
   tree->n_tnodes = (int)cap;
+  if (tree->capture) {
+    wide_alloc<T, D>(tree, wide_capacity(tree), st);
+    wide_fill<T, D>(tree, nr, true, st);
+  }
   if (nt > 0) {
     k_tfill<T, D><<<div_up(nr, 256), 256, 0, st>>>(recs, nr, flag.get(), tid.get(), nodes);
     PPTKG_CHECK_LAUNCH();
@@ -2406,11 +2421,11 @@ void forest_capture_ready(TreeBase* t, cudaStream_t st) {
   grow(&t->tnodes, (size_t)t->n_tnodes * sizeof(TNode<T, D>), (size_t)t->cap_tnodes * sizeof(TNode<T, D>));
   t->n_tnodes = (int)t->cap_tnodes;
   t->tdepth += 8;
-  // wide nodes: twice the first build's; the map covers all input rows
+  // the map covers all input rows; the wide nodes follow from the records and
+  // traversal nodes
   t->capture = true;
-  const int wide_now = t->n_wide;
   wide_begin<T, D>(t, t->n_recs, st);
-  wide_alloc<T, D>(t, (int)std::min<int64_t>(INT32_MAX / 2, 2 * (int64_t)wide_now + 4096 + t->ncloud * t->wlevels), st);
+  wide_alloc<T, D>(t, wide_capacity(t), st);
   wide_fill<T, D>(t, t->n_recs, true, st);
   if (!t->dev_meta) PPTKG_CUDA(dev_malloc((void**)&t->dev_meta, 4 * sizeof(int64_t), st));
   PPTKG_CUDA(cudaStreamSynchronize(st));

@@ -70,6 +70,25 @@ def test_rebuild_with_segments_below_the_planned_levels(gpu, port, dtype, copies
     _are_reference_trees(_rebuilt(A, B, off), B, off, port)
 
 
+def test_rebuild_with_more_wide_nodes_than_the_first_build(gpu, port):
+    # clouds of 40 points: two leaf ranges each in the first build, nine of a
+    # chain in the second, with as many records as before
+    rng = np.random.default_rng(0)
+    clouds = 3000
+    off = 40 * np.arange(clouds + 1)
+    one = rng.random((40, 3)) * 2.0 ** -9
+    one[:8] = 0.0
+    one[:8, 0] = 2.0 ** -np.arange(8)
+    A = rng.random((40 * clouds, 3)).astype(np.float32)
+    B = np.tile(one, (clouds, 1)).astype(np.float32)
+    f = _rebuilt(A, B, off, maxleafsize=1)
+    _are_reference_trees(f, B, off, port, maxleafsize=1)
+    idx, cnt = f.knn(5)
+    oi, oc = port.PortTree(B[:40]).knn_self(np.arange(40, dtype=np.int32), 5)
+    assert np.array_equal(cnt.cpu().numpy(), np.tile(oc, clouds))
+    assert np.array_equal(idx.cpu().numpy(), np.tile(oi, (clouds, 1)) + np.repeat(off[:-1], 40)[:, None])
+
+
 def test_refused_rebuild_leaves_every_record_readable(gpu):
     # ties move every split of a chain of segments above 8,192 points, past the
     # last planned level: the segment left over has a record but no decision
