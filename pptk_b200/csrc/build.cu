@@ -2151,12 +2151,17 @@ TreeBase* build_forest(const T* d_in, int64_t n, const int64_t* orig_off_h, int 
 
   // valid-point compaction (ValidPointIndices, kdtree-impl.h:53-75), per cloud
   std::unique_ptr<Stage> st_prep(new Stage("build.prep", st));
-  BuildBuf<int> flag(n + 1, st), off(n + 1, st);
-  if (n > 0) {
-    k_valid<T, D><<<div_up(n, 256), 256, 0, st>>>(d_in, n, flag.get());
-    PPTKG_CHECK_LAUNCH();
-  }
-  exclusive_scan<int, int>(flag.get(), off.get(), n, off.get() + n, st);
+  BuildBuf<int> flag, off;
+  auto find_valid = [&]() {
+    flag.alloc(n + 1, st);
+    off.alloc(n + 1, st);
+    if (n > 0) {
+      k_valid<T, D><<<div_up(n, 256), 256, 0, st>>>(d_in, n, flag.get());
+      PPTKG_CHECK_LAUNCH();
+    }
+    exclusive_scan<int, int>(flag.get(), off.get(), n, off.get() + n, st);
+  };
+  find_valid();
   k_cloud_off<<<div_up(ncloud + 1, 256), 256, 0, st>>>(off.get(), tree->orig_off, ncloud, tree->valid_off);
   PPTKG_CHECK_LAUNCH();
   tree->valid_off_h.resize(ncloud + 1);
@@ -2171,12 +2176,15 @@ TreeBase* build_forest(const T* d_in, int64_t n, const int64_t* orig_off_h, int 
   SoA<T, D> soa;
   for (int d = 0; d < D; d++) soa.x[d] = xs.get() + (size_t)d * nv;
   soa.id = ids.get();
-  if (n > 0) {
-    k_compact<T, D><<<div_up(n, 256), 256, 0, st>>>(d_in, n, flag.get(), off.get(), soa);
-    PPTKG_CHECK_LAUNCH();
-  }
-  flag.release();
-  off.release();
+  auto take_points = [&]() {
+    if (n > 0) {
+      k_compact<T, D><<<div_up(n, 256), 256, 0, st>>>(d_in, n, flag.get(), off.get(), soa);
+      PPTKG_CHECK_LAUNCH();
+    }
+    flag.release();
+    off.release();
+  };
+  take_points();
   st_prep.reset();
 
   // a binary tree over nv points has at most 2 nv - 1 records
@@ -2187,13 +2195,18 @@ TreeBase* build_forest(const T* d_in, int64_t n, const int64_t* orig_off_h, int 
   st_scr.reset();
 
   const int mid_cap = mid_capacity<T, D>(max_leaf);
-  int small_capn = ncloud + 2 * 64 * (mid_segments<T, D>(nv, max_leaf) + 1);
+  // (small segments are disjoint: at most one per point)
+  int64_t small_capn = std::min<int64_t>(nv, ncloud + 2 * 64 * ((int64_t)mid_segments<T, D>(nv, max_leaf) + 1));
   int64_t most = 0;  // points of the largest cloud
   for (int c = 0; c < ncloud; c++) most = std::max(most, tree->valid_off_h[c + 1] - tree->valid_off_h[c]);
   int depth = 0;
-  for (int attempt = 0; attempt < 4; attempt++, small_capn *= 4) {
+  for (int attempt = 0; attempt < 4; attempt++, small_capn = attempt < 3 ? std::min<int64_t>(nv, 4 * small_capn) : nv) {
     Stage st_att("build.attempt", st);
-    Levels<T, D> lv(tree.get(), nv, n, small_capn, soa, recs, (int)rec_cap, st);
+    if (attempt > 0) {
+      find_valid();
+      take_points();
+    }
+    Levels<T, D> lv(tree.get(), nv, n, (int)small_capn, soa, recs, (int)rec_cap, st);
     BuildCtl* ctl = lv.ctl;
     if (nv > 0) lv.roots(tree->valid_off, tree->orig_off, ncloud);
     int levels = 0;
@@ -2253,8 +2266,9 @@ TreeBase* build_forest(const T* d_in, int64_t n, const int64_t* orig_off_h, int 
       lv.finish(most);
       PPTKG_CUDA(cudaMemcpyAsync(&hctl, ctl, offsetof(BuildCtl, level_cnt), cudaMemcpyDeviceToHost, st));
       PPTKG_CUDA(cudaStreamSynchronize(st));
-      // small list too short: again with more room (the points are partitioned
-      // by now, so every pass of the second attempt finds them in place)
+      // small list too short: again with more room, from the points in their
+      // input order (a split inside a run of equal values divides it by the
+      // order that it finds)
       if (hctl.status == 7 && attempt < 3) continue;
       if (hctl.status)
         throw Error(E_DEVICE, "device build: check failed (code " + std::to_string(hctl.status) + ")");

@@ -32,6 +32,16 @@ def test_more_than_4096_levels_of_large_segments(gpu, port):
     _is_reference_tree(gpu.kdtree._build(P), port.PortTree(P))
 
 
+def test_second_attempt_builds_from_the_input_order(gpu, port):
+    # 2,850 levels give more small segments than the first attempt's list
+    # holds; the lattice below them has splits inside runs of equal values,
+    # whose order depends on that of the points the attempt starts from
+    rng = np.random.default_rng(1)
+    P = np.concatenate([_axis_chains(950, 20.0), rng.integers(0, 9, (1500, 3)) * 1.0])
+    P = P[rng.permutation(len(P))]
+    _is_reference_tree(gpu.kdtree._build(P), port.PortTree(P))
+
+
 def _rebuilt(first, second, off, maxleafsize=10):
     import torch
     from pptk_b200 import ragged
