@@ -44,6 +44,8 @@ int guarded(F&& f) {
   } catch (const Error& e) {
     g_msg = e.what();
     g_code = e.code;
+    // (reported here: the next call's launch checks must not find it again)
+    if (e.code == E_CUDA) (void)cudaGetLastError();
   } catch (const std::bad_alloc&) {
     g_msg = "host allocation failed";
     g_code = PPTKG_E_CUDA;

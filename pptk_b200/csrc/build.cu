@@ -1775,7 +1775,7 @@ void wide_begin(TreeBase* t, int n_recs, cudaStream_t st, const int* n_dev = nul
     most = std::max(most, t->capture ? t->orig_off_h[c + 1] - t->orig_off_h[c] : t->valid_off_h[c + 1] - t->valid_off_h[c]);
   const int levels = wide_levels(t->bucket, most);
   const int64_t words = wide_words(t->capture ? t->n : t->nv);
-  if (!t->wbits || t->wlevels != levels || t->wwords != (int)words) {
+  if (!t->wbits || !t->wrank || t->wlevels != levels || t->wwords != (int)words) {
     if (t->wbits) dev_free(t->wbits, st);
     if (t->wrank) dev_free(t->wrank, st);
     t->wbits = nullptr;
@@ -1852,6 +1852,7 @@ void make_wide(TreeBase* t, cudaStream_t st) {
   wide_alloc<T, D>(t, n, st);
   wide_fill<T, D>(t, t->n_recs, true, st);
   PPTKG_CUDA(cudaStreamSynchronize(st));
+  t->walkable = true;
 }
 
 // ------------------------------------------------------------ host side ----
@@ -2323,6 +2324,7 @@ void make_tnodes(TreeBase* tree, int bucket, cudaStream_t st) {
     dev_free(tree->tnodes, st);
     tree->tnodes = nullptr;
   }
+  tree->walkable = false;
   if (bucket < 1) bucket = 1;
   tree->bucket = bucket;
   const int nr = tree->n_recs;
@@ -2377,6 +2379,7 @@ void make_tnodes(TreeBase* tree, int bucket, cudaStream_t st) {
     tree->root_lo[d] = box[d];
     tree->root_hi[d] = box[4 + d];
   }
+  tree->walkable = true;
 }
 
 #ifndef PPTKG_BUILD_INT
@@ -2435,19 +2438,22 @@ void forest_capture_ready(TreeBase* t, cudaStream_t st) {
   grow(&t->tnodes, (size_t)t->n_tnodes * sizeof(TNode<T, D>), (size_t)t->cap_tnodes * sizeof(TNode<T, D>));
   t->n_tnodes = (int)t->cap_tnodes;
   t->tdepth += 8;
+  if (!t->dev_meta) PPTKG_CUDA(dev_malloc((void**)&t->dev_meta, 4 * sizeof(int64_t), st));
   // the map covers all input rows; the wide nodes follow from the records and
   // traversal nodes
   t->capture = true;
+  t->walkable = false;
   wide_begin<T, D>(t, t->n_recs, st);
   wide_alloc<T, D>(t, wide_capacity(t), st);
   wide_fill<T, D>(t, t->n_recs, true, st);
-  if (!t->dev_meta) PPTKG_CUDA(dev_malloc((void**)&t->dev_meta, 4 * sizeof(int64_t), st));
   PPTKG_CUDA(cudaStreamSynchronize(st));
+  t->walkable = true;
 }
 
 template <typename T, int D>
 void rebuild_forest(TreeBase* t, const T* d_in, cudaStream_t st, int* status) {
   if (!t->capture) throw Error(E_INVALID, "rebuild needs a capture-ready forest");
+  require_walkable(t);
   Stage stage("rebuild", st);
   const int64_t n = t->n;
   const int ncloud = t->ncloud;

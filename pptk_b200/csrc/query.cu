@@ -22,6 +22,7 @@ inline int wide_stack(int levels) { return 34 * (levels > 1 ? levels - 1 : 1); }
 
 template <typename T, int D>
 TreeView<T, D> view_of(const TreeBase* t) {
+  require_walkable(t);
   TreeView<T, D> v;
   v.pts = (const PointRec<T, D>*)t->pts;
   v.nodes = (const TNode<T, D>*)t->tnodes;
@@ -2101,6 +2102,7 @@ static TreeBase* bounds_tree(int depth, int n_nodes, int wlevels, int64_t nv) {
   b->n_tnodes = n_nodes;
   b->wlevels = wlevels;
   b->nv = nv;
+  b->walkable = true;
   return b;
 }
 

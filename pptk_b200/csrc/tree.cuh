@@ -159,6 +159,7 @@ struct TreeBase {
   uint32_t* wbits = nullptr;  // [wlevels * wwords]
   int32_t* wrank = nullptr;   // [wlevels * wwords + 1], the last: nodes of the last build
   int n_wide = 0, wlevels = 0, wwords = 0;
+  bool walkable = false;  // both hierarchies are complete (not while, or where memory ran out as, they change)
   int ncloud = 1;
   int32_t* root_rec = nullptr;    // device [ncloud]: root record per cloud (-1: no valid point)
   int32_t* root_tnode = nullptr;  // device [ncloud]
@@ -185,5 +186,12 @@ struct TreeBase {
   size_t device_bytes() const;
   ~TreeBase();
 };
+
+// A tree whose hierarchies an allocation failure left incomplete is refused
+// until they have been made again (set_bucket).
+inline void require_walkable(const TreeBase* t) {
+  if (!t->walkable)
+    throw Error(E_INVALID, "the tree's hierarchies are incomplete: memory ran out while set_bucket made them");
+}
 
 }  // namespace pptkg
