@@ -411,10 +411,10 @@ class ResultSink:
 # queries.  A scaling constant: the full-size launches are too large to
 # capture, and the traffic of a launch grows with the queries it answers,
 # so the reported traffic is this figure times the queries of a launch.
-TRAFFIC_PER_QUERY = {"tree_order": 126.8, "scattered": 160.5,
+TRAFFIC_PER_QUERY = {"tree_order": 117.4, "scattered": 204.1,
                      # the fused kNN + normal launch (k_normals with kNN outputs) on a
                      # 256-cloud ragged batch of 11.5M points, every point in tree order
-                     "fused_tree_order": 102.1}
+                     "fused_tree_order": 105.5}
 
 
 def roofline(ctx, stage_name, queries, traffic_kind, bytes_per_query=BYTES_PER_QUERY):

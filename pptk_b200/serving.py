@@ -20,9 +20,10 @@ from concurrent.futures import Future, ThreadPoolExecutor
 
 import numpy as np
 
-# Bytes per point of a resident tree (tree-ordered points with index 16 B,
-# forward map 4 B, build records and traversal nodes ~48 B) and of a build's
-# transient scratch; bytes per query of a batch.
+# Bytes per point of a resident tree (tree-ordered points with index 16 B, the
+# index maps 8 B, build records, traversal nodes and the wide hierarchy ~41 B:
+# 1.3 GB for 20M points) and of a build's transient scratch; bytes per query of
+# a batch.
 TREE_BYTES_PER_POINT = 72
 BUILD_SCRATCH_PER_POINT = 160
 QUERY_BYTES = 96
