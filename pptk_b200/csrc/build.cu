@@ -1876,18 +1876,13 @@ constexpr size_t block_smem(int cap) {
 
 // k_block's grid: the blocks that the shared memory of a device's SMs holds.
 static int block_grid(size_t smem, int device) {
-  int nsm = 148, per_sm = 228 * 1024;
-  PPTKG_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device));
+  int per_sm = 228 * 1024;
   PPTKG_CUDA(cudaDeviceGetAttribute(&per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, device));
-  return std::max(nsm, 1) * std::max(1, std::min(8, (int)(per_sm / (smem + 3 * 1024))));
+  return sm_count(device) * std::max(1, std::min(8, (int)(per_sm / (smem + 3 * 1024))));
 }
 
 // Grid of the grid-stride level kernels: eight 256-thread blocks per SM.
-static int level_grid(int device) {
-  int nsm = 148;
-  PPTKG_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device));
-  return std::max(nsm, 1) * 8;
-}
+static int level_grid(int device) { return sm_count(device) * 8; }
 
 // Points of the largest segment that k_subtree takes, its list capacity and
 // its shared memory: 512 float points and their lists take 15 KB, so 14 warps
@@ -1971,10 +1966,9 @@ void lower_tnodes(TreeBase* tree, cudaStream_t st) {
 // k_subtree's grid: the warps that the shared memory of a device's SMs holds
 // (its dynamic part stays below the 48 KB that need no opt-in).
 static int subtree_grid(size_t smem, int device) {
-  int nsm = 148, per_sm = 228 * 1024;
-  PPTKG_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device));
+  int per_sm = 228 * 1024;
   PPTKG_CUDA(cudaDeviceGetAttribute(&per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, device));
-  return std::max(nsm, 1) * std::max(1, std::min(32, (int)(per_sm / (smem + 1024))));
+  return sm_count(device) * std::max(1, std::min(32, (int)(per_sm / (smem + 1024))));
 }
 
 // Segments above small_capacity() points that n points can have at a time.

@@ -46,10 +46,8 @@ TreeView<T, D> view_of(const TreeBase* t) {
   return v;
 }
 
-// Per-warp shared memory: the staging buffer (a leaf chunk in r-near walks,
-// the warp's queries in kNN walks), traversal stack, the 32 x 33 distance
-// matrix and the 32 candidate ids of the kNN bucket scan, and (normals)
-// `logcap` list slots per lane.
+// A warp's staging buffer: a leaf chunk in r-near walks, its queries and their
+// entry bounds in kNN walks.
 template <typename T, int D>
 __host__ __device__ constexpr size_t stage_bytes() {
   typedef typename DistOf<T>::type DistT;
@@ -715,9 +713,9 @@ struct StatusWord {
 };
 
 
-// kNN for k above the register lists' capacity: one thread per query, the
-// per-lane walk with its top-k in a device-memory heap (HeapTop), then a heap
-// sort into ascending order.  Queries run in chunks of `m` slots starting
+// kNN for k > WARP_MAX_K: one thread per query, the per-lane walk with its
+// top-k in a device-memory heap (HeapTop), then a heap sort into ascending
+// order.  Queries run in chunks of `m` slots starting
 // at slot `m0` of the processing order; hd / hp hold one heap per slot.
 constexpr int BIG_STACK = 128;
 
@@ -1640,7 +1638,7 @@ void launch_normals(const TreeBase* t, L ld, const int* order, int mode, int m, 
     // at least 32 warps per SM, then more queries per warp (they share the
     // cost of its solves)
     int per = 1;
-    while (per < 32 && m / (2 * per) >= 4736) per *= 2;
+    while (per < 32 && m / (2 * per) >= 32 * sm_count(t->device)) per *= 2;
     const size_t smem = QWARPS * (wide_stack(t->wlevels) + (size_t)KMAX * 16) * sizeof(int2);
     k_normals_warp<T, KMAX, L, PREC><<<div_up(m, QWARPS * per), QTHREADS, smem, st>>>(
         view_of<T, 3>(t), ld, order, mode, m, per, k, r2, num_eigen, gap_thr, ev, ew, sz, fix, nfix, status, fm, kidx,
@@ -2096,8 +2094,9 @@ void multi_tables(const TreeBase* const* trees, int ntrees, const int64_t* rows,
 
 // A stand-in tree carrying the batch-wide traversal bounds for the launch
 // helpers (which size shared memory from the tree they are given).
-static TreeBase* bounds_tree(int depth, int n_nodes, int wlevels, int64_t nv) {
+static TreeBase* bounds_tree(int device, int depth, int n_nodes, int wlevels, int64_t nv) {
   TreeBase* b = new TreeBase();
+  b->device = device;
   b->tdepth = depth;
   b->n_tnodes = n_nodes;
   b->wlevels = wlevels;
@@ -2156,7 +2155,7 @@ void multi_knn(const TreeBase* const* trees, int ntrees, const void* d_q, int qd
       qs.m = rows[g + 1] - rows[g];
       return qs;
     }, st, true);
-  std::unique_ptr<TreeBase> bt(bounds_tree(mt.depth, mt.n_nodes, mt.wlevels, mt.nv));
+  std::unique_ptr<TreeBase> bt(bounds_tree(trees[0]->device, mt.depth, mt.n_nodes, mt.wlevels, mt.nv));
   DevBuf<int> status(1, st);
   PPTKG_CUDA(cudaMemsetAsync(status.get(), 0, sizeof(int), st));
   const DistT r2 = radius2<DistT>(dmax);
@@ -2196,7 +2195,7 @@ void multi_normals(const TreeBase* const* trees, int ntrees, const int32_t* d_id
       qs.exclude_self = false;
       return qs;
     }, st);
-  std::unique_ptr<TreeBase> bt(bounds_tree(mt.depth, mt.n_nodes, mt.wlevels, mt.nv));
+  std::unique_ptr<TreeBase> bt(bounds_tree(trees[0]->device, mt.depth, mt.n_nodes, mt.wlevels, mt.nv));
   DevBuf<int> status(1, st);
   PPTKG_CUDA(cudaMemsetAsync(status.get(), 0, sizeof(int), st));
   const DistT rr = (DistT)(T)r;

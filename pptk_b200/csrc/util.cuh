@@ -27,6 +27,13 @@ void keep_pool_cached(cudaStream_t st);
 cudaError_t dev_malloc(void** p, size_t bytes, cudaStream_t st);
 void dev_free(void* p, cudaStream_t st);
 
+// Streaming multiprocessors of a device.
+inline int sm_count(int device) {
+  int n = 148;
+  PPTKG_CUDA(cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, device));
+  return n > 0 ? n : 1;
+}
+
 // ------------------------------------------------------------- DevBuf ----
 // Scratch memory that goes back when the buffer goes away, on the stream it
 // was allocated for: from the stream-ordered pool, or (CACHED) from
