@@ -1798,9 +1798,10 @@ void normals_query(const TreeBase* t, const QuerySpec& qs_in, int k, float r, in
   const BatchOrder kind = batch_order(t, qs);
   const bool warps = k == -1 ? rnear_by_warp(t->nv, m) : by_warp<T>(t->nv, m, k, Answer::normals, kind);
   int mode = 0;
-  // (long lists of warps gain nothing from tree order: k = 64, double, 40k
-  // points 602 us as they come, 657 in tree order; k = 16 240 and 232)
-  if (k > 0 && warps && (kind != BatchOrder::tree || k > 16) && m <= warp_unsorted(kind))
+  // (k_normals_warp gains nothing from tree order with long lists: k = 64,
+  // double, 40k points 602 us as they come, 657 in tree order; k = 16 240 and
+  // 232; beyond, the separate solves do: k = 70, 100k points 2767 and 2700)
+  if (k > 0 && warps && (kind != BatchOrder::tree || (k > 16 && k <= KNN_MAX_K)) && m <= warp_unsorted(kind))
     check_indices(t, qs, st);
   else
     mode = make_order<T, 3>(t, qs, order, st);

@@ -28,24 +28,32 @@ enum class Answer { knn, both, normals };
 //   kNN, float:       k = 8: 50x200 80 / 79, 6x5k 90 / 98; k = 16: 100x200 92 / 81, 60x1k 126 / 153,
 //                     1x60k 196 / 169, 5x60k 465 / 636; k = 32: 300x200 153 / 154, 60x5k 784 / 712,
 //                     1x1M 2760 / 2739; k = 64: 1x1M 7862 / 4566
-//   both, float:      k = 16: 50x200 101 / 87, 300x200 129 / 166, 1x60k 219 / 220; k = 32: 300x200
-//                     176 / 204, 1x60k 511 / 276, 200x5k 2974 / 2617; k = 64: 1x1M 8703 / 6647
-//   double:           normals k = 8: 100x200 99 / 102, k = 16: 6x5k 186 / 179, 1x60k 210 / 299,
-//                     k = 32: 1x1M 6598 / 4737; kNN k = 16: 300x1k 728 / 800, k = 64: 1x1M 25593 / 8337
+//   both, float:      k = 10: 1x57k 124 / 190; k = 16: 50x200 101 / 87, 300x200 129 / 166, 1x60k 219 / 220
+//                     k = 24: 11x8k 339 / 379, 1x4.8M (k = 20) 0.89 x; k = 32: 300x200 176 / 204,
+//                     1x60k 511 / 276, 200x5k 2974 / 2617; k = 64: 1x1M 8703 / 6647
+//   double:           normals k = 8: 100x200 99 / 102; k = 16: 6x5k 186 / 179, 1x60k 210 / 299; k = 30:
+//                     175x94 238 / 145, 1300x50 195 / 269; k = 32: 1x1M 6598 / 4737
+//                     kNN k = 16: 300x1k 728 / 800; k = 64: 1x1M 25593 / 8337
 inline int64_t tree_line(int64_t p, int k, bool f64, Answer a) {
   const int64_t all = INT64_MAX;
-  if (p < 128) return f64 && k > 16 ? 16384 : 4096;
-  if (k <= 4) return a != Answer::knn ? 10240 : f64 ? 20480 : 12288;
-  if (k <= 8) return a != Answer::knn ? (f64 ? 16384 : 12288) : f64 ? 28672 : p >= 1000 ? 24576 : 10240;
-  if (k <= 16) {
-    if (f64) return a == Answer::knn ? 200000 : 40960;
-    return a == Answer::knn    ? (p >= 5000 ? 98304 : 32768)
-           : a == Answer::both ? (p >= 5000 ? 65536 : 16384)
-                               : 20480;
+  const bool knn = a == Answer::knn, both = a == Answer::both;
+  if (p < 128) {
+    if (p >= 64 && k > (f64 ? 16 : 32)) return 65536;
+    return f64 && k > 8 ? 16384 : 4096;
   }
-  if (k > 32 || f64) return all;
-  if (p < 1000) return a == Answer::knn ? 65536 : 20480;
-  return a == Answer::knn ? 524288 : a == Answer::both ? all : 40960;
+  if (k <= 4) return !knn ? 10240 : f64 ? 20480 : 12288;
+  if (k <= 8) return !knn ? (f64 ? 16384 : 12288) : f64 ? 28672 : p >= 1000 ? 24576 : 10240;
+  if (k <= 16) {
+    if (f64) return knn ? 200000 : 40960;
+    // (k = 16 fills its list, which costs packets more than 9 to 15 do)
+    const bool full = k == 16 && p >= 5000;
+    return knn ? (full ? 98304 : 32768) : both ? (full ? 65536 : 16384) : 20480;
+  }
+  if (f64 || (knn && k > 32)) return all;
+  if (k > 32) return 131072;  // (above, 0.82 to 1.35 x, by the cloud)
+  if (p < 1000) return knn ? 65536 : 20480;
+  if (k < 32) return knn ? 131072 : 45056;
+  return knn ? 524288 : both ? 131072 : 40960;
 }
 
 // Whether m queries run one warp per query in place of 32-query packets:
