@@ -122,3 +122,23 @@ def test_refused_rebuild_leaves_every_record_readable(gpu):
     idx, cnt = f.knn(4)
     want, _ = ragged.Forest(torch.from_numpy(A).cuda(), [0, n]).knn(4)
     assert torch.equal(idx, want)
+
+
+@pytest.mark.parametrize("dim", [2, 3, 4])
+@pytest.mark.parametrize("dtype", [np.float32, np.float64, np.int8, np.int16, np.int32, np.int64, np.uint8, np.uint16,
+                                   np.uint32, np.uint64])
+def test_segments_at_the_edges_of_block_and_warp(gpu, port, dtype, dim):
+    # the largest segments of a warp and of a block and one point beyond, of
+    # words of 32 points, with and without ties, leaves of one point included
+    rng = np.random.default_rng(dim)
+    top = 1.0 if np.dtype(dtype).kind == "f" else float(min(np.iinfo(dtype).max, 10**6))
+    for n in (255, 257, 511, 513, 1023, 1025, 1056, 2047, 2048, 2049, 5000):
+        for steps in (5, 10**6):  # lattice positions per axis
+            P = (np.floor(rng.random((n, dim)) * steps) / steps * top).astype(dtype)
+            for leaf in (1, 10):
+                _is_reference_tree(gpu.kdtree._build(P, maxleafsize=leaf), port.PortTree(P, maxleafsize=leaf))
+    # every split takes a few points off, or divides a run of equal values
+    P = (np.exp(-rng.random((1500, dim)) * 12.0) * top).astype(dtype)
+    _is_reference_tree(gpu.kdtree._build(P), port.PortTree(P))
+    P[rng.random(1500) < 0.6, 0] = dtype(top / 2)
+    _is_reference_tree(gpu.kdtree._build(P), port.PortTree(P))
